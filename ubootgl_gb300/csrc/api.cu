@@ -506,7 +506,7 @@ int ubg_device_info(char *buf, size_t len) {
              "{\"name\": \"%s\", \"sm\": \"%d.%d\", \"sms\": %d, \"mem_gb\": %.1f, "
              "\"cluster_coarse_solve\": \"%s\"}",
              p.name, p.major, p.minor, p.multiProcessorCount, p.totalGlobalMem / 1e9,
-             cluster_coarse_solve_status());
+             "none: one block solves the coarse levels");
     return UBG_OK;
   });
 }

@@ -1,19 +1,20 @@
 // Multigrid pressure solver (class MG, pressure_solver.{hpp,cpp} of
 // te42kyfo/ubootgl) on the GPU.
 //
-//  k_mg        red-black Gauss-Seidel (rbgs + smoothingKernel,
-//              pressure_solver.cpp:10-24, 35-89), up to 5 sweeps temporally
-//              blocked in shared memory, with an optional prologue
-//              (prolongate + correct, pressure_solver.cpp:134-181), the
-//              zero-gradient boundary after every sweep on level 0
-//              (setZeroGradientBC, pressure_solver.cpp:183-192), and an
-//              optional epilogue that computes the residual and restricts it
-//              to the next level (calculateResidualField + restrict,
-//              pressure_solver.cpp:91-132) without writing the fine residual.
-//  k_mg_tail   the coarse end of the V-cycle in one CTA, in shared memory.
-//  k_mg_ctail  the coarse end from a larger level down in one launch of a
-//              16-CTA cluster: row bands with ghost rows exchanged through
-//              distributed shared memory, the tail's levels in CTA 0.
+//  k_tile      (k_tile.cuh) three red-black Gauss-Seidel sweeps (rbgs +
+//              smoothingKernel, pressure_solver.cpp:10-24, 35-89) on regions
+//              held in registers, after prolongate + correct
+//              (pressure_solver.cpp:134-181) or followed by the residual and
+//              its restriction to the next level (calculateResidualField +
+//              restrict, pressure_solver.cpp:91-132), with the zero-gradient
+//              boundary (setZeroGradientBC, pressure_solver.cpp:183-192).
+//  k_coarse    (k_coarse.cuh) the coarse end of the V-cycle in one block, from
+//              a level of at most 128 x 64 cells down.
+//  k_mg        up to 5 sweeps temporally blocked in shared memory: the
+//              coarsest level of a hierarchy without a tail, and one sweep
+//              with any alpha (the free function rbgs).
+//  k_mg_tail   the coarse end in one block for elongated levels, and in FP64
+//              for the mixed solver.
 //  k_residual  the residual field and its squared L2 norm.
 //  k_coarsen   MG::updateFields (pressure_solver.hpp:34-57), integer exact.
 //
@@ -21,7 +22,6 @@
 // all red points, then all black points, which is the reference's
 // deterministic schedule.  Every kernel reads one buffer and writes another,
 // so tiles never race on their halos.
-#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -148,6 +148,9 @@ struct Sto<float> {
   static __device__ __forceinline__ float tof(float v) { return v; }
   static __device__ __forceinline__ float fromf(float v) { return v; }
   static __device__ __forceinline__ float ldg1(const float *p) { return __ldg(p); }
+  static __device__ __forceinline__ float2 ldg2(const float *p) {
+    return __ldg(reinterpret_cast<const float2 *>(p));
+  }
 };
 template <>
 struct Sto<__half> {
@@ -177,6 +180,9 @@ struct Sto<__half> {
   static __device__ __forceinline__ float tof(__half v) { return __half2float(v); }
   static __device__ __forceinline__ __half fromf(float v) { return __float2half_rn(v); }
   static __device__ __forceinline__ float ldg1(const __half *p) { return __half2float(__ldg(p)); }
+  static __device__ __forceinline__ float2 ldg2(const __half *p) {
+    return __half22float2(__ldg(reinterpret_cast<const __half2 *>(p)));
+  }
 };
 template <>
 struct Sto<__nv_bfloat16> {
@@ -212,6 +218,9 @@ struct Sto<__nv_bfloat16> {
   static __device__ __forceinline__ float ldg1(const __nv_bfloat16 *p) {
     return __bfloat162float(__ldg(p));
   }
+  static __device__ __forceinline__ float2 ldg2(const __nv_bfloat16 *p) {
+    return __bfloat1622float2(__ldg(reinterpret_cast<const __nv_bfloat162 *>(p)));
+  }
 };
 
 // S: storage of the level's own arrays (in, out, rhs); SC: storage of the
@@ -236,8 +245,7 @@ struct MgArgsT {
   int cw, ch;
   float rfac;  // restriction weight: 1/16 (reference), 1/16 * (hc/h)^2 (scaled form)
   int tile;    // smoother tile id (-1: by level width), host side only
-  // epilogue: sum of r^2 over the tile's interior cells
-  double *norm2;
+  int zero_edges;  // the level's edge cells are 0 and stay 0 (the reference's coarse levels)
   // Tolerance-solver hierarchy (ext != 0): zero-gradient edges on every
   // level include the four corner cells, and the prolongation has no
   // zero columns / rows at the east and north ends (the coarse edges there
@@ -268,19 +276,64 @@ __device__ __forceinline__ float coarse_scale(const unsigned *bits, float h1sq, 
   return ldexpf(1.0f, -ex - kexp);
 }
 
+}  // namespace
+}  // namespace ubg
+#include "k_tile.cuh"
+#include "k_coarse.cuh"
+namespace ubg {
+namespace {
+
+template <class S, class SC, bool EXT, bool PRE, int R, int NW>
+__global__ void __launch_bounds__(32 * NW, 1024 / (32 * NW)) k_tile(MgArgsT<S, SC> a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  tile::fill_lut(reinterpret_cast<float2 *>(smem_raw + tile::Mem<R, NW>::lut), threadIdx.x, a.wsum,
+                 a.rwsum);
+  __syncthreads();
+  griddep_wait();
+  tile::run<S, SC, EXT, PRE, R, NW>(a, (int)blockIdx.x, smem_raw);
+}
+// One launch over the members of a batch (FP32): block -> member -> region.
+template <bool PRE, int R, int NW>
+__global__ void __launch_bounds__(32 * NW, 1024 / (32 * NW))
+    k_tile_m(const MgArgs *__restrict__ A, const int *__restrict__ bs, int n, unsigned tag,
+             unsigned *err) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  griddep_wait();
+  if (!table_ok(bs, n, tag, err)) return;
+  const int m = member_of(bs, n);
+  const MgArgs a = A[m];
+  tile::fill_lut(reinterpret_cast<float2 *>(smem_raw + tile::Mem<R, NW>::lut), threadIdx.x,
+                 A[m].wsum, A[m].rwsum);
+  __syncthreads();
+  tile::run<float, float, false, PRE, R, NW>(a, (int)blockIdx.x - __ldg(bs + m), smem_raw);
+}
+
+template <class S>
+__global__ void __launch_bounds__(32 * coarse::kWarps, 1)
+    k_coarse(const __grid_constant__ coarse::Args<S> a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  tile::fill_lut(reinterpret_cast<float2 *>(smem_raw + coarse::kLut), threadIdx.x, a.wsum, a.rwsum);
+  griddep_wait();
+  coarse::run<S>(a, smem_raw);
+}
+// One block per member of a batch (FP32).
+__global__ void __launch_bounds__(32 * coarse::kWarps, 1)
+    k_coarse_m(const coarse::Args<float> *__restrict__ A, const int *__restrict__ bs, int n,
+               unsigned tag, unsigned *err) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  griddep_wait();
+  if (!table_ok(bs, n, tag, err)) return;
+  const coarse::Args<float> &a = A[blockIdx.x];
+  tile::fill_lut(reinterpret_cast<float2 *>(smem_raw + coarse::kLut), threadIdx.x, a.wsum, a.rwsum);
+  coarse::run<float>(a, smem_raw);
+}
+
 template <int TX, int TY, int HALO>
 struct Tile {
   static constexpr int RX = TX + 2 * HALO, RY = TY + 2 * HALO, HX = RX / 2;
-  // coarse window for the prolongation prologue (rows padded to a multiple
-  // of 4 entries for vector access)
-  static constexpr int CW = HX + 4, CH = RY / 2 + 2;
   static_assert(RX % 4 == 0 && HALO % 4 == 0 && TX % 4 == 0 && TY % 2 == 0, "tile alignment");
-  // shared memory for element size ES: p and f in the split layout, codes,
-  // the coarse window (values of element size ESC, and flags)
-  static constexpr size_t smem(size_t ES = 4, size_t ESC = 0) {
-    return (size_t)2 * RY * HX * (2 * ES + 1) +
-           (((size_t)CW * CH * (ESC ? ESC : ES) + 15) / 16 * 16) + ((size_t)CW * CH + 15) / 16 * 16;
-  }
+  // shared memory for element size ES: p and f in the split layout, codes
+  static constexpr size_t smem(size_t ES = 4) { return (size_t)2 * RY * HX * (2 * ES + 1); }
 };
 
 // One multigrid smoothing launch on a tile of TX x TY cells with a halo of
@@ -290,14 +343,10 @@ struct Tile {
 // (no bank conflicts).  Red = (x+y) odd; region parity equals global parity
 // because x0 + y0 is even.  After half sweep i only cells within HALO - i of
 // the tile are still exact, so each half sweep updates just that cone.
-// EXT: the tolerance hierarchy's rules (a.ext, a.scale_bits) compiled in;
-// the reference's path is built without them.
-template <int TX, int TY, int HALO, bool ALPHA1, int NT, class S, class SC, bool EXT = false>
-__device__ __forceinline__ void k_mg_body(const MgArgsT<S, SC> &a, const int bx, const int by) {
-  constexpr int NTY = NT / 32;
+template <int TX, int TY, int HALO, bool ALPHA1, int NT, class S>
+__device__ __forceinline__ void k_mg_body(const MgArgsT<S> &a, const int bx, const int by) {
   using T = Tile<TX, TY, HALO>;
   using St = Sto<S>;
-  using Sc = Sto<SC>;
   constexpr int RX = T::RX, RY = T::RY, HX = T::HX;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   S *sp = reinterpret_cast<S *>(smem_raw);  // [2][RY][HX]
@@ -375,74 +424,6 @@ __device__ __forceinline__ void k_mg_body(const MgArgsT<S, SC> &a, const int bx,
           cv[it][hf] = __ldg(reinterpret_cast<const unsigned *>(a.code + (size_t)gy * P + x));
       }
     }
-    // coarse window of the prolongation prologue (post-smoothing): loaded
-    // while the code loads are in flight, stored before the same barrier
-    if (a.ec) {
-      constexpr int CW = T::CW, CH = T::CH;
-      SC *sec = reinterpret_cast<SC *>(sc + 2 * RY * HX);
-      uint8_t *scf = reinterpret_cast<uint8_t *>(sc + 2 * RY * HX) +
-                     ((size_t)CW * CH * sizeof(SC) + 15) / 16 * 16;
-      const int cxa = x0 >> 1, cya = y0 >> 1;
-      // all of a thread's loads in flight together, then the stores
-      if constexpr (HALO % 8 == 0) {
-        // cxa is a multiple of 4: 4 coarse entries per load (value and flag)
-        constexpr int CQ4 = (CW / 4) * CH, CIT = (CQ4 + NT - 1) / NT;
-        static_assert(CW % 4 == 0, "window rows of whole vectors");
-        float4 ev[CIT];
-        unsigned fv[CIT];
-  #pragma unroll
-        for (int it = 0; it < CIT; it++) {
-          const int q = tid + it * NT;
-          const int ly = q / (CW / 4), lx = 4 * (q - ly * (CW / 4));
-          const int cx = cxa + lx, cy = cya + ly;
-          ev[it] = make_float4(0.f, 0.f, 0.f, 0.f);
-          fv[it] = 0u;
-          if (q < CQ4 && cx >= 0 && cx < a.cw && cy >= 0 && cy < a.ch) {
-            ev[it] = Sc::ldg4(a.ec + (size_t)cy * a.cpitch + cx);
-            fv[it] = __ldg(reinterpret_cast<const unsigned *>(a.codec + (size_t)cy * a.cpitch + cx)) &
-                     0x01010101u;
-            if (cx + 3 >= a.cw) {  // entries at and beyond the level's width are 0
-              if (cx + 1 >= a.cw) ev[it].y = 0.f, fv[it] &= 0x000000ffu;
-              if (cx + 2 >= a.cw) ev[it].z = 0.f, fv[it] &= 0x0000ffffu;
-              ev[it].w = 0.f;
-              fv[it] &= 0x00ffffffu;
-            }
-          }
-        }
-  #pragma unroll
-        for (int it = 0; it < CIT; it++) {
-          const int q = tid + it * NT;
-          if (q < CQ4) {
-            Sc::sts4(sec + 4 * q, ev[it]);
-            *reinterpret_cast<unsigned *>(scf + 4 * q) = fv[it];
-          }
-        }
-      } else {
-        constexpr int CQ = CW * CH, CIT = (CQ + NT - 1) / NT;
-        float ev[CIT];
-        uint8_t fv[CIT];
-  #pragma unroll
-        for (int it = 0; it < CIT; it++) {
-          int q = tid + it * NT;
-          int ly = q / CW, lx = q - ly * CW;
-          int cx = cxa + lx, cy = cya + ly;
-          ev[it] = 0.0f;
-          fv[it] = 0;
-          if (q < CQ && cx >= 0 && cx < a.cw && cy >= 0 && cy < a.ch) {
-            ev[it] = Sc::ldg1(a.ec + (size_t)cy * a.cpitch + cx);
-            fv[it] = __ldg(a.codec + (size_t)cy * a.cpitch + cx) & 1u;
-          }
-        }
-  #pragma unroll
-        for (int it = 0; it < CIT; it++) {
-          int q = tid + it * NT;
-          if (q < CQ) {
-            sec[q] = Sc::fromf(ev[it]);
-            scf[q] = fv[it];
-          }
-        }
-      }
-    }
     load_store(sf, vf);
 #pragma unroll
     for (int it = 0; it < NIT; it++) {
@@ -486,88 +467,6 @@ __device__ __forceinline__ void k_mg_body(const MgArgsT<S, SC> &a, const int bx,
   const int kh = wid % KH, wpar = (wid / KH) & 1;
   const int k0 = 4 * ((lane & 7) + 8 * kh);
   const int rsub = (wid / (2 * KH)) * 8 + wpar + 2 * (lane >> 3);
-  // The prolongation prologue measures faster with wide rows: G threads per
-  // row, a warp on 32 / G rows two apart, its partner warp between them.
-  constexpr int G = HX / 4, RW = 32 / G;
-  static_assert(NT % G == 0 && 32 % G == 0, "vector layout");
-  const int k0w = 4 * (lane % G);
-  const int rsubw = (wid >> 1) * (2 * RW) + (wid & 1) + 2 * (lane / G);
-
-  // ---- prologue: correct(p, prolongate(ec)) on the interior cells, from
-  // the coarse window staged with the field loads above
-  if (a.ec) {
-    constexpr int CW = T::CW, CH = T::CH;
-    SC *sec = reinterpret_cast<SC *>(sc + 2 * RY * HX);
-    uint8_t *scf = reinterpret_cast<uint8_t *>(sc + 2 * RY * HX) +
-                   ((size_t)CW * CH * sizeof(SC) + 15) / 16 * 16;
-    // correction scale of scaled 16-bit coarse levels (1 otherwise)
-    float ecmul = 1.0f;
-    if (EXT && a.scale_bits) coarse_scale(a.scale_bits, a.scale_h1sq, a.scale_kexp, &ecmul);
-    const bool ext = EXT && a.ext != 0;
-    // prolongate (pressure_solver.cpp:134-172); e * fine flag = e here.
-    // Fine cell (rx, ry) = (2k + par, ry) lies over coarse column k of the
-    // window and coarse row ry / 2; x parity is par and y parity ry & 1, both
-    // fixed across the thread's 4 cells.
-#pragma unroll
-    for (int color = 0; color < 2; color++) {
-      for (int ry = rsubw; ry < RY; ry += RPP) {
-        const int par = (ry + color) & 1, yo = ry & 1;
-        const int gy = y0 + ry;
-        if (gy < 1 || gy >= h - 1) continue;
-        const int row = (color * RY + ry) * HX + k0w;
-        const unsigned cw4 = *reinterpret_cast<const unsigned *>(sc + row);
-        if ((cw4 & 0x01010101u) == 0u) continue;  // no fluid cell among the 4
-        const int eo = (ry >> 1) * CW + k0w;
-        const float4 ea = Sc::lds4(sec + eo);
-        const float E0[5] = {ea.x, ea.y, ea.z, ea.w, Sc::tof(sec[eo + 4])};
-        const unsigned fa = *reinterpret_cast<const unsigned *>(scf + eo);
-        const unsigned F0[5] = {fa & 0xffu, (fa >> 8) & 0xffu, (fa >> 16) & 0xffu, fa >> 24,
-                                scf[eo + 4]};
-        float E1[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
-        unsigned F1[5] = {0u, 0u, 0u, 0u, 0u};
-        if (yo) {
-          const float4 eb = Sc::lds4(sec + eo + CW);
-          E1[0] = eb.x;
-          E1[1] = eb.y;
-          E1[2] = eb.z;
-          E1[3] = eb.w;
-          E1[4] = Sc::tof(sec[eo + CW + 4]);
-          const unsigned fb = *reinterpret_cast<const unsigned *>(scf + eo + CW);
-          F1[0] = fb & 0xffu;
-          F1[1] = (fb >> 8) & 0xffu;
-          F1[2] = (fb >> 16) & 0xffu;
-          F1[3] = fb >> 24;
-          F1[4] = scf[eo + CW + 4];
-        }
-        const float4 pv = St::lds4(sp + row);
-        float out[4] = {pv.x, pv.y, pv.z, pv.w};
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-          const int gx = x0 + 2 * (k0w + j) + par;
-          if (gx < 1 || gx >= w - 1 || !((cw4 >> (8 * j)) & C_CENTER)) continue;
-          float pe;
-          if (!par && !yo) {
-            pe = E0[j];
-          } else if (par && !yo) {
-            const int k = F0[j] + F0[j + 1];
-            pe = (!ext && gx >= w - 2) ? 0.0f : div_rn(E0[j] + E0[j + 1], a.wsum[k], a.rwsum[k]);
-          } else if (!par && yo) {
-            const int k = F0[j] + F1[j];
-            pe = (!ext && gy >= h - 2) ? 0.0f : div_rn(E0[j] + E1[j], a.wsum[k], a.rwsum[k]);
-          } else {
-            const int k = F0[j] + F1[j + 1] + F0[j + 1] + F1[j];
-            pe = (!ext && (gx >= w - 2 || gy >= h - 2))
-                     ? 0.0f
-                     : div_rn(((E0[j] + E1[j + 1]) + E0[j + 1]) + E1[j], a.wsum[k], a.rwsum[k]);
-          }
-          if (EXT && a.scale_bits) pe = pe * ecmul;
-          out[j] = out[j] + pe;
-        }
-        St::sts4(sp + row, make_float4(out[0], out[1], out[2], out[3]));
-      }
-    }
-    __syncthreads();
-  }
 
   // setZeroGradientBC on this region (only tiles that touch the domain edge)
   const bool edge = x0 <= 0 || y0 <= 0 || x0 + RX >= w || y0 + RY >= h;
@@ -590,19 +489,7 @@ __device__ __forceinline__ void k_mg_body(const MgArgsT<S, SC> &a, const int bx,
       if (ry < 0 || ry >= RY || rn < 0 || rn >= RY) continue;
       sp[IDX(rx, ry)] = sp[IDX(rx, rn)];
     }
-    if (EXT && a.ext && tid < 4) {  // corner cell <- its diagonal interior neighbour
-      const int cxg = (tid & 1) ? w - 1 : 0, cyg = (tid & 2) ? h - 1 : 0;
-      const int rx = cxg - x0, ry = cyg - y0;
-      const int rnx = rx + ((tid & 1) ? -1 : 1), rny = ry + ((tid & 2) ? -1 : 1);
-      if (rx >= 0 && rx < RX && ry >= 0 && ry < RY && rnx >= 0 && rnx < RX && rny >= 0 &&
-          rny < RY)
-        sp[IDX(rx, ry)] = sp[IDX(rnx, rny)];
-    }
   };
-  if (a.zgbc && edge && a.ec) {
-    zero_gradient();
-    __syncthreads();
-  }
 
   // ---- red-black sweeps: a thread updates the 4 cells of its row group
   // (see the row mapping above)
@@ -720,162 +607,12 @@ __device__ __forceinline__ void k_mg_body(const MgArgsT<S, SC> &a, const int bx,
       if (gx + 2 < w) dst[2] = St::fromf(o.z);
     }
   }
-
-  if (!a.rc && !a.norm2) return;
-  // ---- residual on the tile grown by one cell (in place into f) ----------
-  // (per-thread partial sums of r^2 in FP32, a handful of terms each; the
-  // block and global sums are FP64.  No FP64 arithmetic in the cell loop:
-  // GB300's FP64 rate is a small fraction of FP32.)
-  float acc = 0.0f;
-  const int rlo = a.rc ? HALO - 1 : HALO;
-  const int rhix = a.rc ? HALO + TX : HALO + TX - 1, rhiy = a.rc ? HALO + TY : HALO + TY - 1;
-#pragma unroll
-  for (int color = 0; color < 2; color++) {
-    const S *self = sp + color * RY * HX;
-    const S *oth = sp + (color ^ 1) * RY * HX;
-    S *fs = sf + color * RY * HX;
-    const uint8_t *cs = sc + color * RY * HX;
-    for (int ry = rlo + rsub; ry <= rhiy; ry += RPP) {
-      const int par = (ry + color) & 1;
-      const int gy = y0 + ry;
-      const int row = ry * HX + k0;
-      const float4 o = St::lds4(oth + row);
-      const float ex = St::tof(par ? oth[row + 4] : oth[row - 1]);
-      const float4 os = St::lds4(oth + row - HX);
-      const float4 on = St::lds4(oth + row + HX);
-      const float4 fv = St::lds4(fs + row);
-      const float4 sv = St::lds4(self + row);
-      const uchar4 cv = *reinterpret_cast<const uchar4 *>(cs + row);
-      const float W4[4] = {par ? o.x : ex, par ? o.y : o.x, par ? o.z : o.y, par ? o.w : o.z};
-      const float E4[4] = {par ? o.y : o.x, par ? o.z : o.y, par ? o.w : o.z, par ? ex : o.w};
-      const float S4[4] = {os.x, os.y, os.z, os.w}, N4[4] = {on.x, on.y, on.z, on.w};
-      const float F4[4] = {fv.x, fv.y, fv.z, fv.w}, P4[4] = {sv.x, sv.y, sv.z, sv.w};
-      const unsigned C4[4] = {cv.x, cv.y, cv.z, cv.w};
-      float out[4];
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const int rx = 2 * (k0 + j) + par, gx = x0 + rx;
-        float r = 0.0f;
-        if (rx >= rlo && rx <= rhix && gx >= 1 && gx < w - 1 && gy >= 1 && gy < h - 1) {
-          r = resid1(C4[j], P4[j], W4[j], E4[j], S4[j], N4[j], F4[j], a.ihsq);
-          if (a.norm2 && rx >= HALO && rx < HALO + TX && ry >= HALO && ry < HALO + TY)
-            acc = __fmaf_rn(r, r, acc);
-        }
-        out[j] = r;
-      }
-      if (a.rc) St::sts4(fs + row, make_float4(out[0], out[1], out[2], out[3]));
-    }
-  }
-  __syncthreads();
-  if (a.norm2) {
-    __shared__ double red[NTY];
-    double dacc = (double)acc;
-    for (int o = 16; o > 0; o >>= 1) dacc += __shfl_xor_sync(0xffffffffu, dacc, o);
-    if (tx == 0) red[ty] = dacc;
-    __syncthreads();
-    if (tid == 0) {
-      double t = 0.0;
-      for (int i = 0; i < NTY; i++) t += red[i];
-      atomicAdd(a.norm2, t);
-    }
-  }
-  // ---- restrict (pressure_solver.cpp:118-132) onto the coarse tile -------
-  if (a.rc) {
-    const int cx0 = bx * (TX / 2), cy0 = by * (TY / 2);
-    float rfac = a.rfac;
-    if (EXT && a.scale_bits) {
-      float inv;
-      rfac = rfac * (coarse_scale(a.scale_bits, a.scale_h1sq, a.scale_kexp, &inv) * a.scale_h1sq);
-    }
-    // one coarse cell: full weighting of the 3x3 fine residuals around it
-    auto restrict1 = [&](float m1, float c0, float p1, float m2, float c2, float p2, float m3,
-                         float c3, float p3) {
-      float v = (m1 * 1.0f + c0 * 2.0f) + p1 * 1.0f;
-      v = v + ((m2 * 2.0f + c2 * 4.0f) + p2 * 2.0f);
-      v = v + ((m3 * 1.0f + c3 * 2.0f) + p3 * 1.0f);
-      return v * rfac;
-    };
-    if constexpr (HALO % 8 == 0 && (TX / 2) % 4 == 0) {
-      // 4 consecutive coarse cells per thread.  Coarse column X sits over
-      // fine column rx = 2X - x0 (even): its centre values are entries kc =
-      // rx / 2 of the colour-(ry & 1) rows, its west / east neighbours
-      // entries kc - 1 / kc of the other colour; kc is a multiple of 4.
-      constexpr int CXG = TX / 8, NQR = CXG * (TY / 2);
-      for (int q = tid; q < NQR; q += NT) {
-        const int cyy = q / CXG, g = q - cyy * CXG;
-        const int X0 = cx0 + 4 * g, Y = cy0 + cyy;
-        if (X0 >= a.cw || Y >= a.ch) continue;
-        const int ry = 2 * Y - y0, kc = (2 * X0 - x0) >> 1;
-        float cen[3][4], oth[3][5];
-#pragma unroll
-        for (int e = 0; e < 3; e++) {
-          const int r = ry + e - 1, c = r & 1;
-          const float4 u = St::lds4(sf + (c * RY + r) * HX + kc);
-          const float4 o = St::lds4(sf + ((c ^ 1) * RY + r) * HX + kc);
-          cen[e][0] = u.x;
-          cen[e][1] = u.y;
-          cen[e][2] = u.z;
-          cen[e][3] = u.w;
-          oth[e][0] = St::tof(sf[((c ^ 1) * RY + r) * HX + kc - 1]);
-          oth[e][1] = o.x;
-          oth[e][2] = o.y;
-          oth[e][3] = o.z;
-          oth[e][4] = o.w;
-        }
-        float v[4];
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-          const int X = X0 + j;
-          v[j] = 0.0f;
-          if (X >= 1 && X < a.cw - 1 && Y >= 1 && Y < a.ch - 1)
-            v[j] = restrict1(oth[0][j], cen[0][j], oth[0][j + 1], oth[1][j], cen[1][j],
-                             oth[1][j + 1], oth[2][j], cen[2][j], oth[2][j + 1]);
-        }
-        SC *dst = a.rc + (size_t)Y * a.cpitch + X0;
-        if (X0 + 3 < a.cw) {
-          Sc::st4(dst, make_float4(v[0], v[1], v[2], v[3]));
-        } else {
-#pragma unroll
-          for (int j = 0; j < 4; j++)
-            if (X0 + j < a.cw) dst[j] = Sc::fromf(v[j]);
-        }
-      }
-    } else {
-      for (int q = tid; q < (TX / 2) * (TY / 2); q += NT) {
-        int cyy = q / (TX / 2), cxx = q - cyy * (TX / 2);
-        int X = cx0 + cxx, Y = cy0 + cyy;
-        if (X >= a.cw || Y >= a.ch) continue;
-        float v = 0.0f;
-        if (X >= 1 && X < a.cw - 1 && Y >= 1 && Y < a.ch - 1) {
-          int rx = 2 * X - x0, ry = 2 * Y - y0;
-          auto R = [&](int dx, int dy) { return St::tof(sf[IDX(rx + dx, ry + dy)]); };
-          v = restrict1(R(-1, -1), R(0, -1), R(1, -1), R(-1, 0), R(0, 0), R(1, 0), R(-1, 1),
-                        R(0, 1), R(1, 1));
-        }
-        a.rc[(size_t)Y * a.cpitch + X] = Sc::fromf(v);
-      }
-    }
-  }
 }
 
-template <int TX, int TY, int HALO, bool ALPHA1, int NT, class S = float, class SC = S,
-          bool EXT = false>
-__global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : (NT == 512 ? 2 : 4))
-    k_mg(MgArgsT<S, SC> a) {
+template <int TX, int TY, int HALO, bool ALPHA1, int NT, class S = float>
+__global__ void __launch_bounds__(NT, 4) k_mg(MgArgsT<S> a) {
   griddep_wait();
-  k_mg_body<TX, TY, HALO, ALPHA1, NT, S, SC, EXT>(a, blockIdx.x, blockIdx.y);
-}
-// One launch over the members of a batch (FP32): block -> member -> tile.
-template <int TX, int TY, int HALO, bool ALPHA1, int NT>
-__global__ void __launch_bounds__(NT, NT >= 1024 ? 1 : (NT == 512 ? 2 : 4))
-    k_mg_m(const MgArgs *__restrict__ A, const int *__restrict__ bs, int n, unsigned tag,
-           unsigned *err) {
-  griddep_wait();
-  if (!table_ok(bs, n, tag, err)) return;
-  const int m = member_of(bs, n);
-  const MgArgs &a = A[m];
-  const int l = (int)blockIdx.x - __ldg(bs + m), gx = (a.w + TX - 1) / TX;
-  k_mg_body<TX, TY, HALO, ALPHA1, NT, float, float>(a, l % gx, l / gx);
+  k_mg_body<TX, TY, HALO, ALPHA1, NT, S>(a, blockIdx.x, blockIdx.y);
 }
 
 // ------------------------------------------------------ residual field only
@@ -1202,407 +939,68 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1)
   k_mg_tail_body<float, float>(A[blockIdx.x]);
 }
 
-// ------------------------------------------------ cluster coarse solve
-// The coarse end of the V-cycle from a level of up to ~512x256 cells down,
-// in one launch of a cluster of CT_CTAS thread blocks (the reference's
-// hierarchy, FP32).  Levels cluster_top .. tail_top-1 are split into row
-// bands, one per block, each in its block's shared memory with one ghost
-// row on either side.  After a phase changes the first or last row of a
-// band, the block writes those cells into its neighbours' ghost rows
-// through distributed shared memory, and the cluster barrier makes them
-// visible.  The bands nest: block k owns rows [2b, 2b') of a level when it
-// owns rows [b, b') of the next coarser one (the last block also takes the
-// extra rows of odd heights), so a restriction reads only its band and the
-// ghost row below it, and a prolongation its coarse band and the ghost row
-// above.  The tail's levels (tail_top down) run in block 0 alone, as in the
-// one-block tail kernel.  Every cell goes through the arithmetic of the
-// tiled kernels and the tail, so the results are the same bits.  Each
-// sweep's half only sends the cells of the colour it updated: the
-// neighbour reads only the other colour of its ghost rows in that phase.
-namespace cg = cooperative_groups;
-constexpr int CT_MAXD = 6;
-constexpr int CT_CTAS = 16;
-constexpr size_t CT_SMEM_MAX = 227 * 1024;
-
-struct CtLevel {
-  int w, h, rows;     // level size; local rows per block (largest band + 2)
-  float hh, ihsq, rfac;
-  int oe, orr, orhs;  // float offsets of the local e / r / rhs arrays (rows x w)
-  int oc;             // byte offset of the local codes
-  int band[CT_CTAS + 1];
-  const uint8_t *code;
-  int code_pitch;
-};
-struct CTailArgs {
-  int nd;                    // banded levels
-  CtLevel D[CT_MAXD];
-  int tband[CT_CTAS + 1];    // row bands of the tail's top level (restriction targets)
-  TailArgs<float> tail;      // the tail's levels, run by block 0
-  int tail_fo, tail_bo;      // float / byte offsets of the tail's region
-  int float_words;           // floats before the byte region
-  const float *rhs_top;      // level cluster_top's rhs and result (global)
-  int rhs_pitch;
-  float *e_top;
-  int e_pitch;
-  float wsum[5], rwsum[5];
-};
-
-__global__ void __launch_bounds__(TAIL_THREADS, 1) k_mg_ctail(const __grid_constant__ CTailArgs a) {
-  griddep_wait();
-  cg::cluster_group cl = cg::this_cluster();
-  const int rank = (int)cl.block_rank();
-  constexpr int C = CT_CTAS;
-  constexpr int NT = TAIL_THREADS;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  float *fm = reinterpret_cast<float *>(smem_raw);
-  uint8_t *bm = smem_raw + (size_t)a.float_words * sizeof(float);
-  const int tid = threadIdx.y * 32 + threadIdx.x;
-  const float ws0 = a.wsum[0], ws1 = a.wsum[1], ws2 = a.wsum[2], ws3 = a.wsum[3], ws4 = a.wsum[4];
-  const float rw0 = a.rwsum[0], rw1 = a.rwsum[1], rw2 = a.rwsum[2], rw3 = a.rwsum[3],
-              rw4 = a.rwsum[4];
-  auto DIVW = [&](float x, int k) -> float {
-    const float d = k == 0 ? ws0 : (k == 1 ? ws1 : (k == 2 ? ws2 : (k == 3 ? ws3 : ws4)));
-    const float r = k == 0 ? rw0 : (k == 1 ? rw1 : (k == 2 ? rw2 : (k == 3 ? rw3 : rw4)));
-    return div_rn(x, d, r);
-  };
-  // (row, 32-column segment) items to warps, columns to lanes: one
-  // division per warp item instead of one per cell
-  const int wid = tid >> 5, lane = tid & 31;
-  auto for_cells = [&](int nrows, int ncols, auto &&fn) {
-    const int nseg = (ncols + 31) >> 5;
-    for (int it = wid; it < nrows * nseg; it += NT / 32) {
-      const int r = it / nseg, c = (it - r * nseg) * 32 + lane;
-      if (c < ncols) fn(r, c);
-    }
-  };
-
-  // load: codes of the band and ghost rows, zeroed e / r, level 0's rhs
-  for (int d = 0; d < a.nd; d++) {
-    const CtLevel &L = a.D[d];
-    const int y0 = L.band[rank], y1 = L.band[rank + 1], w = L.w;
-    for_cells(y1 - y0 + 2, w, [&](int lr, int x) {
-      const int y = y0 - 1 + lr, k = lr * w + x;
-      const bool in = y >= 0 && y < L.h;
-      bm[L.oc + k] = in ? L.code[(size_t)y * L.code_pitch + x] : (uint8_t)0;
-      fm[L.oe + k] = 0.0f;
-      fm[L.orr + k] = 0.0f;
-      fm[L.orhs + k] = (d == 0 && y >= y0 && y < y1) ? a.rhs_top[(size_t)y * a.rhs_pitch + x] : 0.0f;
-    });
-  }
-  if (rank == 0) tail_load<float, float>(a.tail, fm + a.tail_fo, bm + a.tail_bo, false);
-  cl.sync();
-
-  // The first / last band row of array `off` of level d into the
-  // neighbours' ghost rows: the cells of colour `color` ((x + y + color)
-  // even), or whole rows for color < 0.
-  auto send_rows = [&](int d, int off, int color, bool first, bool last) {
-    const CtLevel &L = a.D[d];
-    const int y0 = L.band[rank], y1 = L.band[rank + 1], w = L.w;
-    float *arr = fm + off;
-    if (first && rank > 0) {
-      float *dst = cl.map_shared_rank(arr, rank - 1) + (y0 - L.band[rank - 1] + 1) * w;
-      const float *src = arr + w;
-      for (int x = tid; x < w; x += NT)
-        if (color < 0 || ((x + y0 + color) & 1) == 0) dst[x] = src[x];
-    }
-    if (last && rank < C - 1) {
-      float *dst = cl.map_shared_rank(arr, rank + 1);
-      const float *src = arr + (y1 - y0) * w;
-      for (int x = tid; x < w; x += NT)
-        if (color < 0 || ((x + y1 - 1 + color) & 1) == 0) dst[x] = src[x];
-    }
-  };
-
-  // one half-sweep (colour `color`) of level d's band, then the exchange
-  auto dsweep = [&](int d, int color) {
-    const CtLevel &L = a.D[d];
-    const int w = L.w, y0 = L.band[rank], y1 = L.band[rank + 1], hw2 = (w + 1) / 2;
-    float *e = fm + L.oe;
-    const float *f = fm + L.orhs;
-    const uint8_t *c = bm + L.oc;
-    const float hh = L.hh;
-    const int ya = max(y0, 1), yb = min(y1, L.h - 1);
-    for_cells(max(yb - ya, 0), hw2, [&](int ry, int j) {
-      const int y = ya + ry;
-      const int x = 2 * j + ((y + color) & 1);
-      if (x < 1 || x >= w - 1) return;
-      const int i = (y - y0 + 1) * w + x;
-      const unsigned ci = c[i];
-      const float pw = e[i - 1], pe = e[i + 1], ps = e[i - w], pn = e[i + w], fi = f[i];
-      if (ci == (C_CENTER | C_W | C_E | C_S | C_N))
-        e[i] = ((((pw + pe) + ps) + pn) + fi * hh * hh) * 0.25f;
-      else
-        e[i] = rb_update1<float>(ci, pw, pe, ps, pn, fi, hh);
-    });
-    __syncthreads();
-    send_rows(d, L.oe, color, true, true);
-    cl.sync();
-  };
-
-  // residual of level d's band; the last band row goes to the next block
-  auto dresid = [&](int d) {
-    const CtLevel &L = a.D[d];
-    const int w = L.w, y0 = L.band[rank], y1 = L.band[rank + 1];
-    const float *e = fm + L.oe, *f = fm + L.orhs;
-    float *r = fm + L.orr;
-    const uint8_t *c = bm + L.oc;
-    const float ihsq = L.ihsq;
-    for_cells(y1 - y0, w, [&](int ry, int x) {
-      const int y = y0 + ry, q = (ry + 1) * w + x;
-      float rv = 0.0f;
-      if (x >= 1 && x < w - 1 && y >= 1 && y < L.h - 1)
-        rv = resid1<float>(c[q], e[q], e[q - 1], e[q + 1], e[q - w], e[q + w], f[q], ihsq);
-      r[q] = rv;
-    });
-    __syncthreads();
-    send_rows(d, L.orr, -1, false, true);
-    cl.sync();
-  };
-
-  // full-weighting restriction of level d's residual into the next level's
-  // rhs: its band (local) or, below the banded levels, the tail's top level
-  // in block 0
-  auto drestrict = [&](int d) {
-    const CtLevel &L = a.D[d];
-    const bool to_tail = d + 1 == a.nd;
-    const int w = L.w, y0 = L.band[rank];
-    const int wc = to_tail ? a.tail.L[0].w : a.D[d + 1].w;
-    const int hc = to_tail ? a.tail.L[0].h : a.D[d + 1].h;
-    const int Y0 = to_tail ? a.tband[rank] : a.D[d + 1].band[rank];
-    const int Y1 = to_tail ? a.tband[rank + 1] : a.D[d + 1].band[rank + 1];
-    float *rc = to_tail ? cl.map_shared_rank(fm + a.tail_fo + a.tail.L[0].orhs, 0)
-                        : fm + a.D[d + 1].orhs;
-    const float *r = fm + L.orr;
-    const float rfac = L.rfac;
-    for_cells(Y1 - Y0, wc, [&](int rY, int X) {
-      const int Y = Y0 + rY;
-      if (X < 1 || X >= wc - 1 || Y < 1 || Y >= hc - 1) return;
-      const float *R0 = r + (2 * Y - y0 + 1) * w + 2 * X;
-      float v = (R0[-w - 1] * 1.0f + R0[-w] * 2.0f) + R0[-w + 1] * 1.0f;
-      v = v + ((R0[-1] * 2.0f + R0[0] * 4.0f) + R0[1] * 2.0f);
-      v = v + ((R0[w - 1] * 1.0f + R0[w] * 2.0f) + R0[w + 1] * 1.0f);
-      v = v * rfac;
-      if (to_tail)
-        rc[Y * wc + X] = v;
-      else
-        rc[(Y - Y0 + 1) * wc + X] = v;
-    });
-    cl.sync();
-  };
-
-  // prolongation of the next level's e onto level d's band, correction,
-  // then whole first / last rows to the neighbours
-  auto dprolong = [&](int d) {
-    const CtLevel &L = a.D[d];
-    const bool from_tail = d + 1 == a.nd;
-    const int w = L.w, y0 = L.band[rank], y1 = L.band[rank + 1];
-    float *e = fm + L.oe;
-    const uint8_t *c = bm + L.oc;
-    const int wc = from_tail ? a.tail.L[0].w : a.D[d + 1].w;
-    const int Y0 = from_tail ? 0 : a.D[d + 1].band[rank] - 1;
-    const float *ec = from_tail ? cl.map_shared_rank(fm + a.tail_fo + a.tail.L[0].oe, 0)
-                                : fm + a.D[d + 1].oe;
-    const uint8_t *cg_ = from_tail ? a.tail.code[0] : bm + a.D[d + 1].oc;
-    const int cpitch = from_tail ? a.tail.code_pitch[0] : wc;
-    auto E = [&](int xx, int yy) { return ec[(yy - Y0) * wc + xx]; };
-    auto F = [&](int xx, int yy) {
-      return (int)((from_tail ? __ldg(cg_ + (size_t)yy * cpitch + xx)
-                              : cg_[(size_t)(yy - Y0) * cpitch + xx]) &
-                   1u);
-    };
-    for_cells(y1 - y0, w, [&](int ry, int x) {
-      const int y = y0 + ry;
-      if (x < 1 || x >= w - 1 || y < 1 || y >= L.h - 1) return;
-      const int q = (ry + 1) * w + x;
-      if (!(c[q] & C_CENTER)) return;
-      const int cx = x >> 1, cy = y >> 1;
-      const bool xo = x & 1, yo = y & 1;
-      float ev;
-      if (!xo && !yo)
-        ev = E(cx, cy);
-      else if (xo && !yo)
-        ev = (x >= w - 2) ? 0.0f : DIVW(E(cx, cy) + E(cx + 1, cy), F(cx, cy) + F(cx + 1, cy));
-      else if (!xo && yo)
-        ev = (y >= L.h - 2) ? 0.0f : DIVW(E(cx, cy) + E(cx, cy + 1), F(cx, cy) + F(cx, cy + 1));
-      else
-        ev = (x >= w - 2 || y >= L.h - 2)
-                 ? 0.0f
-                 : DIVW(((E(cx, cy) + E(cx + 1, cy + 1)) + E(cx + 1, cy)) + E(cx, cy + 1),
-                        F(cx, cy) + F(cx + 1, cy + 1) + F(cx + 1, cy) + F(cx, cy + 1));
-      e[q] = e[q] + ev;
-    });
-    __syncthreads();
-    send_rows(d, L.oe, -1, true, true);
-    cl.sync();
-  };
-
-  for (int d = 0; d < a.nd; d++) {
-    for (int s = 0; s < 3; s++) {
-      dsweep(d, 1);
-      dsweep(d, 0);
-    }
-    dresid(d);
-    drestrict(d);
-  }
-  if (rank == 0) tail_levels<float, float>(a.tail, fm + a.tail_fo, bm + a.tail_bo);
-  cl.sync();
-  for (int d = a.nd - 1; d >= 0; d--) {
-    dprolong(d);
-    for (int s = 0; s < 3; s++) {
-      dsweep(d, 1);
-      dsweep(d, 0);
-    }
-  }
-  {
-    const CtLevel &L = a.D[0];
-    const int w = L.w, y0 = L.band[rank], y1 = L.band[rank + 1];
-    for_cells(y1 - y0, w, [&](int ry, int x) {
-      a.e_top[(size_t)(y0 + ry) * a.e_pitch + x] = fm[L.oe + (ry + 1) * w + x];
-    });
-  }
-  cl.sync();  // no block leaves while another may still read its memory
-}
-
 // ------------------------------------------------------------ launches
-// The tiles the tolerance hierarchy uses (chosen by level width): the only
-// ones built with its rules.
-template <int TX, int TY, int HALO, bool A1>
-constexpr bool ext_tile() {
-  return A1 && HALO == 8 && ((TX == 112 && TY == 50) || (TX == 48 && TY == 16));
-}
-
-template <int TX, int TY, int HALO, bool A1, int NT = 256, class S = float, class SC = S>
-void launch_mg_t(const MgArgsT<S, SC> &a, cudaStream_t st) {
+template <int TX, int TY, int HALO, bool A1, int NT = 256, class S = float>
+void launch_mg_t(const MgArgsT<S> &a, cudaStream_t st) {
   using T = Tile<TX, TY, HALO>;
   dim3 grid((a.w + TX - 1) / TX, (a.h + TY - 1) / TY);
-  if (a.ext) {
-    if constexpr (ext_tile<TX, TY, HALO, A1>()) {
-      launch_pdl(k_mg<TX, TY, HALO, A1, NT, S, SC, true>, grid, dim3(32, NT / 32),
-                 T::smem(sizeof(S), sizeof(SC)), st, a);
-    } else {
-      throw ArgError("tolerance hierarchy: tile not built with its rules");
-    }
-  } else if constexpr (std::is_same<S, SC>::value) {
-    launch_pdl(k_mg<TX, TY, HALO, A1, NT, S, SC, false>, grid, dim3(32, NT / 32),
-               T::smem(sizeof(S), sizeof(SC)), st, a);
-  } else {
-    throw ArgError("mixed storage types only in the tolerance hierarchy");
-  }
+  launch_pdl(k_mg<TX, TY, HALO, A1, NT, S>, grid, dim3(32, NT / 32), T::smem(sizeof(S)), st, a);
   UBG_LAUNCH_CHECK();
   g_stats.launches++;
 }
 
-template <int TX, int TY, int HALO, bool A1, int NT = 256, class S = float, class SC = S,
-          bool EXT = false>
-void set_smem_attr() {
-  UBG_CUDA(cudaFuncSetAttribute(k_mg<TX, TY, HALO, A1, NT, S, SC, EXT>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)Tile<TX, TY, HALO>::smem(sizeof(S), sizeof(SC))));
-  // one carveout for every kernel of a V-cycle: no L1 / shared-memory
-  // reconfiguration between consecutive launches
-  UBG_CUDA(cudaFuncSetAttribute(k_mg<TX, TY, HALO, A1, NT, S, SC, EXT>,
-                                cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+// One carveout for every kernel of a V-cycle: no L1 / shared-memory
+// reconfiguration between consecutive launches.
+template <class K>
+void set_smem_attr(K *k, size_t bytes) {
+  UBG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  UBG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
 }
 
-template <class S, class T>
-void set_tail_attr() {
-  UBG_CUDA(cudaFuncSetAttribute(k_mg_tail<S, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)TAIL_SMEM_MAX));
-  UBG_CUDA(cudaFuncSetAttribute(k_mg_tail<S, T>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-}
+constexpr size_t kCoarseSmemMax = 200 * 1024;
 
-template <class S>
-void set_vcycle_attrs() {
-  set_smem_attr<112, 50, 8, true, 512, S>();
-  set_smem_attr<48, 16, 8, true, 256, S>();
-  set_smem_attr<40, 8, 12, true, 256, S>();
-  set_smem_attr<112, 24, 8, true, 256, S>();
-  set_smem_attr<48, 40, 8, true, 256, S>();
-  set_smem_attr<112, 114, 8, true, 1024, S>();
+template <class S, class SC, bool EXT, int R>
+void set_tile_attr() {
+  set_smem_attr(k_tile<S, SC, EXT, true, R, tile::kWarps>, tile::Mem<R, tile::kWarps>::bytes);
+  set_smem_attr(k_tile<S, SC, EXT, false, R, tile::kWarps>, tile::Mem<R, tile::kWarps>::bytes);
 }
-
-template <int TX, int TY, int HALO>
-void set_multi_attr() {
-  constexpr int NT = TX == 112 && TY == 50 ? 512 : (TX == 112 && TY == 114 ? 1024 : 256);
-  UBG_CUDA(cudaFuncSetAttribute(k_mg_m<TX, TY, HALO, true, NT>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)Tile<TX, TY, HALO>::smem(4)));
-  UBG_CUDA(cudaFuncSetAttribute(k_mg_m<TX, TY, HALO, true, NT>,
-                                cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+template <class S, class SC, bool EXT>
+void set_tile_attrs() {
+  set_tile_attr<S, SC, EXT, 2>();
+  set_tile_attr<S, SC, EXT, 4>();
 }
 
 // Sets the shared-memory attributes of every smoother and tail kernel, once
 // per process (function-local static initialisation is thread-safe; the
 // server's worker thread and the caller's threads may race here).
-bool g_ctail_ok = false;  // a cluster of the coarse solve fits this device
-char g_ctail_why[160] = "not probed";
-
 static void set_all_kernel_attributes() {
-  set_multi_attr<112, 50, 8>();
-  set_multi_attr<48, 16, 8>();
-  set_multi_attr<40, 8, 12>();
-  set_multi_attr<112, 24, 8>();
-  set_multi_attr<48, 40, 8>();
-  set_multi_attr<112, 114, 8>();
-  UBG_CUDA(cudaFuncSetAttribute(k_mg_tail_m, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)TAIL_SMEM_MAX));
-  UBG_CUDA(cudaFuncSetAttribute(k_mg_tail_m, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-  set_vcycle_attrs<float>();
-  set_smem_attr<56, 24, 4, false>();
-  set_tail_attr<float, float>();
-  set_vcycle_attrs<__half>();
-  set_vcycle_attrs<__nv_bfloat16>();
-  set_tail_attr<__half, double>();
-  set_tail_attr<__nv_bfloat16, double>();
-  // the tolerance solver: its rules on the width-chosen tiles, FP32 level 0
-  // over 16-bit coarse levels, FP32 arithmetic in the tail over 16-bit
-  // storage
-  set_smem_attr<112, 50, 8, true, 512, float, float, true>();
-  set_smem_attr<48, 16, 8, true, 256, float, float, true>();
-  set_smem_attr<112, 50, 8, true, 512, __half, __half, true>();
-  set_smem_attr<48, 16, 8, true, 256, __half, __half, true>();
-  set_smem_attr<112, 50, 8, true, 512, __nv_bfloat16, __nv_bfloat16, true>();
-  set_smem_attr<48, 16, 8, true, 256, __nv_bfloat16, __nv_bfloat16, true>();
-  set_smem_attr<112, 50, 8, true, 512, float, __half, true>();
-  set_smem_attr<48, 16, 8, true, 256, float, __half, true>();
-  set_smem_attr<112, 50, 8, true, 512, float, __nv_bfloat16, true>();
-  set_smem_attr<48, 16, 8, true, 256, float, __nv_bfloat16, true>();
-  set_tail_attr<__half, float>();
-  set_tail_attr<__nv_bfloat16, float>();
-  // the cluster coarse solve: 16 blocks of up to 227 KB each, if the device
-  // can hold such a cluster (else the launches per level are used)
-  g_ctail_ok = false;
-  cudaError_t e1 = cudaFuncSetAttribute(k_mg_ctail, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)CT_SMEM_MAX);
-  cudaError_t e2 = e1 == cudaSuccess
-                       ? cudaFuncSetAttribute(k_mg_ctail,
-                                              cudaFuncAttributeNonPortableClusterSizeAllowed, 1)
-                       : e1;
-  if (e2 != cudaSuccess) {
-    snprintf(g_ctail_why, sizeof(g_ctail_why), "attributes: %s", cudaGetErrorString(e2));
-  } else {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(CT_CTAS);
-    cfg.blockDim = dim3(32, TAIL_THREADS / 32);
-    cfg.dynamicSmemBytes = CT_SMEM_MAX;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = CT_CTAS;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    int nclusters = 0;
-    cudaError_t e3 = cudaOccupancyMaxActiveClusters(&nclusters, k_mg_ctail, &cfg);
-    g_ctail_ok = e3 == cudaSuccess && nclusters >= 1;
-    if (g_ctail_ok)
-      snprintf(g_ctail_why, sizeof(g_ctail_why), "available (%d clusters of %d blocks)",
-               nclusters, CT_CTAS);
-    else
-      snprintf(g_ctail_why, sizeof(g_ctail_why), "occupancy: %s, %d clusters",
-               cudaGetErrorString(e3), nclusters);
-  }
-  cudaGetLastError();
+  set_tile_attrs<float, float, false>();
+  set_tile_attrs<__half, __half, false>();
+  set_tile_attrs<__nv_bfloat16, __nv_bfloat16, false>();
+  // the tolerance hierarchy: FP32 level 0 over FP32 or 16-bit coarse levels
+  set_tile_attrs<float, float, true>();
+  set_tile_attrs<__half, __half, true>();
+  set_tile_attrs<__nv_bfloat16, __nv_bfloat16, true>();
+  set_tile_attrs<float, __half, true>();
+  set_tile_attrs<float, __nv_bfloat16, true>();
+  set_smem_attr(k_tile_m<true, 2, tile::kWarps>, tile::Mem<2, tile::kWarps>::bytes);
+  set_smem_attr(k_tile_m<true, 4, tile::kWarps>, tile::Mem<4, tile::kWarps>::bytes);
+  set_smem_attr(k_tile_m<false, 2, tile::kWarps>, tile::Mem<2, tile::kWarps>::bytes);
+  set_smem_attr(k_tile_m<false, 4, tile::kWarps>, tile::Mem<4, tile::kWarps>::bytes);
+  set_smem_attr(k_mg<40, 8, 12, true, 256, float>, Tile<40, 8, 12>::smem(4));
+  set_smem_attr(k_mg<40, 8, 12, true, 256, __half>, Tile<40, 8, 12>::smem(2));
+  set_smem_attr(k_mg<40, 8, 12, true, 256, __nv_bfloat16>, Tile<40, 8, 12>::smem(2));
+  set_smem_attr(k_mg<56, 24, 4, false, 256, float>, Tile<56, 24, 4>::smem(4));
+  set_smem_attr(k_coarse<float>, kCoarseSmemMax);
+  set_smem_attr(k_coarse<__half>, kCoarseSmemMax);
+  set_smem_attr(k_coarse<__nv_bfloat16>, kCoarseSmemMax);
+  set_smem_attr(k_coarse_m, kCoarseSmemMax);
+  set_smem_attr(k_mg_tail<float, float>, TAIL_SMEM_MAX);
+  set_smem_attr(k_mg_tail<__half, float>, TAIL_SMEM_MAX);
+  set_smem_attr(k_mg_tail<__nv_bfloat16, float>, TAIL_SMEM_MAX);
+  set_smem_attr(k_mg_tail<__half, double>, TAIL_SMEM_MAX);
+  set_smem_attr(k_mg_tail<__nv_bfloat16, double>, TAIL_SMEM_MAX);
+  set_smem_attr(k_mg_tail_m, TAIL_SMEM_MAX);
 }
 
 void init_kernel_attributes() {
@@ -1610,63 +1008,62 @@ void init_kernel_attributes() {
   (void)done;
 }
 
-// 3 sweeps with an optional restriction epilogue need HALO >= 8; the tile
-// is chosen by level width so small levels still fill the GPU.
-// Smoother tiles the autotuner chooses from (3-sweep launches need a halo of
-// 8, 5-sweep launches 12): id -> TX x TY, halo, threads.
-constexpr int kTiles = 6;
-const char *const kTileNames[kTiles] = {"112x50/h8/512", "48x16/h8/256", "40x8/h12/256",
-                                        "112x24/h8/256", "48x40/h8/256", "112x114/h8/1024"};
-bool tile_ok(int id, int nsweeps) { return id >= 0 && id < kTiles && (nsweeps <= 3 || id == 2); }
+// The smoother's regions, by rows of a warp (16 warps): id 0 = 4 rows (128 x
+// 64 cells, 112 x 48 stored), id 1 = 2 rows (128 x 32, 112 x 16).  The taller
+// region recomputes less; the shorter one gives a level of up to 1200 columns
+// more blocks, each with half the rows to go through per half sweep (512x256:
+// 8.5 against 10.0 us).  The autotuner tries both on every level.
+constexpr int kTiles = 2;
+const char *const kTileNames[kTiles] = {"128x64", "128x32"};
+constexpr int kTileRows[kTiles] = {4, 2};
+int tile_for(int w, int choice) { return choice >= 0 && choice < kTiles ? choice : (w >= 1200 ? 0 : 1); }
 
-template <class S>
-void launch_mg_tile(const MgArgsT<S> &a, int id, cudaStream_t st) {
-  switch (id) {
-    case 0: launch_mg_t<112, 50, 8, true, 512, S>(a, st); break;
-    case 1: launch_mg_t<48, 16, 8, true, 256, S>(a, st); break;
-    case 2: launch_mg_t<40, 8, 12, true, 256, S>(a, st); break;
-    case 3: launch_mg_t<112, 24, 8, true, 256, S>(a, st); break;
-    case 4: launch_mg_t<48, 40, 8, true, 256, S>(a, st); break;
-    case 5: launch_mg_t<112, 114, 8, true, 1024, S>(a, st); break;
-    default: throw ArgError("smoother tile id");
-  }
+template <class S, class SC>
+int tile_blocks(const MgArgsT<S, SC> &a, int id) {
+  const bool pre = a.rc != nullptr;
+  return tile::regions(pre ? std::max(a.w, 2 * a.cw) : a.w, 128) *
+         tile::regions(pre ? std::max(a.h, 2 * a.ch) : a.h, kTileRows[id] * tile::kWarps);
 }
 
-// An FP32 level over 16-bit coarse arrays (the tolerance solver's level 0):
-// 3 sweeps, tile by level width.
-template <class SC>
-void launch_mg_mixed_top(const MgArgsT<float, SC> &a, cudaStream_t st) {
-  if (!ALPHA_IS_ONE(a.alpha) || a.nsweeps < 1 || a.nsweeps > 3)
-    throw ArgError("mixed top level: alpha = 1, at most 3 sweeps");
-  if (a.w >= 1200)
-    launch_mg_t<112, 50, 8, true, 512, float, SC>(a, st);
-  else
-    launch_mg_t<48, 16, 8, true, 256, float, SC>(a, st);
+template <class S, class SC, bool EXT, bool PRE, int R>
+void launch_tile_t(const MgArgsT<S, SC> &a, int blocks, cudaStream_t st) {
+  launch_pdl(k_tile<S, SC, EXT, PRE, R, tile::kWarps>, dim3(blocks), dim3(32 * tile::kWarps),
+             tile::Mem<R, tile::kWarps>::bytes, st, a);
+  UBG_LAUNCH_CHECK();
+  g_stats.launches++;
 }
-
-template <class S>
-void launch_mg(const MgArgsT<S> &a, cudaStream_t st) {
-  if (ALPHA_IS_ONE(a.alpha) && a.nsweeps > 1 && a.nsweeps <= 5 && tile_ok(a.tile, a.nsweeps)) {
-    launch_mg_tile(a, a.tile, st);
-    return;
-  }
-  if (!ALPHA_IS_ONE(a.alpha) || a.nsweeps == 1) {
-    if constexpr (std::is_same<S, float>::value) {
-      if (a.nsweeps != 1) throw ArgError("general alpha: one sweep per launch");
-      launch_mg_t<56, 24, 4, false>(a, st);
+// Three sweeps with residual and restriction (a.rc) or with prolongation and
+// correction first (a.ec).
+template <class S, class SC>
+void launch_tile(const MgArgsT<S, SC> &a, cudaStream_t st) {
+  if (!ALPHA_IS_ONE(a.alpha) || a.nsweeps != 3 || (a.rc != nullptr) == (a.ec != nullptr))
+    throw ArgError("smoothing launch: alpha = 1, three sweeps, one transfer");
+  const int id = tile_for(a.w, a.tile), nb = tile_blocks(a, id);
+  auto go = [&](auto ext) {
+    constexpr bool EXT = decltype(ext)::value;
+    if (a.rc) {
+      if (id == 0)
+        launch_tile_t<S, SC, EXT, true, 4>(a, nb, st);
+      else
+        launch_tile_t<S, SC, EXT, true, 2>(a, nb, st);
+    } else if (id == 0) {
+      launch_tile_t<S, SC, EXT, false, 4>(a, nb, st);
     } else {
-      throw ArgError("16-bit smoother: alpha = 1 only");
+      launch_tile_t<S, SC, EXT, false, 2>(a, nb, st);
     }
-  } else if (a.nsweeps <= 3) {
-    if (a.w >= 1200)
-      launch_mg_t<112, 50, 8, true, 512, S>(a, st);
-    else
-      launch_mg_t<48, 16, 8, true, 256, S>(a, st);
-  } else if (a.nsweeps <= 5) {
-    launch_mg_t<40, 8, 12, true, 256, S>(a, st);
-  } else {
-    throw ArgError("smoother: at most 5 sweeps per launch");
-  }
+  };
+  if (a.ext)
+    go(std::true_type{});
+  else if constexpr (std::is_same<S, SC>::value)
+    go(std::false_type{});
+  else
+    throw ArgError("mixed storage types only in the tolerance hierarchy");
+}
+
+// The coarsest level's five sweeps where no tail covers it.
+template <class S>
+void launch_coarsest(const MgArgsT<S> &a, cudaStream_t st) {
+  launch_mg_t<40, 8, 12, true, 256, S>(a, st);
 }
 
 MgArgs level_args(MgLevel &L, const float *in, float *out, int ns, float alpha) {
@@ -1763,122 +1160,59 @@ void run_tail_t(MgHier &mg, int lt, const S *rhs_top, S *e_top, const float *rfa
   g_stats.launches++;
 }
 
-void run_tail(MgHier &mg, int lt, cudaStream_t st) {
-  run_tail_t<float, float>(mg, lt, mg.lv[lt].rhs, mg.lv[lt].e[0], nullptr, st);
-}
-
-// Arguments of the cluster coarse solve from level ct (banded levels ct ..
-// tail_top-1, the tail below); false if the hierarchy or the shared memory
-// does not allow it.
-bool ctail_args(MgHier &mg, int ct, CTailArgs &a, size_t &smem) {
-  const int T = mg.tail_top;
-  if (mg.ext || ct < 1 || T < 2 || ct >= T || T - ct > CT_MAXD || T > mg_coarsest(mg))
-    return false;
-  constexpr int C = CT_CTAS;
-  if (mg.lv[T].h < C) return false;
-  for (int l = ct; l < T; l++)
-    if (mg.lv[l + 1].h != mg.lv[l].h / 2 || mg.lv[l + 1].w != mg.lv[l].w / 2) return false;
-  a = CTailArgs{};
-  size_t tsm = 0;
-  try {
-    a.tail = tail_args<float, float>(mg, T, nullptr, nullptr, nullptr, &tsm);
-  } catch (const ArgError &) {
-    return false;
+// Arguments of the coarse end of the V-cycle from level lt on (scaled: the
+// h^2-scaled form of 16-bit levels, hh = 1 and restriction weights rfac).
+template <class S>
+coarse::Args<S> coarse_args(MgHier &mg, int lt, const S *rhs_top, S *e_top, const float *rfac,
+                            size_t *smem_out) {
+  coarse::Args<S> a{};
+  const int nl = mg_coarsest(mg) + 1 - lt;
+  a.nlev = nl;
+  a.ext = mg.ext ? 1 : 0;
+  a.ncoarse = mg.ncoarse;
+  size_t off = coarse::kLevels;
+  for (int t = 0; t < nl; t++) {
+    MgLevel &L = mg.lv[lt + t];
+    coarse::Level &C = a.L[t];
+    C.w = L.w;
+    C.h = L.h;
+    C.lanes = (L.w + 3) / 4;
+    C.hh = rfac ? 1.0f : L.hh;
+    C.ihsq = rfac ? 1.0f : 1.0f / L.hh / L.hh;
+    C.rfac = rfac ? rfac[lt + t] : 1.0f / 16.0f;
+    const size_t n = (size_t)C.lanes * C.h;
+    C.oe = (int)off;
+    C.of = (int)(off + 16 * n);
+    C.oc = (int)(off + 32 * n);
+    off = (off + 36 * n + 15) / 16 * 16;
+    C.code = L.code;
+    C.code_pitch = L.pitch;
   }
-  a.nd = T - ct;
-  // bands: the tail's top level split evenly, each finer level's bands the
-  // doubled ones (the last block takes the extra rows of odd heights)
-  const int hT = mg.lv[T].h;
-  for (int k = 0; k < C; k++) a.tband[k] = (int)(((long long)k * hT) / C);
-  a.tband[C] = hT;
-  const int *next = a.tband;
-  for (int d = a.nd - 1; d >= 0; d--) {
-    CtLevel &D = a.D[d];
-    const MgLevel &L = mg.lv[ct + d];
-    for (int k = 0; k < C; k++) D.band[k] = 2 * next[k];
-    D.band[C] = L.h;
-    int rows = 0;
-    for (int k = 0; k < C; k++) {
-      if (D.band[k + 1] <= D.band[k]) return false;
-      rows = std::max(rows, D.band[k + 1] - D.band[k]);
-    }
-    D.rows = rows + 2;
-    D.w = L.w;
-    D.h = L.h;
-    D.hh = L.hh;
-    D.ihsq = 1.0f / L.hh / L.hh;
-    D.rfac = 1.0f / 16.0f;
-    D.code = L.code;
-    D.code_pitch = L.pitch;
-    next = D.band;
-  }
-  size_t fo = 0, bo = 0;
-  for (int d = 0; d < a.nd; d++) {
-    CtLevel &D = a.D[d];
-    const size_t n = (size_t)D.rows * D.w;
-    D.oe = (int)fo;
-    fo += (n + 3) / 4 * 4;
-    D.orr = (int)fo;
-    fo += (n + 3) / 4 * 4;
-    D.orhs = (int)fo;
-    fo += (n + 3) / 4 * 4;
-    D.oc = (int)bo;
-    bo += (n + 15) / 16 * 16;
-  }
-  a.tail_fo = (int)fo;
-  fo += (size_t)a.tail.float_words;
-  a.tail_bo = (int)bo;
-  bo += tsm - (size_t)a.tail.float_words * sizeof(float);
-  a.float_words = (int)fo;
-  smem = fo * sizeof(float) + bo;
-  if (smem > CT_SMEM_MAX) return false;
-  const MgLevel &top = mg.lv[ct];
-  a.rhs_top = top.rhs;
+  if (off > kCoarseSmemMax) throw ArgError("coarse levels exceed the shared memory of a block");
+  MgLevel &top = mg.lv[lt];
+  a.rhs_top = rhs_top;
   a.rhs_pitch = top.pitch;
-  a.e_top = top.e[0];
+  a.e_top = e_top;
   a.e_pitch = top.pitch;
   for (int k = 0; k < 5; k++) {
     a.wsum[k] = (float)((double)(float)k + 0.0001);
     a.rwsum[k] = 1.0f / a.wsum[k];
   }
-  return true;
+  *smem_out = off;
+  return a;
 }
 
-// The lowest level from which the cluster coarse solve covers the rest of
-// the V-cycle, or -1.
-int choose_cluster(MgHier &mg) {
-  init_kernel_attributes();
-  if (!g_ctail_ok) return -1;
-  int best = -1;
-  for (int ct = mg.tail_top - 1; ct >= 1; ct--) {
-    CTailArgs a;
-    size_t smem = 0;
-    if (!ctail_args(mg, ct, a, smem)) break;
-    best = ct;
+template <class S>
+void run_coarse(MgHier &mg, int lt, const S *rhs_top, S *e_top, const float *rfac,
+                cudaStream_t st) {
+  if (mg.tail_wide) {
+    run_tail_t<S, float>(mg, lt, rhs_top, e_top, rfac, st);
+    return;
   }
-  return best;
-}
-
-void run_ctail(MgHier &mg, int ct, cudaStream_t st) {
   ProfScope ps_(KC_TAIL, st);
-  CTailArgs a;
   size_t smem = 0;
-  if (!ctail_args(mg, ct, a, smem)) throw ArgError("cluster coarse solve: hierarchy does not fit");
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(CT_CTAS);
-  cfg.blockDim = dim3(32, TAIL_THREADS / 32);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute at[2];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = CT_CTAS;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
-  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 2;
-  UBG_CUDA(cudaLaunchKernelEx(&cfg, k_mg_ctail, a));
+  const coarse::Args<S> a = coarse_args<S>(mg, lt, rhs_top, e_top, rfac, &smem);
+  launch_pdl(k_coarse<S>, dim3(1), dim3(32 * coarse::kWarps), smem, st, a);
   UBG_LAUNCH_CHECK();
   g_stats.launches++;
 }
@@ -1887,13 +1221,8 @@ void run_ctail(MgHier &mg, int ct, cudaStream_t st) {
 void solve_level(MgHier &mg, std::vector<int> &cur, int l, bool zgbc, cudaStream_t st) {
   bool bc = zgbc && l == 0;
   MgLevel &L = mg.lv[l];
-  if (l >= 1 && l == mg.cluster_top) {
-    run_ctail(mg, l, st);
-    cur[l] = 0;
-    return;
-  }
   if (l >= 1 && l == mg.tail_top) {
-    run_tail(mg, l, st);
+    run_coarse<float>(mg, l, L.rhs, L.e[0], nullptr, st);
     cur[l] = 0;
     return;
   }
@@ -1901,7 +1230,7 @@ void solve_level(MgHier &mg, std::vector<int> &cur, int l, bool zgbc, cudaStream
     ProfScope ps_(l == 0 ? KC_SMOOTH_L0 : (l == 1 ? KC_SMOOTH_L1 : KC_SMOOTH_COARSE), st);
     MgArgs a = level_args(L, L.e[cur[l]], L.e[1 - cur[l]], 5, 1.0f);
     a.zero_init = l > 0;
-    launch_mg(a, st);
+    launch_coarsest(a, st);
     cur[l] ^= 1;
     return;
   }
@@ -1909,6 +1238,7 @@ void solve_level(MgHier &mg, std::vector<int> &cur, int l, bool zgbc, cudaStream
   {
     ProfScope ps_(l == 0 ? KC_SMOOTH_L0 : (l == 1 ? KC_SMOOTH_L1 : KC_SMOOTH_COARSE), st);
     MgArgs a = level_args(L, L.e[cur[l]], L.e[1 - cur[l]], 3, 1.0f);
+    a.zero_edges = l > 0;
     a.zgbc = bc;
     a.zero_init = l > 0;
     a.tile = L.tile_pre;
@@ -1916,13 +1246,14 @@ void solve_level(MgHier &mg, std::vector<int> &cur, int l, bool zgbc, cudaStream
     a.cw = C.w;
     a.ch = C.h;
     a.cpitch = C.pitch;
-    launch_mg(a, st);
+    launch_tile(a, st);
     cur[l] ^= 1;
   }
   solve_level(mg, cur, l + 1, false, st);
   {
     ProfScope ps_(l == 0 ? KC_SMOOTH_L0 : (l == 1 ? KC_SMOOTH_L1 : KC_SMOOTH_COARSE), st);
     MgArgs a = level_args(L, L.e[cur[l]], L.e[1 - cur[l]], 3, 1.0f);
+    a.zero_edges = l > 0;
     a.zgbc = bc;
     a.tile = L.tile_post;
     a.ec = C.e[cur[l + 1]];
@@ -1930,8 +1261,7 @@ void solve_level(MgHier &mg, std::vector<int> &cur, int l, bool zgbc, cudaStream
     a.cpitch = C.pitch;
     a.cw = C.w;
     a.ch = C.h;
-    if (l == 0) a.norm2 = mg.post_norm2;
-    launch_mg(a, st);
+    launch_tile(a, st);
     cur[l] ^= 1;
   }
 }
@@ -2180,7 +1510,7 @@ void solve_level_lo(MgHier &mg, MgLow &lo, std::vector<int> &cur, int l, cudaStr
     MgArgsT<S> a = level_args_lo<S>(mg, lo, l, cur[l], 5);
     a.zero_init = 1;
     a.zgbc = l == 0;
-    launch_mg(a, st);
+    launch_coarsest(a, st);
     cur[l] ^= 1;
     return;
   }
@@ -2188,6 +1518,7 @@ void solve_level_lo(MgHier &mg, MgLow &lo, std::vector<int> &cur, int l, cudaStr
   {
     ProfScope ps_(kc, st);
     MgArgsT<S> a = level_args_lo<S>(mg, lo, l, cur[l], 3);
+    a.zero_edges = l > 0;
     a.zero_init = 1;
     a.zgbc = l == 0;
     a.tile = mg.lv[l].tile_pre;
@@ -2195,13 +1526,14 @@ void solve_level_lo(MgHier &mg, MgLow &lo, std::vector<int> &cur, int l, cudaStr
     a.cw = C.w;
     a.ch = C.h;
     a.cpitch = C.pitch;
-    launch_mg(a, st);
+    launch_tile(a, st);
     cur[l] ^= 1;
   }
   solve_level_lo<S>(mg, lo, cur, l + 1, st);
   {
     ProfScope ps_(kc, st);
     MgArgsT<S> a = level_args_lo<S>(mg, lo, l, cur[l], 3);
+    a.zero_edges = l > 0;
     a.zgbc = l == 0;
     a.tile = mg.lv[l].tile_post;
     a.ec = (const S *)lo.e[cur[l + 1]][l + 1];
@@ -2209,7 +1541,7 @@ void solve_level_lo(MgHier &mg, MgLow &lo, std::vector<int> &cur, int l, cudaStr
     a.cpitch = C.pitch;
     a.cw = C.w;
     a.ch = C.h;
-    launch_mg(a, st);
+    launch_tile(a, st);
     cur[l] ^= 1;
   }
 }
@@ -2275,27 +1607,33 @@ int solve_mixed_t(MgHier &mg, MgLow &lo, double tol, int max_cycles, double fnor
 
 size_t align256(size_t v) { return (v + 255) / 256 * 256; }
 
-// The first level whose whole coarse end fits the tail kernel (arithmetic
-// elements of elem_bytes: 4 for FP32, 8 for the mixed solver's FP64) with a
-// top level of at most max_cells.
-int choose_tail(const std::vector<MgLevel> &lv, int max_cells, size_t elem_bytes = 4,
-                int last = -1) {
-  int L = (int)lv.size();
-  if (last < 0) last = L - 2;
-  for (int lt = 1; lt <= last; lt++) {
+// The first level whose whole coarse end fits the tail kernel of any shape
+// (arithmetic elements of elem_bytes) with a top level of at most max_cells.
+int choose_tail_any(const std::vector<MgLevel> &lv, int max_cells, size_t elem_bytes, int last) {
+  for (int lt = 1; lt <= last; lt++)
     if (tail_smem_bytes(lv, lt, elem_bytes, last) <= TAIL_SMEM_MAX &&
         (size_t)lv[lt].w * lv[lt].h <= (size_t)max_cells)
       return lt;
-  }
   return -1;
+}
+// The first level from which the coarse solve in registers (levels of at most
+// 128 x 64 cells) covers the rest, with a top level of at most max_cells.
+int choose_tail(const std::vector<MgLevel> &lv, int max_cells, int last) {
+  for (int lt = 1; lt <= last; lt++)
+    if (lv[lt].w <= coarse::kMaxW && lv[lt].h <= coarse::kMaxH && last - lt < coarse::kMaxLevels &&
+        (size_t)lv[lt].w * lv[lt].h <= (size_t)max_cells)
+      return lt;
+  return -1;
+}
+// Sets the hierarchy's tail: the coarse solve in registers, or the kernel of
+// any shape for elongated levels of at most wide_cells.
+void set_tail(MgHier &mg, int last, int wide_cells) {
+  mg.tail_top = choose_tail(mg.lv, mg.tail_cells, last);
+  mg.tail_wide = mg.tail_top < 1;
+  if (mg.tail_wide) mg.tail_top = choose_tail_any(mg.lv, wide_cells, 4, last);
 }
 
 }  // namespace
-
-const char *cluster_coarse_solve_status() {
-  init_kernel_attributes();
-  return g_ctail_why;
-}
 
 namespace {
 std::vector<MgLevel> level_shapes(int W, int H, float h0) {
@@ -2348,18 +1686,10 @@ void mg_bind(MgHier &mg, int W, int H, float h0, void *arena, size_t bytes) {
     p += align256(n);
   }
   mg.norm = (double *)p;
-  mg.post_norm2 = nullptr;
-  mg.tail_top = choose_tail(lv, mg.tail_cells);
-  mg.tail_top_fp64 = choose_tail(lv, 128, 8);
+  mg.tail_top_fp64 = choose_tail_any(lv, 128, 8, (int)lv.size() - 2);
   mg.lv = lv;
   mg.levels = (int)lv.size();
-  // the cluster coarse solve from two levels above the tail (the autotuner
-  // measured that choice fastest at 1024x512, 4096x2048 and 8192x4096;
-  // from larger levels its 16 blocks have too much work per phase)
-  {
-    const int lowest = choose_cluster(mg);
-    mg.cluster_top = lowest >= 1 ? std::max(lowest, mg.tail_top - 2) : -1;
-  }
+  set_tail(mg, mg.levels - 2, 2048);
   mg.arena = nullptr;  // not owned
   mg.arena_bytes = bytes;
   mg.cur0 = 0;
@@ -2476,7 +1806,7 @@ double time_ms(EvPair &ev, cudaStream_t st, int warm, int reps, F &&f) {
 // simulations of one size (the members of a batch, the sessions of a
 // server) share the first one's trials.
 struct TuneChoice {
-  int tail_cells = 0, tail_top = 0, cluster_top = -1;
+  int tail_cells = 0, tail_top = 0;
   std::vector<int> pre, post;
 };
 std::mutex g_tune_mu;
@@ -2492,7 +1822,6 @@ void mg_autotune(MgHier &mg, cudaStream_t st, std::string *report) {
     if (it != g_tune_cache.end() && (int)it->second.pre.size() == nl) {
       mg.tail_cells = it->second.tail_cells;
       mg.tail_top = it->second.tail_top;
-      mg.cluster_top = it->second.cluster_top;
       for (int l = 0; l < nl; l++) {
         mg.lv[l].tile_pre = it->second.pre[l];
         mg.lv[l].tile_post = it->second.post[l];
@@ -2500,8 +1829,8 @@ void mg_autotune(MgHier &mg, cudaStream_t st, std::string *report) {
       if (report) {
         char buf[160];
         snprintf(buf, sizeof(buf),
-                 "{\"cached\": true, \"tail_cells\": %d, \"tail_top\": %d, \"cluster_top\": %d, \"levels\": [",
-                 mg.tail_cells, mg.tail_top, mg.cluster_top);
+                 "{\"cached\": true, \"tail_cells\": %d, \"tail_top\": %d, \"cluster_top\": -1, \"levels\": [",
+                 mg.tail_cells, mg.tail_top);
         std::string rep = buf;
         const int last = (mg.tail_top >= 1 ? mg.tail_top : nl - 1) - 1;
         for (int l = 0; l <= std::min(last, nl - 3); l++) {
@@ -2547,9 +1876,6 @@ void mg_autotune(MgHier &mg, cudaStream_t st, std::string *report) {
     cudaGraphExecDestroy(ge);
     return 1e3 * ms;
   };
-  // the tail and the tiles are tuned with launches per level; the cluster
-  // coarse solve is tried last
-  mg.cluster_top = -1;
   std::string rep = "{\"trials\": [";
   bool first = true;
   auto note = [&](const char *what, int level, const char *choice, double us) {
@@ -2562,10 +1888,10 @@ void mg_autotune(MgHier &mg, cudaStream_t st, std::string *report) {
   double best = vcycle_us();
   note("start", -1, "default", best);
   // tail size
-  const int tail_cand[] = {512, 1024, 2048, 4096, 8192};
+  const int tail_cand[] = {512, 2048, 8192};
   int best_tc = mg.tail_cells, best_lt = mg.tail_top;
   for (int tc : tail_cand) {
-    int lt = choose_tail(mg.lv, tc);
+    int lt = mg.tail_wide ? -1 : choose_tail(mg.lv, tc, nl - 2);
     if (lt < 1 || lt == best_lt) continue;
     int keep = mg.tail_top;
     mg.tail_top = lt;
@@ -2602,27 +1928,12 @@ void mg_autotune(MgHier &mg, cudaStream_t st, std::string *report) {
       slot = keep;
     }
   }
-  {
-    // every feasible first level of the cluster coarse solve
-    const int lowest = choose_cluster(mg);
-    int keep = -1;
-    for (int ct = mg.tail_top - 1; lowest >= 1 && ct >= lowest; ct--) {
-      mg.cluster_top = ct;
-      double t = vcycle_us();
-      note("cluster", ct, "on", t);
-      if (t < best) {
-        best = t;
-        keep = ct;
-      }
-    }
-    mg.cluster_top = keep;
-  }
   UBG_CUDA(cudaMemcpyAsync(L0.e[c0], saved, pbytes, cudaMemcpyDeviceToDevice, st));
   UBG_CUDA(cudaStreamSynchronize(st));
   cudaFree(saved);
   char buf[256];
-  snprintf(buf, sizeof(buf), "], \"vcycle_us\": %.2f, \"tail_cells\": %d, \"tail_top\": %d, \"cluster_top\": %d, \"levels\": [",
-           best, mg.tail_cells, mg.tail_top, mg.cluster_top);
+  snprintf(buf, sizeof(buf), "], \"vcycle_us\": %.2f, \"tail_cells\": %d, \"tail_top\": %d, \"cluster_top\": -1, \"levels\": [",
+           best, mg.tail_cells, mg.tail_top);
   rep += buf;
   for (int l = 0; l <= std::min(last, nl - 3); l++) {
     const MgLevel &L = mg.lv[l];
@@ -2636,7 +1947,6 @@ void mg_autotune(MgHier &mg, cudaStream_t st, std::string *report) {
   TuneChoice tc;
   tc.tail_cells = mg.tail_cells;
   tc.tail_top = mg.tail_top;
-  tc.cluster_top = mg.cluster_top;
   for (int l = 0; l < nl; l++) {
     tc.pre.push_back(mg.lv[l].tile_pre);
     tc.post.push_back(mg.lv[l].tile_post);
@@ -2716,15 +2026,6 @@ int mg_solve_mixed(MgHier &mg, MgLow &lo, double tol, int max_cycles, double fno
 
 // ------------------------------------------------- fused batch V-cycle
 namespace {
-int tile_for(const MgLevel &L, int choice) {
-  if (tile_ok(choice, 3)) return choice;
-  return L.w >= 1200 ? 0 : 1;  // the width rule of launch_mg for 3 sweeps
-}
-int tile_tx(int id) { return id == 0 || id == 3 || id == 5 ? 112 : (id == 2 ? 40 : 48); }
-int tile_ty(int id) {
-  const int ty[kTiles] = {50, 16, 8, 24, 40, 114};
-  return ty[id];
-}
 template <class A>
 void slot_add(MultiSlot &s, const A &a, int blocks) {
   const char *p = reinterpret_cast<const char *>(&a);
@@ -2771,32 +2072,39 @@ void mg_multi_vcycle(const std::vector<MgHier *> &mgs, std::vector<MultiSlot> &o
         a.cw = C.w;
         a.ch = C.h;
       }
-      const int id = tile_for(L, pre ? L.tile_pre : L.tile_post);
-      a.tile = id;
+      a.zero_edges = l > 0;
+      const int id = tile_for(L.w, pre ? L.tile_pre : L.tile_post);
       MultiSlot &sl = by_tile[id];
       sl.kind = MK_MG;
-      sl.tile = id;
-      const int tx = tile_tx(id), ty = tile_ty(id);
-      slot_add(sl, a, ((L.w + tx - 1) / tx) * ((L.h + ty - 1) / ty));
+      sl.tile = 2 * id + (pre ? 0 : 1);
+      slot_add(sl, a, tile_blocks(a, id));
       cur[i][l] ^= 1;
     }
     for (auto &kv : by_tile) out.push_back(std::move(kv.second));
   };
   for (int l = 0; l < maxt; l++) level_slots(l, true);
-  {
+  for (int wide = 0; wide < 2; wide++) {
     MultiSlot sl;
     sl.kind = MK_TAIL;
+    sl.tile = wide;
     for (int i = 0; i < n; i++) {
       MgHier &mg = *mgs[i];
+      if ((int)mg.tail_wide != wide) continue;
       const int lt = mg.tail_top;
       size_t smem = 0;
-      TailArgs<float> a = tail_args<float, float>(mg, lt, mg.lv[lt].rhs, mg.lv[lt].e[0], nullptr,
-                                                  &smem);
+      if (wide) {
+        const TailArgs<float> a =
+            tail_args<float, float>(mg, lt, mg.lv[lt].rhs, mg.lv[lt].e[0], nullptr, &smem);
+        slot_add(sl, a, 1);
+      } else {
+        const coarse::Args<float> a =
+            coarse_args<float>(mg, lt, mg.lv[lt].rhs, mg.lv[lt].e[0], nullptr, &smem);
+        slot_add(sl, a, 1);
+      }
       sl.smem = std::max(sl.smem, smem);
-      slot_add(sl, a, 1);
       cur[i][lt] = 0;
     }
-    out.push_back(std::move(sl));
+    if (sl.n) out.push_back(std::move(sl));
   }
   for (int l = maxt - 1; l >= 0; l--) level_slots(l, false);
   for (int i = 0; i < n; i++)
@@ -2805,24 +2113,24 @@ void mg_multi_vcycle(const std::vector<MgHier *> &mgs, std::vector<MultiSlot> &o
 
 void launch_multi_mg(const MultiSlot &slot, const void *dargs, const int *dbs, unsigned tag,
                      unsigned *err, cudaStream_t st) {
-  if (slot.kind == MK_TAIL) {
+  if (slot.kind == MK_TAIL && slot.tile) {
     launch_pdl(k_mg_tail_m, dim3(slot.n), dim3(32, 32), slot.smem, st,
                (const TailArgs<float> *)dargs, dbs, slot.n, tag, err);
+  } else if (slot.kind == MK_TAIL) {
+    launch_pdl(k_coarse_m, dim3(slot.n), dim3(32 * coarse::kWarps), slot.smem, st,
+               (const coarse::Args<float> *)dargs, dbs, slot.n, tag, err);
   } else {
     const MgArgs *A = (const MgArgs *)dargs;
+    auto go = [&](auto *k, int rows) {
+      launch_pdl(k, dim3(slot.blocks), dim3(32 * tile::kWarps),
+                 rows == 4 ? tile::Mem<4, tile::kWarps>::bytes : tile::Mem<2, tile::kWarps>::bytes,
+                 st, A, dbs, slot.n, tag, err);
+    };
     switch (slot.tile) {
-#define UBG_MULTI_TILE(ID, TX, TY, HALO, NT)                                                   \
-  case ID:                                                                                     \
-    launch_pdl(k_mg_m<TX, TY, HALO, true, NT>, dim3(slot.blocks), dim3(32, NT / 32),          \
-               Tile<TX, TY, HALO>::smem(4), st, A, dbs, slot.n, tag, err);                     \
-    break;
-      UBG_MULTI_TILE(0, 112, 50, 8, 512)
-      UBG_MULTI_TILE(1, 48, 16, 8, 256)
-      UBG_MULTI_TILE(2, 40, 8, 12, 256)
-      UBG_MULTI_TILE(3, 112, 24, 8, 256)
-      UBG_MULTI_TILE(4, 48, 40, 8, 256)
-      UBG_MULTI_TILE(5, 112, 114, 8, 1024)
-#undef UBG_MULTI_TILE
+      case 0: go(k_tile_m<true, 4, tile::kWarps>, 4); break;
+      case 1: go(k_tile_m<false, 4, tile::kWarps>, 4); break;
+      case 2: go(k_tile_m<true, 2, tile::kWarps>, 2); break;
+      case 3: go(k_tile_m<false, 2, tile::kWarps>, 2); break;
       default:
         throw ArgError("fused batch: smoother tile id");
     }
@@ -3008,10 +2316,7 @@ void ext_vcycle_t(MgHier &mg, MgLow *lo, const unsigned *scale_bits, cudaStream_
   };
   auto launch_top = [&](const MgArgsT<float, SC> &a) {
     ProfScope ps_(KC_SMOOTH_L0, st);
-    if constexpr (scaled)
-      launch_mg_mixed_top<SC>(a, st);
-    else
-      launch_mg(a, st);
+    launch_tile(a, st);
   };
   // down
   {
@@ -3029,12 +2334,12 @@ void ext_vcycle_t(MgHier &mg, MgLow *lo, const unsigned *scale_bits, cudaStream_
     a.cw = mg.lv[l + 1].w;
     a.ch = mg.lv[l + 1].h;
     a.cpitch = mg.lv[l + 1].pitch;
-    launch_mg(a, st);
+    launch_tile(a, st);
     cur[l] ^= 1;
   }
   {
     std::vector<float> rf(mg.levels, 0.25f);
-    run_tail_t<SC, float>(mg, T, rhs(T), arr(T, 0), scaled ? rf.data() : nullptr, st);
+    run_coarse<SC>(mg, T, rhs(T), arr(T, 0), scaled ? rf.data() : nullptr, st);
     cur[T] = 0;
   }
   // up
@@ -3046,7 +2351,7 @@ void ext_vcycle_t(MgHier &mg, MgLow *lo, const unsigned *scale_bits, cudaStream_
     a.cpitch = mg.lv[l + 1].pitch;
     a.cw = mg.lv[l + 1].w;
     a.ch = mg.lv[l + 1].h;
-    launch_mg(a, st);
+    launch_tile(a, st);
     cur[l] ^= 1;
   }
   {
@@ -3096,12 +2401,11 @@ void ext_hier_alloc(MgHier &mg, int W, int H, float h0) {
     p += align256(n);
   }
   mg.norm = (double *)p;
-  mg.post_norm2 = nullptr;
   mg.ext = true;
   mg.ncoarse = 16;
   mg.lv = lv;
   mg.levels = (int)lv.size();
-  mg.tail_top = choose_tail(lv, 4096, 4, mg.levels - 1);
+  set_tail(mg, mg.levels - 1, 4096);
   if (mg.tail_top < 1) mg.tail_top = mg.levels - 1;
   mg.tail_top_fp64 = -1;
   mg.arena = arena;

@@ -1,0 +1,603 @@
+// The smoothing launch of the multigrid on tiles held in registers (included
+// by k_mg.cu, which defines the stencil codes and the launch arguments).
+//
+// A block of NW warps owns a region of 128 columns x NW * R rows: a warp R
+// consecutive rows, a lane 4 columns of them, as the column pairs (0, 2) and
+// (1, 3).  p and f h^2 stay in registers over the three red-black sweeps: the
+// neighbours in a row come from the next lane by shuffle, those above and
+// below are the lane's own registers, and only a warp's first and last row go
+// through shared memory, one barrier per half sweep.  A half sweep updates
+// one pair of every row, so its sums are packed FP32 additions.
+//
+// A solid cell holds 0, so a sum needs no flag tests: the flags only decide
+// what it is divided by.  A warp whose cells and all their neighbours are
+// fluid takes val / 4; any other reads two factors per cell (s = 1/n and its
+// correction for n = 3) from shared memory, where the block put them when it
+// loaded the codes.
+//
+// After half sweep i, the cells within i of the region's edge are no longer
+// exact, so regions overlap by 16 columns and rows and store what is 8 or
+// more inside (all of it at the domain's edge).
+//
+// What bounds it: instruction issue and the FP32 pipe on large levels, the
+// latency of loads, six barriers and one pass through the code on small ones.
+// Against tiles in shared memory (red/black-split, 112 x 50 and 48 x 16
+// cells), ncu: level 0 of 4096x2048 58 us (89 with the residual, 98 with the
+// prolongation), 2048x1024 18 us (33, 38), 1024x512 8 us (18, 20), 256x128
+// 6 us.
+#pragma once
+
+namespace ubg {
+namespace {
+namespace tile {
+
+constexpr int kHalo = 8;
+constexpr int kWarps = 16;
+constexpr float kThird = 1.0f / 3.0f;
+constexpr unsigned kFull = 0x1f1f1f1fu;
+
+// Regions of n cells each with an overlap of 2 * kHalo that cover c cells.
+__host__ __device__ constexpr int regions(int c, int n) {
+  return c <= n ? 1 : (c - 2 * kHalo + n - 2 * kHalo - 1) / (n - 2 * kHalo);
+}
+// Shared memory: factors (16 bytes per pair), exchanged rows, table of
+// factors by code and of the prolongation's weight sums.
+constexpr int kLutBytes = (64 + 5) * 8;
+template <int R, int NW>
+struct Mem {
+  static constexpr int fac = 0, xch = fac + R * NW * 1024, res = xch + 2 * NW * 512,
+                       lut = res + NW * 256, bytes = lut + kLutBytes;
+};
+
+// Two operations in one instruction, each lane rounded as its scalar form.
+// No product is added by add2: ptxas may fuse a packed product with a packed
+// addition.
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 ra, rb, rd;\n\t"
+      "mov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"
+      "add.rn.f32x2 rd, ra, rb;\n\tmov.b64 {%0, %1}, rd;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+// Asynchronous copy of B bytes to shared memory (zeros unless ok).
+template <int B>
+__device__ __forceinline__ void copy_async(void *dst, const void *src, bool ok) {
+  const int n = ok ? B : 0;
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(
+                   (unsigned)__cvta_generic_to_shared(dst)),
+               "l"(src), "n"(B), "r"(n)
+               : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+
+template <class S>
+__device__ __forceinline__ float rnd(float v) {
+  if constexpr (std::is_same<S, float>::value)
+    return v;
+  else
+    return Sto<S>::tof(Sto<S>::fromf(v));
+}
+template <class S>
+__device__ __forceinline__ float2 rnd2(float2 v) {
+  return make_float2(rnd<S>(v.x), rnd<S>(v.y));
+}
+
+// val / n of a pair: s = 1/n (the rounded third for n = 3; 0 for a solid cell
+// or one without fluid neighbours), c = s for n = 3, else 0.  n = 1, 2, 4
+// are exact products; n = 3 is Markstein's correction, whose remainder
+// v - 3 q is exact for every finite v, subnormal results included (3 has two
+// bits).  For finite sums only: 0 * infinity would be NaN.
+__device__ __forceinline__ float2 scaled2(float2 v, float2 s, float2 c) {
+  const float2 q = f2_mul(v, s);
+  return f2_fma(f2_fma(q, f2(-3.0f), v), c, q);
+}
+// The same for any v (a solid cell is 0 whatever its sum).
+__device__ __forceinline__ float scaled_any(float v, float s, float c) {
+  const float q = v * s;
+  const float q3 = __fmaf_rn(__fmaf_rn(-q, 3.0f, v), c, q);
+  const float n = (c != 0.0f && fabsf(v) < __int_as_float(0x7f800000)) ? q3 : q;
+  return s != 0.0f ? n : 0.0f;
+}
+// Magnitude bound under which six (ten) half sweeps stay finite.
+constexpr float kBig = 0x1p+60f;
+
+// Unsigned bits without the sign, less one: a value is 0 (all ones) or its
+// division by div_rn's correction is exact when the key is in [lo, hi] of
+// 2^-100 and 2^100.
+__device__ __forceinline__ unsigned key(float v) {
+  const unsigned u = __float_as_uint(v);
+  return u + u - 1u;
+}
+constexpr unsigned kKeyLo = 2u * 0x0d800000u - 1u, kKeyHi = 2u * 0x71800000u - 1u;
+
+// Fills the table: factors (s, c) by code, 32 + code for a cell that is not
+// smoothed; then the weight sums of the prolongation and their reciprocals.
+__device__ __forceinline__ void fill_lut(float2 *lut, int i, const float *wsum,
+                                         const float *rwsum) {
+  if (i < 64) {
+    const int n = __popc((i >> 1) & 15);
+    float s = n == 4 ? 0.25f : (n == 3 ? kThird : (n == 2 ? 0.5f : (n == 1 ? 1.0f : 0.0f)));
+    if (!(i & (int)C_CENTER) || i >= 32) s = 0.0f;
+    lut[i] = make_float2(s, s == kThird ? s : 0.0f);
+  } else if (i < 69) {
+    lut[i] = make_float2(wsum[i - 64], rwsum[i - 64]);
+  }
+}
+
+// prolongate (pressure_solver.cpp:134-172) onto two rows of a lane's four
+// columns: coarse columns X/2, X/2 + 1 and X/2 + 2 of the coarse row below
+// (e, flags g, one byte each) and the next one (f, g1); the first row lies
+// over the coarse row, the second between the two.  u[row][column].
+__device__ __forceinline__ void prolongate2(const float (&e)[3], const float (&f)[3], unsigned g,
+                                            unsigned g1, const float2 *lut, float (&u)[2][4]) {
+  const float v[6] = {e[0] + e[1],
+                      e[1] + e[2],
+                      e[0] + f[0],
+                      ((e[0] + f[1]) + e[1]) + f[0],
+                      e[1] + f[1],
+                      ((e[1] + f[2]) + e[2]) + f[1]};
+  float2 d[6];
+  if (__all_sync(0xffffffffu, (g & g1) == 0x010101u)) {
+    const float2 d2 = lut[66], d4 = lut[68];
+#pragma unroll
+    for (int i = 0; i < 6; i++) d[i] = i == 3 || i == 5 ? d4 : d2;
+  } else {
+    const unsigned t = g + g1;  // flag sums of the column pairs, a byte each
+    d[0] = lut[64 + (g & 1u) + ((g >> 8) & 1u)];
+    d[1] = lut[64 + ((g >> 8) & 1u) + (g >> 16)];
+    d[2] = lut[64 + (t & 0xffu)];
+    d[3] = lut[64 + (t & 0xffu) + ((t >> 8) & 0xffu)];
+    d[4] = lut[64 + ((t >> 8) & 0xffu)];
+    d[5] = lut[64 + ((t >> 8) & 0xffu) + (t >> 16)];
+  }
+  float q[6];
+  unsigned lo = ~0u;
+  float m = 0.0f;
+#pragma unroll
+  for (int i = 0; i < 6; i++) {  // div_rn's correction
+    const float q0 = v[i] * d[i].y;
+    q[i] = __fmaf_rn(__fmaf_rn(-q0, d[i].x, v[i]), d[i].y, q0);
+    lo = min(lo, key(v[i]));
+    m = m + fabsf(v[i]);
+  }
+  // sums the correction is not exact for (zeros are fine)
+  if (!__all_sync(0xffffffffu, lo >= kKeyLo && m <= 0x1p+100f)) {
+#pragma unroll
+    for (int i = 0; i < 6; i++) q[i] = div_rn(v[i], d[i].x, d[i].y);
+  }
+  u[0][0] = e[0];
+  u[0][1] = q[0];
+  u[0][2] = e[1];
+  u[0][3] = q[1];
+#pragma unroll
+  for (int b = 0; b < 4; b++) u[1][b] = q[2 + b];
+}
+
+// Residuals (calculateResidualField, pressure_solver.cpp:91-116) of a lane's
+// four cells with codes c (center bit clear: 0): values C, W, E, S, N, right
+// hand side F.
+__device__ __forceinline__ void residual4(unsigned c, const float (&C)[4], const float (&W)[4],
+                                          const float (&E)[4], const float (&S)[4],
+                                          const float (&N)[4], const float (&F)[4], float ihsq,
+                                          float (&q)[4]) {
+#pragma unroll
+  for (int b = 0; b < 4; b++) {
+    const unsigned k = c >> (8 * b);
+    const float v = (((((k & C_W) ? W[b] : C[b]) + ((k & C_E) ? E[b] : C[b])) +
+                      ((k & C_S) ? S[b] : C[b])) +
+                     ((k & C_N) ? N[b] : C[b])) +
+                    -4.0f * C[b];
+    q[b] = (k & C_CENTER) ? F[b] + v * ihsq : 0.0f;
+  }
+}
+
+// One region of the level: columns from 112 * sx, rows from (NW * R - 16) * sy.  PRE: residual and restriction (a.rc); else prolongation and
+// correction (a.ec) first.  Red points are those with x + y odd; even rows
+// hold them in the pair (1, 3).
+template <class S, class SC, bool EXT, bool PRE, int R, int NW>
+__device__ __forceinline__ void run(const MgArgsT<S, SC> &a, const int region,
+                                    unsigned char *smem) {
+  static_assert(R % 2 == 0, "row parity");
+  using M = Mem<R, NW>;
+  using St = Sto<S>;
+  using Sc = Sto<SC>;
+  constexpr int RY = R * NW;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int w = a.w, h = a.h;
+  const size_t P = (size_t)a.pitch;
+  const int nsx = regions(PRE ? max(w, 2 * a.cw) : w, 128);
+  const int nsy = regions(PRE ? max(h, 2 * a.ch) : h, RY);
+  const int sx = region % nsx, sy = region / nsx;
+  const int x0 = (128 - 2 * kHalo) * sx, y0 = (RY - 2 * kHalo) * sy;
+  const int X = x0 + 4 * lane, y = y0 + R * wid;  // the lane's first column and row
+  const bool ext = EXT && a.ext != 0, zg = a.zgbc != 0;
+  const bool first = sx == 0, has_east = w - 1 - x0 < 128;
+  // stored columns and rows
+  const bool mine = (lane >= 2 || first) && (lane < 30 || sx == nsx - 1);
+  const int ya = sy == 0 ? 0 : y0 + kHalo, yb = sy == nsy - 1 ? y0 + RY : y0 + RY - kHalo;
+  float4 *const fac = reinterpret_cast<float4 *>(smem + M::fac) + (R * wid) * 64 + lane;
+  float2 *const xch = reinterpret_cast<float2 *>(smem + M::xch) + lane;
+  float2 *const res = reinterpret_cast<float2 *>(smem + M::res) + lane;
+  const float2 *const lut = reinterpret_cast<const float2 *>(smem + M::lut);
+  // exchanged rows: buffer (half sweep parity), warp, its first or last row
+  auto slot = [&](int buf, int wd, int lastrow) -> float2 & {
+    return xch[((buf * NW + wd) * 2 + lastrow) * 32];
+  };
+
+  // ---- loads: all in flight together; f is copied to where the lane's
+  // factors will be (16 registers less while the rest arrives)
+  const bool colok = X < w;
+  float4 pv[R];
+  unsigned cw[R];
+#pragma unroll
+  for (int r = 0; r < R; r++) {
+    const bool ok = colok && y + r < h;
+    const size_t o = ok ? (size_t)(y + r) * P + X : 0;
+    copy_async<4 * (int)sizeof(S)>(fac + r * 64, a.rhs + o, ok);
+    pv[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+    cw[r] = 0u;
+    if (ok) {
+      if (!a.zero_init) pv[r] = St::ldg4(a.in + o);
+      cw[r] = __ldg(reinterpret_cast<const unsigned *>(a.code + o));
+    }
+  }
+  copy_commit();
+  unsigned inmask = 0u;  // columns that are smoothed
+  {
+    unsigned colmask = 0u;
+#pragma unroll
+    for (int b = 0; b < 4; b++) {
+      colmask |= X + b < w ? 0xffu << (8 * b) : 0u;
+      inmask |= X + b >= 1 && X + b < w - 1 ? 0xffu << (8 * b) : 0u;
+    }
+#pragma unroll
+    for (int r = 0; r < R; r++) cw[r] &= colmask;
+  }
+  bool full = true;
+#pragma unroll
+  for (int r = 0; r < R; r++) full = full && cw[r] == kFull;
+  // the warp's rows or columns touch the domain's edge (rows 1 and h-2 too:
+  // their neighbours on the edge follow them); where the edge cells are 0 and
+  // stay so, the factor 0 does it
+  const bool rim = first || has_east || y <= 1 || y + R >= h - 1;
+  const bool wedge = rim && !a.zero_edges;
+  full = __all_sync(0xffffffffu, full) && !rim;
+
+  if constexpr (!PRE) {
+    // ---- prolongate (pressure_solver.cpp:134-172) + correct: an even row
+    // lies over one coarse row, an odd row between two
+    constexpr int RC = R / 2 + 1;
+    const int c0 = X >> 1, cy = y >> 1;
+    float2 ev[RC];
+    unsigned fl[RC];
+#pragma unroll
+    for (int k = 0; k < RC; k++) {
+      ev[k] = make_float2(0.f, 0.f);
+      fl[k] = 0u;
+      if (c0 < a.cw && cy + k < a.ch) {
+        const size_t o = (size_t)(cy + k) * a.cpitch + c0;
+        ev[k] = Sc::ldg2(a.ec + o);
+        fl[k] = __ldg(reinterpret_cast<const unsigned short *>(a.codec + o)) & 0x0101u;
+        if (c0 + 1 >= a.cw) {
+          ev[k].y = 0.0f;
+          fl[k] &= 0x00ffu;
+        }
+      }
+    }
+    float ecmul = 1.0f;
+    if (EXT && a.scale_bits) coarse_scale(a.scale_bits, a.scale_h1sq, a.scale_kexp, &ecmul);
+    float e[3] = {ev[0].x, ev[0].y, __shfl_down_sync(0xffffffffu, ev[0].x, 1)};
+    unsigned g = fl[0] | ((__shfl_down_sync(0xffffffffu, fl[0], 1) & 1u) << 16);
+#pragma unroll
+    for (int k = 0; k < R / 2; k++) {
+      const float f[3] = {ev[k + 1].x, ev[k + 1].y, __shfl_down_sync(0xffffffffu, ev[k + 1].x, 1)};
+      const unsigned g1 = fl[k + 1] | ((__shfl_down_sync(0xffffffffu, fl[k + 1], 1) & 1u) << 16);
+      float u[2][4];
+      prolongate2(e, f, g, g1, lut, u);
+      if (rim && !ext) {  // no coarse cell beyond: columns and rows from w-2, h-2 on
+#pragma unroll
+        for (int b = 0; b < 4; b++) {
+          if ((b & 1) && X + b >= w - 2) u[0][b] = u[1][b] = 0.0f;
+          if (y + 2 * k + 1 >= h - 2) u[1][b] = 0.0f;
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 2; i++) {
+        const int r = 2 * k + i;
+        const unsigned c = full ? kFull : (y + r >= 1 && y + r < h - 1 ? cw[r] & inmask : 0u);
+        float *p = &pv[r].x;
+#pragma unroll
+        for (int b = 0; b < 4; b++) {
+          const float ub = EXT && a.scale_bits ? u[i][b] * ecmul : u[i][b];
+          p[b] = (c >> (8 * b)) & C_CENTER ? rnd<S>(p[b] + ub) : p[b];
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 3; i++) e[i] = f[i];
+      g = g1;
+    }
+  }
+
+  // ---- registers: pairs of p (0 in solid cells) and of f h^2; factors
+  float2 A[R], B[R], FA[R], FB[R];
+  const float hh = a.hh;
+  copy_wait();
+  bool ok = true;  // magnitudes for which no half sweep can overflow
+#pragma unroll
+  for (int r = 0; r < R; r++) {
+    float *p = &pv[r].x;
+    const float4 fv = St::lds4(reinterpret_cast<const S *>(fac + r * 64));
+    float F[4] = {fv.x * hh * hh, fv.y * hh * hh, fv.z * hh * hh, fv.w * hh * hh};
+    if (!full) {
+      const bool brow = y + r == 0 || y + r == h - 1;
+      const unsigned in = brow ? 0u : inmask;
+      // codes, 32 + flag where the cell keeps its value
+      const unsigned c = (cw[r] & in & 0x1f1f1f1fu) | (~in & ((cw[r] & 0x01010101u) | 0x20202020u));
+#pragma unroll
+      for (int b = 0; b < 4; b++)
+        if (!((c >> (8 * b)) & C_CENTER)) p[b] = F[b] = 0.0f;
+      float2 s[4];
+#pragma unroll
+      for (int b = 0; b < 4; b++) s[b] = lut[(c >> (8 * b)) & 0x3fu];
+      fac[r * 64] = make_float4(s[0].x, s[2].x, s[0].y, s[2].y);
+      fac[r * 64 + 32] = make_float4(s[1].x, s[3].x, s[1].y, s[3].y);
+    }
+    ok = ok && ((fabsf(p[0]) + fabsf(p[1])) + (fabsf(p[2]) + fabsf(p[3]))) +
+                       ((fabsf(F[0]) + fabsf(F[1])) + (fabsf(F[2]) + fabsf(F[3]))) <
+                   kBig;
+    A[r] = make_float2(p[0], p[2]);
+    B[r] = make_float2(p[1], p[3]);
+    FA[r] = make_float2(F[0], F[2]);
+    FB[r] = make_float2(F[1], F[3]);
+  }
+  slot(0, wid, 0) = A[0];
+  slot(0, wid, 1) = B[R - 1];
+  const bool careful = __syncthreads_or(!ok) != 0;
+  // the block's barrier from any of the variants below
+  auto sync = [] { asm volatile("bar.sync 1, %0;" ::"n"(32 * NW) : "memory"); };
+
+  // ---- three sweeps.  Red updates the pair (1, 3) of even rows and (0, 2)
+  // of odd rows, black the others; what a warp reads of its neighbours' rows
+  // was updated in the half sweep before.
+  // At the domain's edge a cell's neighbour on the edge holds the cell's own
+  // value of the sweep before (zero gradient; 0 if the edge cell is solid).
+  const int xe = w - 2 - X;  // place of column w-2 in the lane
+  // MODE 0: an all-fluid warp, 1: any flags, 2: and the domain's edge, 3: and
+  // sums that may not be finite.
+  auto half = [&](auto modec, auto redc, const bool grad) {
+    constexpr int MODE = decltype(modec)::value;
+    constexpr int RED = decltype(redc)::value;
+    constexpr bool EDGE = MODE >= 2;
+    const int buf = RED ? 0 : 1;
+    float2 below = make_float2(0.f, 0.f), above = below;
+    if (wid > 0) below = slot(buf, wid - 1, 1);
+    if (wid < NW - 1) above = slot(buf, wid + 1, 0);
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+      const bool onB = ((r & 1) ^ RED) != 0;  // which pair of this row
+      float2 &own = onB ? B[r] : A[r];
+      float2 W, E;
+      if (onB) {
+        W = A[r];
+        E = make_float2(A[r].y, __shfl_down_sync(0xffffffffu, A[r].x, 1));
+      } else {
+        W = make_float2(__shfl_up_sync(0xffffffffu, B[r].y, 1), B[r].x);
+        E = B[r];
+      }
+      float2 Sv = r > 0 ? (onB ? B[r > 0 ? r - 1 : 0] : A[r > 0 ? r - 1 : 0]) : below;
+      float2 Nv = r < R - 1 ? (onB ? B[r < R - 1 ? r + 1 : 0] : A[r < R - 1 ? r + 1 : 0]) : above;
+      if (EDGE && grad) {
+        const unsigned c0 = cw[r] >> (onB ? 8 : 0), c1 = c0 >> 16;
+        if (onB && first && lane == 0) W.x = (c0 & C_W) ? own.x : 0.0f;
+        if (xe == (onB ? 1 : 0)) E.x = (c0 & C_E) ? own.x : 0.0f;
+        if (xe == (onB ? 3 : 2)) E.y = (c1 & C_E) ? own.y : 0.0f;
+        if (y + r == 1) Sv = make_float2((c0 & C_S) ? own.x : 0.0f, (c1 & C_S) ? own.y : 0.0f);
+        if (y + r == h - 2) Nv = make_float2((c0 & C_N) ? own.x : 0.0f, (c1 & C_N) ? own.y : 0.0f);
+      }
+      const float2 v = add2(add2(add2(add2(W, E), Sv), Nv), onB ? FB[r] : FA[r]);
+      float2 n;
+      if (MODE == 0) {
+        n = make_float2(v.x * 0.25f, v.y * 0.25f);
+      } else {
+        const float4 s = fac[r * 64 + (onB ? 32 : 0)];
+        if (MODE == 3)
+          n = make_float2(scaled_any(v.x, s.x, s.z), scaled_any(v.y, s.y, s.w));
+        else
+          n = scaled2(v, make_float2(s.x, s.y), make_float2(s.z, s.w));
+      }
+      n = rnd2<S>(n);
+      if (EDGE) {  // cells on the domain's edge keep their values
+        if (y + r == 0 || y + r == h - 1) n = own;
+        if (!onB && first && lane == 0) n.x = own.x;
+        if (xe + 1 == (onB ? 1 : 0)) n.x = own.x;
+        if (xe + 1 == (onB ? 3 : 2)) n.y = own.y;
+      }
+      own = n;
+    }
+    slot(buf ^ 1, wid, 0) = RED ? B[0] : A[0];
+    slot(buf ^ 1, wid, 1) = RED ? A[R - 1] : B[R - 1];
+    sync();
+  };
+  auto sweeps = [&](auto modec) {
+    const std::integral_constant<int, 1> red{};
+    const std::integral_constant<int, 0> black{};
+#pragma unroll 1
+    for (int s = 0; s < 3; s++) {
+      half(modec, red, zg && (!PRE || s > 0));
+      half(modec, black, zg && (!PRE || s > 0));
+    }
+  };
+  if (full)
+    sweeps(std::integral_constant<int, 0>{});
+  else if (careful)
+    sweeps(std::integral_constant<int, 3>{});
+  else if (wedge)
+    sweeps(std::integral_constant<int, 2>{});
+  else
+    sweeps(std::integral_constant<int, 1>{});
+
+  // ---- store
+  if (!wedge) {
+#pragma unroll
+    for (int r = 0; r < R; r++)
+      if (mine && y + r >= ya && y + r < yb && y + r < h && X < w) {
+        S *dst = a.out + (size_t)(y + r) * P + X;
+        if (X + 3 < w) {
+          St::st4(dst, make_float4(A[r].x, B[r].x, A[r].y, B[r].y));
+        } else {
+          dst[0] = St::fromf(A[r].x);
+          if (X + 1 < w) dst[1] = St::fromf(B[r].x);
+          if (X + 2 < w) dst[2] = St::fromf(A[r].y);
+        }
+      }
+  } else {
+    auto old = [&](int xx, int yy) {
+      return a.zero_init ? 0.0f : St::ldg1(a.in + (size_t)yy * P + xx);
+    };
+    auto store = [&](int yy, const float (&o)[4]) {
+      if (!mine || X >= w || yy < ya || yy >= yb) return;
+      S *dst = a.out + (size_t)yy * P + X;
+      if (X + 3 < w) {
+        St::st4(dst, make_float4(o[0], o[1], o[2], o[3]));
+      } else {
+#pragma unroll
+        for (int b = 0; b < 3; b++)
+          if (X + b < w) dst[b] = St::fromf(o[b]);
+      }
+    };
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+      const int yy = y + r;
+      if (yy >= h) break;
+      float o[4] = {A[r].x, B[r].x, A[r].y, B[r].y};
+      // columns 0 and w-1: the inner neighbour's value, or as they were
+      const float left = __shfl_up_sync(0xffffffffu, B[r].y, 1);
+      const float in[4] = {left, A[r].x, B[r].x, A[r].y};
+      if (yy == 0 || yy == h - 1) {
+        if (zg) continue;  // written with rows 1 and h-2
+#pragma unroll
+        for (int b = 0; b < 4; b++) o[b] = X + b < w ? old(X + b, yy) : 0.0f;
+        store(yy, o);
+        continue;
+      }
+      if (first && lane == 0) o[0] = zg ? o[1] : old(0, yy);
+#pragma unroll
+      for (int b = 0; b < 4; b++)
+        if (X + b == w - 1) o[b] = zg ? in[b] : old(w - 1, yy);
+      store(yy, o);
+      if (zg && (yy == 1 || yy == h - 2)) {
+        const int ye = yy == 1 ? 0 : h - 1;
+        if (!ext) {  // corner cells are left as they were
+          if (first && lane == 0) o[0] = old(0, ye);
+#pragma unroll
+          for (int b = 0; b < 4; b++)
+            if (X + b == w - 1) o[b] = old(w - 1, ye);
+        }
+        store(ye, o);
+      }
+    }
+  }
+
+  if constexpr (PRE) {
+    // ---- residual (calculateResidualField, pressure_solver.cpp:91-116) of
+    // every row, restricted (pressure_solver.cpp:118-132): a lane holds the
+    // columns over coarse columns X/2 and X/2 + 1
+    float4 fr[R];  // f: where it was copied to, unless factors took the place
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+      if (full) {
+        fr[r] = St::lds4(reinterpret_cast<const S *>(fac + r * 64));
+      } else {
+        fr[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (colok && y + r < h) fr[r] = St::ldg4(a.rhs + (size_t)(y + r) * P + X);
+      }
+    }
+    // rows below and above: (0, 2) and (1, 3) from the two buffers
+    float2 bA = make_float2(0.f, 0.f), bB = bA, tA = bA, tB = bA;
+    if (wid > 0) {
+      bA = slot(1, wid - 1, 1);
+      bB = slot(0, wid - 1, 1);
+    }
+    if (wid < NW - 1) {
+      tA = slot(0, wid + 1, 0);
+      tB = slot(1, wid + 1, 0);
+    }
+    float2 tt[R];  // odd rows: 1-2-1 sums; even rows: 2-4-2 sums
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+      const float2 SA = r > 0 ? A[r > 0 ? r - 1 : 0] : bA, SB = r > 0 ? B[r > 0 ? r - 1 : 0] : bB;
+      const float2 NA = r < R - 1 ? A[r < R - 1 ? r + 1 : 0] : tA,
+                   NB = r < R - 1 ? B[r < R - 1 ? r + 1 : 0] : tB;
+      const float l = __shfl_up_sync(0xffffffffu, B[r].y, 1);
+      const float rr = __shfl_down_sync(0xffffffffu, A[r].x, 1);
+      const float C4[4] = {A[r].x, B[r].x, A[r].y, B[r].y};
+      const float F4[4] = {fr[r].x, fr[r].y, fr[r].z, fr[r].w};
+      float q[4];
+      if (full) {
+        const float2 va = add2(add2(add2(make_float2(l, B[r].x), B[r]), SA), NA);
+        const float2 vb = add2(add2(add2(A[r], make_float2(A[r].y, rr)), SB), NB);
+        const float V4[4] = {va.x, vb.x, va.y, vb.y};
+#pragma unroll
+        for (int b = 0; b < 4; b++) q[b] = rnd<S>(F4[b] + (V4[b] + -4.0f * C4[b]) * a.ihsq);
+      } else {
+        const unsigned c = y + r >= 1 && y + r < h - 1 ? cw[r] & inmask : 0u;
+        float W4[4] = {l, A[r].x, B[r].x, A[r].y}, E4[4] = {B[r].x, A[r].y, B[r].y, rr};
+        float S4[4] = {SA.x, SB.x, SA.y, SB.y}, N4[4] = {NA.x, NB.x, NA.y, NB.y};
+        if (wedge && zg) {  // the edge cells have this cell's value
+#pragma unroll
+          for (int b = 0; b < 4; b++) {
+            if (X + b == 1) W4[b] = C4[b];
+            if (X + b == w - 2) E4[b] = C4[b];
+            if (y + r == 1) S4[b] = C4[b];
+            if (y + r == h - 2) N4[b] = C4[b];
+          }
+        }
+        residual4(c, C4, W4, E4, S4, N4, F4, a.ihsq, q);
+#pragma unroll
+        for (int b = 0; b < 4; b++) q[b] = rnd<S>(q[b]);
+      }
+      const float ql = __shfl_up_sync(0xffffffffu, q[3], 1);
+      if (r & 1)
+        tt[r] = make_float2((ql * 1.0f + q[0] * 2.0f) + q[1] * 1.0f,
+                            (q[1] * 1.0f + q[2] * 2.0f) + q[3] * 1.0f);
+      else
+        tt[r] = make_float2((ql * 2.0f + q[0] * 4.0f) + q[1] * 2.0f,
+                            (q[1] * 2.0f + q[2] * 4.0f) + q[3] * 2.0f);
+    }
+    res[wid * 32] = tt[R - 1];
+    sync();
+    float2 below = make_float2(0.f, 0.f);
+    if (wid > 0) below = res[(wid - 1) * 32];
+    float rfac = a.rfac;
+    if (EXT && a.scale_bits) {
+      float inv;
+      rfac = rfac * (coarse_scale(a.scale_bits, a.scale_h1sq, a.scale_kexp, &inv) * a.scale_h1sq);
+    }
+    const int c0 = X >> 1;
+#pragma unroll
+    for (int r = 0; r < R; r += 2) {
+      const int yy = y + r, Y = yy >> 1;
+      if (!(mine && yy >= ya && yy < yb && Y < a.ch && c0 < a.cw)) continue;
+      const float2 tb = r > 0 ? tt[r > 0 ? r - 1 : 0] : below;
+      float v0 = ((tb.x + tt[r].x) + tt[r + 1].x) * rfac;
+      float v1 = ((tb.y + tt[r].y) + tt[r + 1].y) * rfac;
+      if (rim) {
+        const bool yz = Y == 0 || Y == a.ch - 1;
+        if (yz || c0 == 0 || c0 >= a.cw - 1) v0 = 0.0f;
+        if (yz || c0 + 1 >= a.cw - 1) v1 = 0.0f;
+      }
+      SC *dst = a.rc + (size_t)Y * a.cpitch + c0;
+      if (c0 + 1 < a.cw)
+        Sc::sts2(dst, v0, v1);
+      else
+        dst[0] = Sc::fromf(v0);
+    }
+  }
+}
+
+}  // namespace tile
+}  // namespace
+}  // namespace ubg

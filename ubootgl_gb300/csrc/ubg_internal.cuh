@@ -286,7 +286,7 @@ __device__ __forceinline__ bool table_ok(const int *__restrict__ bs, int n, unsi
 // back to back, the block prefix sums and the dynamic shared memory.
 struct MultiSlot {
   int kind = 0;
-  int tile = -1;  // MK_MG: smoother tile id
+  int tile = -1;  // MK_MG: smoother tile id; MK_TAIL: 1 = the kernel of any shape
   int n = 0;
   int blocks = 0;
   size_t smem = 0;
@@ -321,16 +321,12 @@ struct MgHier {
   std::vector<MgLevel> lv;
   int cur0 = 0;                  // which e[] of level 0 holds p
   int tail_top = -1;             // first level solved by the one-CTA tail kernel
-  int tail_cells = 2048;         // largest top level the tail takes (autotuned)
+  bool tail_wide = false;        // elongated levels: the tail kernel of any shape
+  int tail_cells = 8192;         // largest top level the tail takes (autotuned)
   int tail_top_fp64 = -1;        // the same for the mixed solver's FP64 tail
-  // First level of the cluster coarse solve (levels cluster_top ..
-  // tail_top-1 in row bands over a thread-block cluster, the tail's levels
-  // in its first CTA; one launch), or -1: launches per level.
-  int cluster_top = -1;
   void *arena = nullptr;
   size_t arena_bytes = 0;
   double *norm = nullptr;        // device scalar for residual norms
-  double *post_norm2 = nullptr;  // if set: ||r||^2 after each level-0 post-smoothing
   // The tolerance solver's own hierarchy (ext_hier_*): level sizes
   // floor(w/2)+1, zero-gradient edges on every level, coarsest level = the
   // last one, solved with `ncoarse` sweeps.  The reference's hierarchy
@@ -339,8 +335,6 @@ struct MgHier {
   int ncoarse = 5;
 };
 inline int mg_coarsest(const MgHier &mg) { return mg.ext ? mg.levels - 1 : mg.levels - 2; }
-// Whether the cluster coarse solve can run on this device, and why not.
-const char *cluster_coarse_solve_status();
 
 // Times the candidate smoother tiles of every level and the tail sizes on
 // this hierarchy's own arrays (state preserved: trials write only scratch
