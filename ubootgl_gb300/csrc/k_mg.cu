@@ -1176,11 +1176,12 @@ coarse::Args<S> coarse_args(MgHier &mg, int lt, const S *rhs_top, S *e_top, cons
     coarse::Level &C = a.L[t];
     C.w = L.w;
     C.h = L.h;
-    C.lanes = (L.w + 3) / 4;
+    C.lsh = coarse::lane_shift(L.w);
+    C.warps = coarse::warps_of(L.w, L.h);
     C.hh = rfac ? 1.0f : L.hh;
     C.ihsq = rfac ? 1.0f : 1.0f / L.hh / L.hh;
     C.rfac = rfac ? rfac[lt + t] : 1.0f / 16.0f;
-    const size_t n = (size_t)C.lanes * C.h;
+    const size_t n = (size_t)C.h << C.lsh;
     C.oe = (int)off;
     C.of = (int)(off + 16 * n);
     C.oc = (int)(off + 32 * n);
@@ -1616,11 +1617,11 @@ int choose_tail_any(const std::vector<MgLevel> &lv, int max_cells, size_t elem_b
       return lt;
   return -1;
 }
-// The first level from which the coarse solve in registers (levels of at most
-// 128 x 64 cells) covers the rest, with a top level of at most max_cells.
+// The first level from which the one-block coarse solve covers the rest, with
+// a top level of at most max_cells.
 int choose_tail(const std::vector<MgLevel> &lv, int max_cells, int last) {
   for (int lt = 1; lt <= last; lt++)
-    if (lv[lt].w <= coarse::kMaxW && lv[lt].h <= coarse::kMaxH && last - lt < coarse::kMaxLevels &&
+    if (coarse::fits(lv[lt].w, lv[lt].h) && last - lt < coarse::kMaxLevels &&
         (size_t)lv[lt].w * lv[lt].h <= (size_t)max_cells)
       return lt;
   return -1;
@@ -1888,7 +1889,7 @@ void mg_autotune(MgHier &mg, cudaStream_t st, std::string *report) {
   double best = vcycle_us();
   note("start", -1, "default", best);
   // tail size
-  const int tail_cand[] = {512, 2048, 8192};
+  const int tail_cand[] = {512, 2048, 4096};
   int best_tc = mg.tail_cells, best_lt = mg.tail_top;
   for (int tc : tail_cand) {
     int lt = mg.tail_wide ? -1 : choose_tail(mg.lv, tc, nl - 2);

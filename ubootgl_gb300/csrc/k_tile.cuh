@@ -22,9 +22,12 @@
 // What bounds it: instruction issue and the FP32 pipe on large levels, the
 // latency of loads, six barriers and one pass through the code on small ones.
 // Against tiles in shared memory (red/black-split, 112 x 50 and 48 x 16
-// cells), ncu: level 0 of 4096x2048 58 us (89 with the residual, 98 with the
+// cells), ncu: level 0 of 4096x2048 56 us (89 with the residual, 98 with the
 // prolongation), 2048x1024 18 us (33, 38), 1024x512 8 us (18, 20), 256x128
-// 6 us.
+// 6 us.  Of those 56 us, bounds checks outside the blocks that need them, the
+// packed magnitude check and W + E as scalar additions (no register moves)
+// are 2 us (32.4 -> 25.5 M warp instructions).  Regions of 8 rows per warp
+// (8 warps), and of 128 x 32 cells, are slower there (58-60, 65 us).
 #pragma once
 
 namespace ubg {
@@ -40,13 +43,14 @@ constexpr unsigned kFull = 0x1f1f1f1fu;
 __host__ __device__ constexpr int regions(int c, int n) {
   return c <= n ? 1 : (c - 2 * kHalo + n - 2 * kHalo - 1) / (n - 2 * kHalo);
 }
-// Shared memory: factors (16 bytes per pair), exchanged rows, table of
-// factors by code and of the prolongation's weight sums.
+// Shared memory: factors (16 bytes per pair), exchanged rows of each warp
+// (and of one below and one above: zeros), restriction rows, table of factors
+// by code and of the prolongation's weight sums.
 constexpr int kLutBytes = (64 + 5) * 8;
 template <int R, int NW>
 struct Mem {
-  static constexpr int fac = 0, xch = fac + R * NW * 1024, res = xch + 2 * NW * 512,
-                       lut = res + NW * 256, bytes = lut + kLutBytes;
+  static constexpr int fac = 0, xch = fac + R * NW * 1024, res = xch + 2 * (NW + 2) * 512,
+                       lut = res + (NW + 1) * 256, bytes = lut + kLutBytes;
 };
 
 // Two operations in one instruction, each lane rounded as its scalar form.
@@ -101,8 +105,9 @@ __device__ __forceinline__ float scaled_any(float v, float s, float c) {
   const float n = (c != 0.0f && fabsf(v) < __int_as_float(0x7f800000)) ? q3 : q;
   return s != 0.0f ? n : 0.0f;
 }
-// Magnitude bound under which six (ten) half sweeps stay finite.
-constexpr float kBig = 0x1p+60f;
+// Bound of the sum of squares of what a lane holds under which six (ten)
+// half sweeps stay finite.
+constexpr float kBigSq = 0x1p+120f;
 
 // Unsigned bits without the sign, less one: a value is 0 (all ones) or its
 // division by div_rn's correction is exact when the key is in [lo, hi] of
@@ -224,47 +229,60 @@ __device__ __forceinline__ void run(const MgArgsT<S, SC> &a, const int region,
   const float2 *const lut = reinterpret_cast<const float2 *>(smem + M::lut);
   // exchanged rows: buffer (half sweep parity), warp, its first or last row
   auto slot = [&](int buf, int wd, int lastrow) -> float2 & {
-    return xch[((buf * NW + wd) * 2 + lastrow) * 32];
+    return xch[((buf * (NW + 2) + 1 + wd) * 2 + lastrow) * 32];
   };
 
   // ---- loads: all in flight together; f is copied to where the lane's
   // factors will be (16 registers less while the rest arrives)
+  const bool inner = !first && !has_east && y0 > 0 && y0 + RY < h - 1;  // no bounds to check
   const bool colok = X < w;
+  const size_t o0 = (size_t)y * P + X;
   float4 pv[R];
   unsigned cw[R];
+  unsigned inmask = ~0u;  // columns that are smoothed
+  if (inner) {
 #pragma unroll
-  for (int r = 0; r < R; r++) {
-    const bool ok = colok && y + r < h;
-    const size_t o = ok ? (size_t)(y + r) * P + X : 0;
-    copy_async<4 * (int)sizeof(S)>(fac + r * 64, a.rhs + o, ok);
-    pv[r] = make_float4(0.f, 0.f, 0.f, 0.f);
-    cw[r] = 0u;
-    if (ok) {
-      if (!a.zero_init) pv[r] = St::ldg4(a.in + o);
-      cw[r] = __ldg(reinterpret_cast<const unsigned *>(a.code + o));
+    for (int r = 0; r < R; r++) copy_async<4 * (int)sizeof(S)>(fac + r * 64, a.rhs + o0 + r * P, true);
+    if (!a.zero_init) {
+#pragma unroll
+      for (int r = 0; r < R; r++) pv[r] = St::ldg4(a.in + o0 + r * P);
+    } else {
+#pragma unroll
+      for (int r = 0; r < R; r++) pv[r] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
-  }
-  copy_commit();
-  unsigned inmask = 0u;  // columns that are smoothed
-  {
+#pragma unroll
+    for (int r = 0; r < R; r++)
+      cw[r] = __ldg(reinterpret_cast<const unsigned *>(a.code + o0 + r * P));
+  } else {
     unsigned colmask = 0u;
+    inmask = 0u;
 #pragma unroll
     for (int b = 0; b < 4; b++) {
       colmask |= X + b < w ? 0xffu << (8 * b) : 0u;
       inmask |= X + b >= 1 && X + b < w - 1 ? 0xffu << (8 * b) : 0u;
     }
 #pragma unroll
-    for (int r = 0; r < R; r++) cw[r] &= colmask;
+    for (int r = 0; r < R; r++) {
+      const bool ok = colok && y + r < h;
+      copy_async<4 * (int)sizeof(S)>(fac + r * 64, a.rhs + (ok ? o0 + r * P : 0), ok);
+      pv[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+      cw[r] = 0u;
+      if (ok) {
+        if (!a.zero_init) pv[r] = St::ldg4(a.in + o0 + r * P);
+        cw[r] = __ldg(reinterpret_cast<const unsigned *>(a.code + o0 + r * P)) & colmask;
+      }
+    }
   }
-  bool full = true;
+  copy_commit();
+  unsigned all = cw[0];
 #pragma unroll
-  for (int r = 0; r < R; r++) full = full && cw[r] == kFull;
+  for (int r = 1; r < R; r++) all &= cw[r];
   // the warp's rows or columns touch the domain's edge (rows 1 and h-2 too:
   // their neighbours on the edge follow them); where the edge cells are 0 and
   // stay so, the factor 0 does it
   const bool rim = first || has_east || y <= 1 || y + R >= h - 1;
   const bool wedge = rim && !a.zero_edges;
-  full = __all_sync(0xffffffffu, full) && !rim;
+  const bool full = __all_sync(0xffffffffu, all == kFull) && !rim;
 
   if constexpr (!PRE) {
     // ---- prolongate (pressure_solver.cpp:134-172) + correct: an even row
@@ -275,13 +293,13 @@ __device__ __forceinline__ void run(const MgArgsT<S, SC> &a, const int region,
     unsigned fl[RC];
 #pragma unroll
     for (int k = 0; k < RC; k++) {
+      const size_t o = (size_t)(cy + k) * a.cpitch + c0;
       ev[k] = make_float2(0.f, 0.f);
       fl[k] = 0u;
-      if (c0 < a.cw && cy + k < a.ch) {
-        const size_t o = (size_t)(cy + k) * a.cpitch + c0;
+      if (inner || (c0 < a.cw && cy + k < a.ch)) {
         ev[k] = Sc::ldg2(a.ec + o);
         fl[k] = __ldg(reinterpret_cast<const unsigned short *>(a.codec + o)) & 0x0101u;
-        if (c0 + 1 >= a.cw) {
+        if (!inner && c0 + 1 >= a.cw) {
           ev[k].y = 0.0f;
           fl[k] &= 0x00ffu;
         }
@@ -307,12 +325,19 @@ __device__ __forceinline__ void run(const MgArgsT<S, SC> &a, const int region,
 #pragma unroll
       for (int i = 0; i < 2; i++) {
         const int r = 2 * k + i;
-        const unsigned c = full ? kFull : (y + r >= 1 && y + r < h - 1 ? cw[r] & inmask : 0u);
         float *p = &pv[r].x;
+        if (EXT && a.scale_bits) {
 #pragma unroll
-        for (int b = 0; b < 4; b++) {
-          const float ub = EXT && a.scale_bits ? u[i][b] * ecmul : u[i][b];
-          p[b] = (c >> (8 * b)) & C_CENTER ? rnd<S>(p[b] + ub) : p[b];
+          for (int b = 0; b < 4; b++) u[i][b] = u[i][b] * ecmul;
+        }
+        if (full) {
+#pragma unroll
+          for (int b = 0; b < 4; b++) p[b] = rnd<S>(p[b] + u[i][b]);
+        } else {
+          const unsigned c = y + r >= 1 && y + r < h - 1 ? cw[r] & inmask : 0u;
+#pragma unroll
+          for (int b = 0; b < 4; b++)
+            p[b] = (c >> (8 * b)) & C_CENTER ? rnd<S>(p[b] + u[i][b]) : p[b];
         }
       }
 #pragma unroll
@@ -325,7 +350,7 @@ __device__ __forceinline__ void run(const MgArgsT<S, SC> &a, const int region,
   float2 A[R], B[R], FA[R], FB[R];
   const float hh = a.hh;
   copy_wait();
-  bool ok = true;  // magnitudes for which no half sweep can overflow
+  float2 sq = make_float2(0.f, 0.f);  // sums of squares of p and f h^2
 #pragma unroll
   for (int r = 0; r < R; r++) {
     float *p = &pv[r].x;
@@ -345,17 +370,19 @@ __device__ __forceinline__ void run(const MgArgsT<S, SC> &a, const int region,
       fac[r * 64] = make_float4(s[0].x, s[2].x, s[0].y, s[2].y);
       fac[r * 64 + 32] = make_float4(s[1].x, s[3].x, s[1].y, s[3].y);
     }
-    ok = ok && ((fabsf(p[0]) + fabsf(p[1])) + (fabsf(p[2]) + fabsf(p[3]))) +
-                       ((fabsf(F[0]) + fabsf(F[1])) + (fabsf(F[2]) + fabsf(F[3]))) <
-                   kBig;
     A[r] = make_float2(p[0], p[2]);
     B[r] = make_float2(p[1], p[3]);
     FA[r] = make_float2(F[0], F[2]);
     FB[r] = make_float2(F[1], F[3]);
+    sq = f2_fma(FB[r], FB[r], f2_fma(FA[r], FA[r], f2_fma(B[r], B[r], f2_fma(A[r], A[r], sq))));
   }
   slot(0, wid, 0) = A[0];
   slot(0, wid, 1) = B[R - 1];
-  const bool careful = __syncthreads_or(!ok) != 0;
+  if (wid == 0)
+    slot(0, -1, 1) = slot(1, -1, 1) = slot(0, NW, 0) = slot(1, NW, 0) = res[0] =
+        make_float2(0.f, 0.f);
+  // false for infinities and NaNs too
+  const bool careful = __syncthreads_or(!(sq.x + sq.y < kBigSq)) != 0;
   // the block's barrier from any of the variants below
   auto sync = [] { asm volatile("bar.sync 1, %0;" ::"n"(32 * NW) : "memory"); };
 
@@ -372,9 +399,7 @@ __device__ __forceinline__ void run(const MgArgsT<S, SC> &a, const int region,
     constexpr int RED = decltype(redc)::value;
     constexpr bool EDGE = MODE >= 2;
     const int buf = RED ? 0 : 1;
-    float2 below = make_float2(0.f, 0.f), above = below;
-    if (wid > 0) below = slot(buf, wid - 1, 1);
-    if (wid < NW - 1) above = slot(buf, wid + 1, 0);
+    const float2 below = slot(buf, wid - 1, 1), above = slot(buf, wid + 1, 0);
 #pragma unroll
     for (int r = 0; r < R; r++) {
       const bool onB = ((r & 1) ^ RED) != 0;  // which pair of this row
@@ -397,7 +422,9 @@ __device__ __forceinline__ void run(const MgArgsT<S, SC> &a, const int region,
         if (y + r == 1) Sv = make_float2((c0 & C_S) ? own.x : 0.0f, (c1 & C_S) ? own.y : 0.0f);
         if (y + r == h - 2) Nv = make_float2((c0 & C_N) ? own.x : 0.0f, (c1 & C_N) ? own.y : 0.0f);
       }
-      const float2 v = add2(add2(add2(add2(W, E), Sv), Nv), onB ? FB[r] : FA[r]);
+      // (W + E needs no pair of its own: scalar additions, without moves)
+      const float2 we = make_float2(W.x + E.x, W.y + E.y);
+      const float2 v = add2(add2(add2(we, Sv), Nv), onB ? FB[r] : FA[r]);
       float2 n;
       if (MODE == 0) {
         n = make_float2(v.x * 0.25f, v.y * 0.25f);
@@ -439,8 +466,14 @@ __device__ __forceinline__ void run(const MgArgsT<S, SC> &a, const int region,
   else
     sweeps(std::integral_constant<int, 1>{});
 
-  // ---- store
-  if (!wedge) {
+  // ---- store (ya and yb are multiples of R: all of a warp's rows or none)
+  if (inner) {
+    if (mine && y >= ya && y < yb) {
+#pragma unroll
+      for (int r = 0; r < R; r++)
+        St::st4(a.out + o0 + r * P, make_float4(A[r].x, B[r].x, A[r].y, B[r].y));
+    }
+  } else if (!wedge) {
 #pragma unroll
     for (int r = 0; r < R; r++)
       if (mine && y + r >= ya && y + r < yb && y + r < h && X < w) {
@@ -516,15 +549,8 @@ __device__ __forceinline__ void run(const MgArgsT<S, SC> &a, const int region,
       }
     }
     // rows below and above: (0, 2) and (1, 3) from the two buffers
-    float2 bA = make_float2(0.f, 0.f), bB = bA, tA = bA, tB = bA;
-    if (wid > 0) {
-      bA = slot(1, wid - 1, 1);
-      bB = slot(0, wid - 1, 1);
-    }
-    if (wid < NW - 1) {
-      tA = slot(0, wid + 1, 0);
-      tB = slot(1, wid + 1, 0);
-    }
+    const float2 bA = slot(1, wid - 1, 1), bB = slot(0, wid - 1, 1);
+    const float2 tA = slot(0, wid + 1, 0), tB = slot(1, wid + 1, 0);
     float2 tt[R];  // odd rows: 1-2-1 sums; even rows: 2-4-2 sums
 #pragma unroll
     for (int r = 0; r < R; r++) {
@@ -537,11 +563,13 @@ __device__ __forceinline__ void run(const MgArgsT<S, SC> &a, const int region,
       const float F4[4] = {fr[r].x, fr[r].y, fr[r].z, fr[r].w};
       float q[4];
       if (full) {
-        const float2 va = add2(add2(add2(make_float2(l, B[r].x), B[r]), SA), NA);
-        const float2 vb = add2(add2(add2(A[r], make_float2(A[r].y, rr)), SB), NB);
+        const float2 va = add2(add2(make_float2(l + B[r].x, B[r].x + B[r].y), SA), NA);
+        const float2 vb = add2(add2(make_float2(A[r].x + A[r].y, A[r].y + rr), SB), NB);
         const float V4[4] = {va.x, vb.x, va.y, vb.y};
+        // (-4 c is exact, so the fused form is the reference's sum)
 #pragma unroll
-        for (int b = 0; b < 4; b++) q[b] = rnd<S>(F4[b] + (V4[b] + -4.0f * C4[b]) * a.ihsq);
+        for (int b = 0; b < 4; b++)
+          q[b] = rnd<S>(F4[b] + __fmaf_rn(-4.0f, C4[b], V4[b]) * a.ihsq);
       } else {
         const unsigned c = y + r >= 1 && y + r < h - 1 ? cw[r] & inmask : 0u;
         float W4[4] = {l, A[r].x, B[r].x, A[r].y}, E4[4] = {B[r].x, A[r].y, B[r].y, rr};
@@ -560,17 +588,16 @@ __device__ __forceinline__ void run(const MgArgsT<S, SC> &a, const int region,
         for (int b = 0; b < 4; b++) q[b] = rnd<S>(q[b]);
       }
       const float ql = __shfl_up_sync(0xffffffffu, q[3], 1);
+      // 1-2-1 or 2-4-2 (products by powers of two are exact)
       if (r & 1)
-        tt[r] = make_float2((ql * 1.0f + q[0] * 2.0f) + q[1] * 1.0f,
-                            (q[1] * 1.0f + q[2] * 2.0f) + q[3] * 1.0f);
+        tt[r] = make_float2(__fmaf_rn(q[0], 2.0f, ql) + q[1], __fmaf_rn(q[2], 2.0f, q[1]) + q[3]);
       else
-        tt[r] = make_float2((ql * 2.0f + q[0] * 4.0f) + q[1] * 2.0f,
-                            (q[1] * 2.0f + q[2] * 4.0f) + q[3] * 2.0f);
+        tt[r] = make_float2(__fmaf_rn(q[1], 2.0f, __fmaf_rn(q[0], 4.0f, ql * 2.0f)),
+                            __fmaf_rn(q[3], 2.0f, __fmaf_rn(q[2], 4.0f, q[1] * 2.0f)));
     }
-    res[wid * 32] = tt[R - 1];
+    res[(wid + 1) * 32] = tt[R - 1];
     sync();
-    float2 below = make_float2(0.f, 0.f);
-    if (wid > 0) below = res[(wid - 1) * 32];
+    const float2 below = res[wid * 32];
     float rfac = a.rfac;
     if (EXT && a.scale_bits) {
       float inv;
@@ -580,7 +607,8 @@ __device__ __forceinline__ void run(const MgArgsT<S, SC> &a, const int region,
 #pragma unroll
     for (int r = 0; r < R; r += 2) {
       const int yy = y + r, Y = yy >> 1;
-      if (!(mine && yy >= ya && yy < yb && Y < a.ch && c0 < a.cw)) continue;
+      if (!(mine && y >= ya && y < yb)) continue;
+      if (!inner && !(Y < a.ch && c0 < a.cw)) continue;
       const float2 tb = r > 0 ? tt[r > 0 ? r - 1 : 0] : below;
       float v0 = ((tb.x + tt[r].x) + tt[r + 1].x) * rfac;
       float v1 = ((tb.y + tt[r].y) + tt[r + 1].y) * rfac;
@@ -590,7 +618,7 @@ __device__ __forceinline__ void run(const MgArgsT<S, SC> &a, const int region,
         if (yz || c0 + 1 >= a.cw - 1) v1 = 0.0f;
       }
       SC *dst = a.rc + (size_t)Y * a.cpitch + c0;
-      if (c0 + 1 < a.cw)
+      if (inner || c0 + 1 < a.cw)
         Sc::sts2(dst, v0, v1);
       else
         dst[0] = Sc::fromf(v0);
