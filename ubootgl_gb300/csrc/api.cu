@@ -338,14 +338,29 @@ struct ubg_sim {
   }
 
   // Everything of step() after the scalars are staged and the accumulated
-  // velocity is applied; captured into a graph in fixed-cycle mode.  The
-  // final setVBCs completes max|u| over all faces.
+  // velocity is applied; captured into a graph in fixed-cycle mode.  setVBCs
+  // and setPBC are part of the kernels before and after them: the first sweep
+  // also stands for the vy boundary refreshed before it (diffuse() above), and
+  // the gradient kernel for setPBC, the final setVBCs and max|u| over all
+  // faces (the tolerance solver's gradient kernel leaves those to launches).
   void step_body(int nsink_cells) {
-    diffuse();
-    advect();
-    set_vbcs();
-    project(nsink_cells);
-    launch_vbc(v, fx, fy, bc, true, true, st, d_umax);
+    for (int i = 1; i <= 2; i++) {
+      launch_diffuse_sweep(v, fx, fy, d_sc, 3, st, i, bc);
+      fx ^= 1;
+      fy ^= 1;
+    }
+    launch_advect(v, fx, fy, d_sc, st, true, bc, d_umax);
+    fx ^= 1;
+    fy ^= 1;
+    if (opt.solver_mode == UBG_SOLVE_TOLERANCE) {
+      project(nsink_cells);
+      launch_vbc(v, fx, fy, bc, true, true, st, d_umax);
+      return;
+    }
+    launch_divergence(v, fx, fy, f(), d_sc, st);
+    launch_sinks(f(), P, d_sinks, nsink_cells, st);
+    solve_pressure();
+    launch_gradient(v, fx, fy, p(), d_sc, d_umax, st, true, bc);
   }
 
   void step(float dt, bool device_dt, float cfl) {
@@ -1442,16 +1457,6 @@ void fused_plan(const std::vector<ubg_sim *> &sims, const float *cfl,
     sl.blocks += blocks;
     sl.n++;
   };
-  auto vbc = [&](bool dvx, bool dvy, bool umax) {
-    MultiSlot sl;
-    sl.kind = MK_VBC;
-    for (int i = 0; i < n; i++) {
-      ubg_sim *s = sims[i];
-      VbcM a{s->v, fx[i], fy[i], dvx, dvy, s->bc, umax ? s->d_umax : nullptr};
-      add(sl, &a, sizeof(a), multi_blocks_vbc(a));
-    }
-    slots.push_back(std::move(sl));
-  };
   {  // dt = cfl h / max|u| from the previous step's max|u|
     MultiSlot sl;
     sl.kind = MK_CFL;
@@ -1462,28 +1467,25 @@ void fused_plan(const std::vector<ubg_sim *> &sims, const float *cfl,
     }
     slots.push_back(std::move(sl));
   }
-  // diffuse (simulation.cpp:104-162)
-  vbc(false, true, false);
-  for (int k = 0; k < 2; k++) {
+  for (int k = 1; k <= 2; k++) {  // diffuse (simulation.cpp:104-162)
     MultiSlot sl;
     sl.kind = MK_DIFFUSE;
     for (int i = 0; i < n; i++) {
       ubg_sim *s = sims[i];
-      DiffuseM a{s->v, fx[i], fy[i], 3, 0, 0, s->d_sc};
+      DiffuseM a{s->v, fx[i], fy[i], k, 0, s->d_sc, s->bc};
       int b = multi_blocks_diffuse(a);
       add(sl, &a, sizeof(a), b);
       fx[i] ^= 1;
       fy[i] ^= 1;
     }
     slots.push_back(std::move(sl));
-    vbc(true, true, false);
   }
   {  // advect
     MultiSlot sl;
     sl.kind = MK_ADVECT;
     for (int i = 0; i < n; i++) {
       ubg_sim *s = sims[i];
-      AdvectM a{s->v, fx[i], fy[i], 0, s->d_sc};
+      AdvectM a{s->v, fx[i], fy[i], 0, s->d_sc, s->bc, s->d_umax};
       int b = multi_blocks_advect(a);
       add(sl, &a, sizeof(a), b);
       fx[i] ^= 1;
@@ -1491,7 +1493,6 @@ void fused_plan(const std::vector<ubg_sim *> &sims, const float *cfl,
     }
     slots.push_back(std::move(sl));
   }
-  vbc(true, true, false);
   {  // project: divergence
     MultiSlot sl;
     sl.kind = MK_DIVERGENCE;
@@ -1509,28 +1510,17 @@ void fused_plan(const std::vector<ubg_sim *> &sims, const float *cfl,
   for (auto *s : sims)
     if (s->opt.vcycles != vc) throw ArgError("fused batch: members need the same V-cycle count");
   for (int c = 0; c < vc; c++) mg_multi_vcycle(mgs, slots);
-  {  // setPBC, then the gradient update with max|u| (umax zeroed first)
-    MultiSlot sl;
-    sl.kind = MK_PBC;
-    for (int i = 0; i < n; i++) {
-      ubg_sim *s = sims[i];
-      PbcM a{s->p(), s->P, s->W, s->H, s->bc, s->d_umax};
-      add(sl, &a, sizeof(a), multi_blocks_pbc(a));
-    }
-    slots.push_back(std::move(sl));
-  }
-  {
+  {  // setPBC, the gradient update, setVBCs and max|u|
     MultiSlot sl;
     sl.kind = MK_GRADIENT;
     for (int i = 0; i < n; i++) {
       ubg_sim *s = sims[i];
-      GradientM a{s->v, fx[i], fy[i], 0, s->p(), s->d_sc, s->d_umax};
+      GradientM a{s->v, fx[i], fy[i], 0, s->p(), s->d_sc, s->d_umax, s->bc};
       int b = multi_blocks_gradient(a);
       add(sl, &a, sizeof(a), b);
     }
     slots.push_back(std::move(sl));
   }
-  vbc(true, true, true);
   afx = fx;
   afy = fy;
 }

@@ -131,6 +131,42 @@ __device__ void vbc_component(const float *s, float *b0, float *b1, int pitch, i
   }
 }
 
+// The same boundary values from the thread that has just computed interior
+// face (x, y): the cells of the edge next to it and, next to two edges, the
+// corner.  In the step this replaces six launches of edge cells only (setVBCs
+// five times, setPBC), 2 to 3 us each: 107 -> 97 us per step at 256x128.  old(x, y): the edge's value before; put(x, y, value) stores.  Each
+// edge cell's old value is read by this thread alone, and before it is
+// overwritten.
+template <bool XPAR, class Old, class Put>
+__device__ __forceinline__ void edge_cells(int x, int y, float v, int w, int h, Bcs bc, Old &&old,
+                                           Put &&put) {
+  auto edge_x = [&](int side, float a, float b) {
+    return XPAR ? vbc_par(side, a, b) : vbc_per(side, a, b);
+  };
+  auto edge_y = [&](int side, float a, float b) {
+    return XPAR ? vbc_per(side, a, b) : vbc_par(side, a, b);
+  };
+  const bool W = x == 1, E = x == w - 2, S = y == 1, N = y == h - 2;
+  float l = 0.0f, r = 0.0f;
+  if (W) l = edge_x(bc.w, v, old(0, y));
+  if (E) r = edge_x(bc.e, v, old(w - 1, y));
+#pragma unroll 1
+  for (int k = 0; k < 2; k++) {
+    if (!(k ? N : S)) continue;
+    const int ye = k ? h - 1 : 0, side = k ? bc.n : bc.s;
+    const float o = old(x, ye);
+    if (W) put(0, ye, edge_y(side, l, edge_x(bc.w, o, old(0, ye))));
+    if (E) put(w - 1, ye, edge_y(side, r, edge_x(bc.e, o, old(w - 1, ye))));
+    put(x, ye, edge_y(side, v, o));
+  }
+  if (W) put(0, y, l);
+  if (E) put(w - 1, y, r);
+}
+// Whether faces x .. x + 3 of row y have one next to an edge.
+__device__ __forceinline__ bool near_edge(int x, int y, int w, int h) {
+  return x <= 1 || x + 3 >= w - 2 || y == 1 || y == h - 2;
+}
+
 __device__ __forceinline__ void k_vbc_body(VelBufs v, int fx, int fy, Bcs bc, int do_vx, int do_vy,
                       unsigned int *umax_bits, const int bx, const int by, const int bz) {
   int t = bx * blockDim.x + threadIdx.x;
@@ -254,63 +290,138 @@ __device__ __forceinline__ void st4_masked(float *row, int x, int lo, int hi, co
   }
 }
 
-__device__ __forceinline__ void k_diffuse_body(VelBufs v, int srcx, int srcy,
-                                                 const StepScalars *__restrict__ sc, int comps, const int bx, const int by, const int bz) {
+// Four faces of a sweep: (c + a val) / den where the face is open, 0
+// elsewhere, val the sum of the neighbours t1 .. t4 in the reference's order.
+// Faces with only open neighbours (codes k) need no selects, and the division
+// one range check for the four: the sweep is bound by issue as much as by
+// memory (405 -> 316 warp instructions per 8 faces a thread; 33 -> 28 us at
+// 4096x2048, where 151 MB at the copy rate are 22 us).
+__device__ __forceinline__ void diffuse4(unsigned k, const float (&c)[4], const float (&t1)[4],
+                                         const float (&t2)[4], const float (&t3)[4],
+                                         const float (&t4)[4], float a, float den, float rden,
+                                         float (&o)[4]) {
+  constexpr unsigned kOpen = (FC_M | FC_T1 | FC_T2 | FC_T3 | FC_T4) * 0x01010101u;
+  const bool open = (k & kOpen) == kOpen;
+  float x[4];
+  if (open) {
+#pragma unroll
+    for (int j = 0; j < 4; j++) x[j] = c[j] + a * (((t1[j] + t2[j]) + t3[j]) + t4[j]);
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const unsigned q = k >> (8 * j);
+      float val = 0.0f;
+      val = val + ((q & FC_T1) ? t1[j] : 0.0f);
+      val = val + ((q & FC_T2) ? t2[j] : 0.0f);
+      val = val + ((q & FC_T3) ? t3[j] : -c[j]);
+      val = val + ((q & FC_T4) ? t4[j] : -c[j]);
+      x[j] = c[j] + a * val;
+    }
+  }
+  // div_rn, its range checked once for the four (zeros are exact too)
+  unsigned lo = ~0u;
+  float m = 0.0f;
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    lo = min(lo, div_key(x[j]));
+    m = m + fabsf(x[j]);
+  }
+  if (lo >= kDivKeyLo && m <= 0x1p+100f) {
+#pragma unroll
+    for (int j = 0; j < 4; j += 2) {
+      const float2 xx = make_float2(x[j], x[j + 1]);
+      const float2 q0 = f2_mul(xx, f2(rden));
+      const float2 q = f2_fma(f2_fma(q0, f2(-den), xx), f2(rden), q0);
+      o[j] = q.x;
+      o[j + 1] = q.y;
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; j++) o[j] = x[j] / den;
+  }
+  if (!open) {
+#pragma unroll
+    for (int j = 0; j < 4; j++) o[j] = ((k >> (8 * j)) & FC_M) ? o[j] : 0.0f;
+  }
+}
+
+// edges: 0 = the sweep alone; 1, 2 = the first / second sweep of a step, with
+// setVBCs after it (into the sweep's result) and, for vy before the first
+// sweep, the boundary values that setVBCs gives the field as it is.  The
+// first sweep's vx edges come from the buffer it writes (setVBCs reads that
+// buffer's own edge values), every other from the one it reads.
+template <int EDGES>
+__device__ __forceinline__ void k_diffuse_body(const VelBufs &v, int srcx, int srcy,
+                                               const StepScalars *__restrict__ sc, int comps,
+                                               Bcs bc, const int bx, const int by) {
   const int x = 4 * (bx * VX + threadIdx.x), y = by * VY + threadIdx.y;
   const int W = v.W, H = v.H, P = v.pitch;
   const float a = sc->a, den = sc->den, rden = sc->rden;
-  // both components per thread (independent arrays; twice the loads in
-  // flight per thread)
-  (void)bz;
-  if ((comps & 1) && y >= 1 && y < H - 1 && x <= W - 3 && x + 3 >= 1) {
+  if ((comps & 1) && y >= 1 && y < H - 1 && x <= W - 3) {
     // vx: interior faces x in [1, W-3], y in [1, H-2]
     const float *s = pick(v.vx, srcx);
-    float4 C = ld4(s, P, x, y), N = ld4(s, P, x, y + 1), S = ld4(s, P, x, y - 1);
-    uchar4 K = __ldg(reinterpret_cast<const uchar4 *>(v.cx + (size_t)y * P + x));
-    float L = x >= 1 ? ld(s, P, x - 1, y) : 0.0f;
-    float R = x + 4 < W - 1 ? ld(s, P, x + 4, y) : 0.0f;
+    const float4 C = ld4(s, P, x, y), N = ld4(s, P, x, y + 1), S = ld4(s, P, x, y - 1);
+    const unsigned K = __ldg(reinterpret_cast<const unsigned *>(v.cx + (size_t)y * P + x));
+    const float L = x >= 1 ? ld(s, P, x - 1, y) : 0.0f;
+    const float R = x + 4 < W - 1 ? ld(s, P, x + 4, y) : 0.0f;
+    const float c[4] = {C.x, C.y, C.z, C.w}, e[4] = {C.y, C.z, C.w, R}, w[4] = {L, C.x, C.y, C.z};
+    const float n[4] = {N.x, N.y, N.z, N.w}, ss[4] = {S.x, S.y, S.z, S.w};
     float o[4];
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      unsigned k = compu(K, j);
-      float c = comp(C, j);
-      float t1 = j < 3 ? comp(C, j + 1) : R, t2 = j > 0 ? comp(C, j - 1) : L;
-      float val = 0.0f;
-      val = val + ((k & FC_T1) ? t1 : 0.0f);
-      val = val + ((k & FC_T2) ? t2 : 0.0f);
-      val = val + ((k & FC_T3) ? comp(N, j) : -c);
-      val = val + ((k & FC_T4) ? comp(S, j) : -c);
-      o[j] = (k & FC_M) ? div_rn(c + a * val, den, rden) : 0.0f;
-    }
+    diffuse4(K, c, e, w, n, ss, a, den, rden, o);
     st4_masked(pick(v.vx, 1 - srcx) + (size_t)y * P, x, 1, W - 3, o);
   }
-  if ((comps & 2) && y >= 1 && y < H - 2 && x <= W - 2 && x + 3 >= 1) {
+  if ((comps & 2) && y >= 1 && y < H - 2 && x <= W - 2) {
     // vy: interior faces x in [1, W-2], y in [1, H-3]
     const float *s = pick(v.vy, srcy);
-    float4 C = ld4(s, P, x, y), N = ld4(s, P, x, y + 1), S = ld4(s, P, x, y - 1);
-    uchar4 K = __ldg(reinterpret_cast<const uchar4 *>(v.cy + (size_t)y * P + x));
-    float L = x >= 1 ? ld(s, P, x - 1, y) : 0.0f;
-    float R = x + 4 < W ? ld(s, P, x + 4, y) : 0.0f;
-    float o[4];
+    const float4 C = ld4(s, P, x, y), N = ld4(s, P, x, y + 1), S = ld4(s, P, x, y - 1);
+    const unsigned K = __ldg(reinterpret_cast<const unsigned *>(v.cy + (size_t)y * P + x));
+    const float L = x >= 1 ? ld(s, P, x - 1, y) : 0.0f;
+    const float R = x + 4 < W ? ld(s, P, x + 4, y) : 0.0f;
+    const float c[4] = {C.x, C.y, C.z, C.w};
+    float e[4] = {C.y, C.z, C.w, R}, w[4] = {L, C.x, C.y, C.z};
+    float n[4] = {N.x, N.y, N.z, N.w}, ss[4] = {S.x, S.y, S.z, S.w};
+    if (EDGES == 1 && near_edge(x, y, W, H - 1)) {  // the edges as setVBCs would set them first
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      unsigned k = compu(K, j);
-      float c = comp(C, j);
-      float t3 = j < 3 ? comp(C, j + 1) : R, t4 = j > 0 ? comp(C, j - 1) : L;
-      float val = 0.0f;
-      val = val + ((k & FC_T1) ? comp(S, j) : 0.0f);
-      val = val + ((k & FC_T2) ? comp(N, j) : 0.0f);
-      val = val + ((k & FC_T3) ? t3 : -c);
-      val = val + ((k & FC_T4) ? t4 : -c);
-      o[j] = (k & FC_M) ? div_rn(c + a * val, den, rden) : 0.0f;
+      for (int j = 0; j < 4; j++) {
+        if (x + j == 1) w[j] = vbc_per(bc.w, c[j], w[j]);
+        if (x + j == W - 2) e[j] = vbc_per(bc.e, c[j], e[j]);
+        if (y == 1) ss[j] = vbc_par(bc.s, c[j], ss[j]);
+        if (y == H - 3) n[j] = vbc_par(bc.n, c[j], n[j]);
+      }
     }
+    float o[4];
+    diffuse4(K, c, ss, n, e, w, a, den, rden, o);
     st4_masked(pick(v.vy, 1 - srcy) + (size_t)y * P, x, 1, W - 2, o);
   }
+  // edges, after both components' loads and stores; not unrolled and with the
+  // values read back: few threads come here, and the others should not pay
+  // registers for it
+  if (EDGES && y >= 1 && y < H - 1 && x <= W - 2 &&
+      (near_edge(x, y, W - 1, H) || near_edge(x, y, W, H - 1))) {
+    const float *sx = pick(v.vx, srcx), *sy = pick(v.vy, srcy);
+    float *dx = pick(v.vx, 1 - srcx), *dy = pick(v.vy, 1 - srcy);
+    const float *ex = EDGES == 1 ? dx : sx;
+#pragma unroll 1
+    for (int xx = max(x, 1); xx <= min(x + 3, W - 2); xx++) {
+      if (xx <= W - 3)
+        edge_cells<true>(
+            xx, y, dx[(size_t)y * P + xx], W - 1, H, bc,
+            [&](int a, int b) { return ex[(size_t)b * P + a]; },
+            [&](int a, int b, float q) { dx[(size_t)b * P + a] = q; });
+      if (y <= H - 3)
+        edge_cells<false>(
+            xx, y, dy[(size_t)y * P + xx], W, H - 1, bc,
+            [&](int a, int b) { return sy[(size_t)b * P + a]; },
+            [&](int a, int b, float q) { dy[(size_t)b * P + a] = q; });
+    }
+  }
 }
+template <int EDGES>
 __global__ void __launch_bounds__(256) k_diffuse(VelBufs v, int srcx, int srcy,
-                                                 const StepScalars *__restrict__ sc, int comps) {
+                                                 const StepScalars *__restrict__ sc, int comps,
+                                                 Bcs bc) {
   griddep_wait();
-  k_diffuse_body(v, srcx, srcy, sc, comps, blockIdx.x, blockIdx.y, blockIdx.z);
+  k_diffuse_body<EDGES>(v, srcx, srcy, sc, comps, bc, blockIdx.x, blockIdx.y);
 }
 
 // ----------------------------------------------------------------- advect
@@ -439,9 +550,11 @@ constexpr int AD_TX = 64, AD_TY = 16, AD_H = 4;
 constexpr int AD_SW = AD_TX + 2 * AD_H, AD_SH = AD_TY + 2 * AD_H;
 
 // BIL: the advection option's bilinearSample instead of bicubicSample.
-template <bool BIL>
-__device__ __forceinline__ void k_advect_body(VelBufs v, int srcx, int srcy,
-                                                const StepScalars *__restrict__ sc, const int bx, const int by, const int bz) {
+// EDGES: with the setVBCs that follows in a step, into the buffer written.
+template <bool BIL, bool EDGES>
+__device__ __forceinline__ void k_advect_body(const VelBufs &v, int srcx, int srcy,
+                                              const StepScalars *__restrict__ sc, Bcs bc,
+                                              const int bx, const int by) {
   __shared__ __align__(16) float sxv[AD_SH * AD_SW];
   __shared__ __align__(16) float syv[AD_SH * AD_SW];
   __shared__ __align__(16) uint8_t scx[AD_TY * AD_TX], scy[AD_TY * AD_TX];
@@ -539,16 +652,52 @@ __device__ __forceinline__ void k_advect_body(VelBufs v, int srcx, int srcy,
         float endx = posx - vx2 * cfull;
         float endy = posy - vy2 * cfull;
         float r = SAMPLE(wy, vy, P, W, H - 1, endx, endy - 0.5f);
-        outy[(size_t)y * P + x] = (k & FC_M) ? r : 0.0f;
+        r = (k & FC_M) ? r : 0.0f;
+        // (row H-2 is vy's northern edge: kept only where setVBCs keeps it)
+        if (!EDGES || y < H - 2 || bc.n == UBG_BC_INFLOW) outy[(size_t)y * P + x] = r;
       }
     }
   }
+  if (!EDGES) return;
+  // setVBCs: the edge cells next to the tile's faces, once those are written
+  if (X0 > 1 && X0 + AD_TX <= W - 3 && Y0 > 1 && Y0 + AD_TY <= H - 3) return;
+  __syncthreads();
+#pragma unroll 1
+  for (int i = tid; i < AD_TX * AD_TY; i += 256) {
+    const int ty = i / AD_TX, x = X0 + i - ty * AD_TX, y = Y0 + ty;
+    if (y < 1 || y >= H - 1 || x < 1 || x > W - 2) continue;
+    if (x <= W - 3 && (x == 1 || x == W - 3 || y == 1 || y == H - 2))
+      edge_cells<true>(
+          x, y, outx[(size_t)y * P + x], W - 1, H, bc,
+          [&](int xx, int yy) { return vx[(size_t)yy * P + xx]; },
+          [&](int xx, int yy, float q) { outx[(size_t)yy * P + xx] = q; });
+    if (!(x == 1 || x == W - 2 || y == 1 || y >= H - 3)) continue;
+    if (y < H - 2) {
+      edge_cells<false>(
+          x, y, outy[(size_t)y * P + x], W, H - 1, bc,
+          [&](int xx, int yy) { return vy[(size_t)yy * P + xx]; },
+          [&](int xx, int yy, float q) {
+            // an inflow in the north keeps row H-2, which its own faces write
+            if (yy != H - 2 || bc.n != UBG_BC_INFLOW) outy[(size_t)yy * P + xx] = q;
+          });
+    } else if (bc.n == UBG_BC_INFLOW) {
+      const size_t row = (size_t)y * P;
+      if (!(scy[i] & FC_A)) outy[row + x] = vy[row + x];
+      const float o = outy[row + x];
+      if (x == 1) outy[row] = vbc_per(bc.w, o, vy[row]);
+      if (x == W - 2) outy[row + W - 1] = vbc_per(bc.e, o, vy[row + W - 1]);
+    }
+  }
 }
-template <bool BIL>
+// umax_zero: max|u|, zeroed for the step's gradient kernel to accumulate (the
+// step's dt has been formed from it).
+template <bool BIL, bool EDGES>
 __global__ void __launch_bounds__(256) k_advect(VelBufs v, int srcx, int srcy,
-                                                const StepScalars *__restrict__ sc) {
+                                                const StepScalars *__restrict__ sc, Bcs bc,
+                                                unsigned int *umax_zero) {
   griddep_wait();
-  k_advect_body<BIL>(v, srcx, srcy, sc, blockIdx.x, blockIdx.y, blockIdx.z);
+  if (EDGES && (blockIdx.x | blockIdx.y | threadIdx.x | threadIdx.y) == 0) *umax_zero = 0u;
+  k_advect_body<BIL, EDGES>(v, srcx, srcy, sc, bc, blockIdx.x, blockIdx.y);
 }
 
 // ------------------------------------------------------------- divergence
@@ -620,18 +769,23 @@ __global__ void k_pbc(float *p, int P, int W, int H, Bcs bc) {
 // ---------------------------------------------------------------- gradient
 // Pressure-gradient update; also folds max(|vx|, |vy|) of every interior
 // face (after the update) into *umax_bits for the next step's CFL dt.
-__device__ __forceinline__ void k_gradient_body(VelBufs v, int fx, int fy,
-                                                  const float *__restrict__ p,
-                                                  const StepScalars *__restrict__ sc,
-                                                  unsigned int *umax_bits, const int bx, const int by, const int bz) {
+// EDGES: with setPBC before it (the update reads no edge cell of p) and with
+// the setVBCs that ends a step, into both buffers, its values folded into
+// max|u| too.
+template <bool EDGES>
+__device__ __forceinline__ void k_gradient_body(const VelBufs &v, int fx, int fy, float *p,
+                                                const StepScalars *__restrict__ sc,
+                                                unsigned int *umax_bits, Bcs bc, const int bx,
+                                                const int by) {
   const int x = 4 * (bx * VX + threadIdx.x), y = by * VY + threadIdx.y;
   const int W = v.W, H = v.H, P = v.pitch;
   float m = 0.0f;
   if (y >= 1 && y < H - 1 && x <= W - 2 && x + 3 >= 1) {
     const float ih = sc->ih;
     float *vx = pick(v.vx, fx), *vy = pick(v.vy, fy);
-    float4 P0 = ld4(p, P, x, y), PN = ld4(p, P, x, y + 1);
-    float PR = x + 4 < W ? ld(p, P, x + 4, y) : 0.0f;
+    float4 P0 = *reinterpret_cast<const float4 *>(p + (size_t)y * P + x);
+    float4 PN = *reinterpret_cast<const float4 *>(p + (size_t)(y + 1) * P + x);
+    float PR = x + 4 < W ? p[(size_t)y * P + x + 4] : 0.0f;
     float4 U = *reinterpret_cast<const float4 *>(vx + (size_t)y * P + x);
     float4 V = *reinterpret_cast<const float4 *>(vy + (size_t)y * P + x);
     uchar4 KX = __ldg(reinterpret_cast<const uchar4 *>(v.cx + (size_t)y * P + x));
@@ -650,6 +804,41 @@ __device__ __forceinline__ void k_gradient_body(VelBufs v, int fx, int fy,
     }
     st4_masked(vx + (size_t)y * P, x, 1, W - 3, ox);
     if (y <= H - 3) st4_masked(vy + (size_t)y * P, x, 1, W - 2, oy);
+    if (EDGES && (near_edge(x, y, W - 1, H) || y >= H - 3)) {
+      float *bx_ = pick(v.vx, 1 - fx), *by_ = pick(v.vy, 1 - fy);
+#pragma unroll 1
+      for (int xx = max(x, 1); xx <= min(x + 3, W - 2); xx++) {
+        if (xx <= W - 3)
+          edge_cells<true>(
+              xx, y, vx[(size_t)y * P + xx], W - 1, H, bc, [&](int a, int b) { return vx[(size_t)b * P + a]; },
+              [&](int a, int b, float q) {
+                vx[(size_t)b * P + a] = bx_[(size_t)b * P + a] = q;
+                m = fmaxf(m, fabsf(q));
+              });
+        if (y <= H - 3)
+          edge_cells<false>(
+              xx, y, vy[(size_t)y * P + xx], W, H - 1, bc, [&](int a, int b) { return vy[(size_t)b * P + a]; },
+              [&](int a, int b, float q) {
+                vy[(size_t)b * P + a] = by_[(size_t)b * P + a] = q;
+                m = fmaxf(m, fabsf(q));
+              });
+        // setPBC, x edges first (so a corner is two of them)
+        const float pc = p[(size_t)y * P + xx];
+        const bool w1 = xx == 1, e1 = xx == W - 2;
+        const float l = single_pbc(bc.w, pc), r = single_pbc(bc.e, pc);
+        if (w1) p[(size_t)y * P] = l;
+        if (e1) p[(size_t)y * P + W - 1] = r;
+#pragma unroll 1
+        for (int k = 0; k < 2; k++) {
+          if (y != (k ? H - 2 : 1)) continue;
+          float *row = p + (size_t)(k ? H - 1 : 0) * P;
+          const int side = k ? bc.n : bc.s;
+          row[xx] = single_pbc(side, pc);
+          if (w1) row[0] = single_pbc(side, l);
+          if (e1) row[W - 1] = single_pbc(side, r);
+        }
+      }
+    }
   }
   if (umax_bits) {
     // one atomic per block: per-warp atomics on one address serialise
@@ -664,12 +853,12 @@ __device__ __forceinline__ void k_gradient_body(VelBufs v, int fx, int fy,
     }
   }
 }
-__global__ void __launch_bounds__(256) k_gradient(VelBufs v, int fx, int fy,
-                                                  const float *__restrict__ p,
+template <bool EDGES>
+__global__ void __launch_bounds__(256, 6) k_gradient(VelBufs v, int fx, int fy, float *p,
                                                   const StepScalars *__restrict__ sc,
-                                                  unsigned int *umax_bits) {
+                                                  unsigned int *umax_bits, Bcs bc) {
   griddep_wait();
-  k_gradient_body(v, fx, fy, p, sc, umax_bits, blockIdx.x, blockIdx.y, blockIdx.z);
+  k_gradient_body<EDGES>(v, fx, fy, p, sc, umax_bits, bc, blockIdx.x, blockIdx.y);
 }
 
 // ------------------------------------------------------ staged host I/O
@@ -774,14 +963,6 @@ inline dim3 grid_vec(int w, int h, int z = 1) {
 
 
 // ---------------------------------------------------- multi-member kernels
-__global__ void k_vbc_m(const VbcM *__restrict__ A, const int *__restrict__ bs, int n,
-        unsigned tag, unsigned *err) {
-  griddep_wait();
-  if (!table_ok(bs, n, tag, err)) return;
-  const int m = member_of(bs, n);
-  const VbcM a = A[m];
-  k_vbc_body(a.v, a.fx, a.fy, a.bc, a.do_vx, a.do_vy, a.umax, (int)blockIdx.x - __ldg(bs + m), 0, 0);
-}
 __global__ void __launch_bounds__(256) k_diffuse_m(const DiffuseM *__restrict__ A, const int *__restrict__ bs, int n,
             unsigned tag, unsigned *err) {
   griddep_wait();
@@ -789,17 +970,21 @@ __global__ void __launch_bounds__(256) k_diffuse_m(const DiffuseM *__restrict__ 
   const int m = member_of(bs, n);
   const DiffuseM a = A[m];
   const int l = (int)blockIdx.x - __ldg(bs + m);
-  k_diffuse_body(a.v, a.srcx, a.srcy, a.sc, a.comps, l % a.gx, (l / a.gx) % a.gy, l / (a.gx * a.gy));
+  if (a.edges == 1)
+    k_diffuse_body<1>(a.v, a.srcx, a.srcy, a.sc, 3, a.bc, l % a.gx, l / a.gx);
+  else
+    k_diffuse_body<2>(a.v, a.srcx, a.srcy, a.sc, 3, a.bc, l % a.gx, l / a.gx);
 }
-__global__ void __launch_bounds__(256) k_advect_m(const AdvectM *__restrict__ A, const int *__restrict__ bs, int n,
+__global__ void __launch_bounds__(256, 6) k_advect_m(const AdvectM *__restrict__ A, const int *__restrict__ bs, int n,
            unsigned tag, unsigned *err) {
   griddep_wait();
   if (!table_ok(bs, n, tag, err)) return;
   const int m = member_of(bs, n);
   const AdvectM a = A[m];
   const int l = (int)blockIdx.x - __ldg(bs + m);
+  if (l == 0 && (threadIdx.x | threadIdx.y) == 0) *a.umax_zero = 0u;
   // fused members advect bicubically (the bilinear option is not fused)
-  k_advect_body<false>(a.v, a.srcx, a.srcy, a.sc, l % a.gx, l / a.gx, 0);
+  k_advect_body<false, true>(a.v, a.srcx, a.srcy, a.sc, a.bc, l % a.gx, l / a.gx);
 }
 __global__ void __launch_bounds__(256) k_divergence_m(const DivergenceM *__restrict__ A, const int *__restrict__ bs, int n,
                unsigned tag, unsigned *err) {
@@ -810,24 +995,14 @@ __global__ void __launch_bounds__(256) k_divergence_m(const DivergenceM *__restr
   const int l = (int)blockIdx.x - __ldg(bs + m);
   k_divergence_body(a.vx, a.vy, a.f, a.P, a.W, a.H, a.sc, l % a.gx, l / a.gx, 0);
 }
-__global__ void k_pbc_m(const PbcM *__restrict__ A, const int *__restrict__ bs, int n,
-        unsigned tag, unsigned *err) {
-  griddep_wait();
-  if (!table_ok(bs, n, tag, err)) return;
-  const int m = member_of(bs, n);
-  const PbcM a = A[m];
-  const int l = (int)blockIdx.x - __ldg(bs + m);
-  if (l == 0 && threadIdx.x == 0 && a.umax_zero) *a.umax_zero = 0u;
-  k_pbc_body(a.p, a.P, a.W, a.H, a.bc, l, 0, 0);
-}
-__global__ void __launch_bounds__(256) k_gradient_m(const GradientM *__restrict__ A, const int *__restrict__ bs, int n,
+__global__ void __launch_bounds__(256, 5) k_gradient_m(const GradientM *__restrict__ A, const int *__restrict__ bs, int n,
              unsigned tag, unsigned *err) {
   griddep_wait();
   if (!table_ok(bs, n, tag, err)) return;
   const int m = member_of(bs, n);
   const GradientM a = A[m];
   const int l = (int)blockIdx.x - __ldg(bs + m);
-  k_gradient_body(a.v, a.fx, a.fy, a.p, a.sc, a.umax, l % a.gx, l / a.gx, 0);
+  k_gradient_body<true>(a.v, a.fx, a.fy, a.p, a.sc, a.umax, a.bc, l % a.gx, l / a.gx);
 }
 __global__ void k_cfl_m(const CflM *__restrict__ A, const int *__restrict__ bs, int n, unsigned tag,
                         unsigned *err) {
@@ -863,20 +1038,21 @@ void launch_accum(const VelBufs &v, int fx, int fy, float *ax, float *ay, cudaSt
 }
 
 void launch_diffuse_sweep(const VelBufs &v, int srcx, int srcy, const StepScalars *sc, int comps,
-                          cudaStream_t st) {
+                          cudaStream_t st, int edges, Bcs bc) {
   ProfScope ps_(KC_DIFFUSE, st);
-  launch_pdl(k_diffuse, grid_vec(v.W, v.H), dim3(VX, VY), 0, st, v, srcx, srcy, sc, comps);
+  auto *k = edges == 0 ? k_diffuse<0> : (edges == 1 ? k_diffuse<1> : k_diffuse<2>);
+  launch_pdl(k, grid_vec(v.W, v.H), dim3(VX, VY), 0, st, v, srcx, srcy, sc, comps, bc);
   UBG_LAUNCH_CHECK();
   g_stats.launches++;
 }
 
-void launch_advect(const VelBufs &v, int srcx, int srcy, const StepScalars *sc, cudaStream_t st) {
+void launch_advect(const VelBufs &v, int srcx, int srcy, const StepScalars *sc, cudaStream_t st,
+                   bool edges, Bcs bc, unsigned int *umax_zero) {
   ProfScope ps_(KC_ADVECT, st);
   dim3 grid((v.W + AD_TX - 1) / AD_TX, (v.H + AD_TY - 1) / AD_TY);
-  if (v.advect_bilinear)
-    launch_pdl(k_advect<true>, grid, dim3(BX, BY), 0, st, v, srcx, srcy, sc);
-  else
-    launch_pdl(k_advect<false>, grid, dim3(BX, BY), 0, st, v, srcx, srcy, sc);
+  auto *k = v.advect_bilinear ? (edges ? k_advect<true, true> : k_advect<true, false>)
+                              : (edges ? k_advect<false, true> : k_advect<false, false>);
+  launch_pdl(k, grid, dim3(BX, BY), 0, st, v, srcx, srcy, sc, bc, umax_zero);
   UBG_LAUNCH_CHECK();
   g_stats.launches++;
 }
@@ -906,10 +1082,11 @@ void launch_pbc(float *p, int pitch, int W, int H, Bcs bc, cudaStream_t st) {
   g_stats.launches++;
 }
 
-void launch_gradient(const VelBufs &v, int fx, int fy, const float *p, const StepScalars *sc,
-                     unsigned int *umax_bits, cudaStream_t st) {
+void launch_gradient(const VelBufs &v, int fx, int fy, float *p, const StepScalars *sc,
+                     unsigned int *umax_bits, cudaStream_t st, bool edges, Bcs bc) {
   ProfScope ps_(KC_GRADIENT, st);
-  launch_pdl(k_gradient, grid_vec(v.W, v.H), dim3(VX, VY), 0, st, v, fx, fy, p, sc, umax_bits);
+  launch_pdl(edges ? k_gradient<true> : k_gradient<false>, grid_vec(v.W, v.H), dim3(VX, VY), 0, st,
+             v, fx, fy, p, sc, umax_bits, bc);
   UBG_LAUNCH_CHECK();
   g_stats.launches++;
 }
@@ -954,15 +1131,10 @@ void launch_cfl(const VelBufs &v, int fx, int fy, float cfl, float h, float mu, 
 }  // namespace ubg
 
 namespace ubg {
-int multi_blocks_vbc(const VbcM &a) {
-  int n = (a.v.H - 2) + (a.v.W - 1) + (a.v.H - 3) + a.v.W;
-  return (n + 255) / 256;
-}
 int multi_blocks_diffuse(DiffuseM &a) {
   dim3 g = grid_vec(a.v.W, a.v.H);
   a.gx = (int)g.x;
-  a.gy = (int)g.y;
-  return (int)(g.x * g.y * g.z);
+  return (int)(g.x * g.y);
 }
 int multi_blocks_advect(AdvectM &a) {
   a.gx = (a.v.W + AD_TX - 1) / AD_TX;
@@ -973,7 +1145,6 @@ int multi_blocks_divergence(DivergenceM &a) {
   a.gx = (int)g.x;
   return (int)(g.x * g.y);
 }
-int multi_blocks_pbc(const PbcM &a) { return ((a.H - 2) + a.W + 255) / 256; }
 int multi_blocks_gradient(GradientM &a) {
   dim3 g = grid_vec(a.v.W, a.v.H);
   a.gx = (int)g.x;
@@ -983,9 +1154,6 @@ int multi_blocks_gradient(GradientM &a) {
 void launch_multi_step(int kind, const void *args, const int *bs, int n, int blocks,
                        unsigned tag, unsigned *err, cudaStream_t st) {
   switch (kind) {
-    case MK_VBC:
-      launch_pdl(k_vbc_m, dim3(blocks), dim3(256), 0, st, (const VbcM *)args, bs, n, tag, err);
-      break;
     case MK_DIFFUSE:
       launch_pdl(k_diffuse_m, dim3(blocks), dim3(VX, VY), 0, st, (const DiffuseM *)args, bs, n, tag, err);
       break;
@@ -995,9 +1163,6 @@ void launch_multi_step(int kind, const void *args, const int *bs, int n, int blo
     case MK_DIVERGENCE:
       launch_pdl(k_divergence_m, dim3(blocks), dim3(VX, VY), 0, st, (const DivergenceM *)args, bs,
                  n, tag, err);
-      break;
-    case MK_PBC:
-      launch_pdl(k_pbc_m, dim3(blocks), dim3(256), 0, st, (const PbcM *)args, bs, n, tag, err);
       break;
     case MK_GRADIENT:
       launch_pdl(k_gradient_m, dim3(blocks), dim3(VX, VY), 0, st, (const GradientM *)args, bs, n, tag, err);

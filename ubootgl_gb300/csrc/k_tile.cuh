@@ -109,15 +109,6 @@ __device__ __forceinline__ float scaled_any(float v, float s, float c) {
 // half sweeps stay finite.
 constexpr float kBigSq = 0x1p+120f;
 
-// Unsigned bits without the sign, less one: a value is 0 (all ones) or its
-// division by div_rn's correction is exact when the key is in [lo, hi] of
-// 2^-100 and 2^100.
-__device__ __forceinline__ unsigned key(float v) {
-  const unsigned u = __float_as_uint(v);
-  return u + u - 1u;
-}
-constexpr unsigned kKeyLo = 2u * 0x0d800000u - 1u, kKeyHi = 2u * 0x71800000u - 1u;
-
 // Fills the table: factors (s, c) by code, 32 + code for a cell that is not
 // smoothed; then the weight sums of the prolongation and their reciprocals.
 __device__ __forceinline__ void fill_lut(float2 *lut, int i, const float *wsum,
@@ -165,11 +156,11 @@ __device__ __forceinline__ void prolongate2(const float (&e)[3], const float (&f
   for (int i = 0; i < 6; i++) {  // div_rn's correction
     const float q0 = v[i] * d[i].y;
     q[i] = __fmaf_rn(__fmaf_rn(-q0, d[i].x, v[i]), d[i].y, q0);
-    lo = min(lo, key(v[i]));
+    lo = min(lo, div_key(v[i]));
     m = m + fabsf(v[i]);
   }
   // sums the correction is not exact for (zeros are fine)
-  if (!__all_sync(0xffffffffu, lo >= kKeyLo && m <= 0x1p+100f)) {
+  if (!__all_sync(0xffffffffu, lo >= kDivKeyLo && m <= 0x1p+100f)) {
 #pragma unroll
     for (int i = 0; i < 6; i++) q[i] = div_rn(v[i], d[i].x, d[i].y);
   }

@@ -123,12 +123,18 @@ void launch_vbc(const VelBufs &v, int fx, int fy, Bcs bc, bool do_vx, bool do_vy
 void launch_accum(const VelBufs &v, int fx, int fy, float *ax, float *ay, cudaStream_t st);
 // One Jacobi diffusion sweep, buffer src -> buffer 1-src of each component
 // (simulation.cpp:112-129, 138-155); comps bit 0 = vx, bit 1 = vy.
+// edges: 0 = the sweep alone; 1, 2 = the first / second of a step's sweeps
+// with the setVBCs around them (1: also the vy boundary before it), the
+// edges' values left in the buffer written only.
 void launch_diffuse_sweep(const VelBufs &v, int srcx, int srcy, const StepScalars *sc, int comps,
-                          cudaStream_t st);
+                          cudaStream_t st, int edges = 0, Bcs bc = Bcs{});
 // advect (simulation.cpp:241-354): reads buffer `src` of vx / vy, writes the
 // advected faces into buffer 1-src (faces the reference does not advect keep
 // their value).
-void launch_advect(const VelBufs &v, int srcx, int srcy, const StepScalars *sc, cudaStream_t st);
+// edges: with the setVBCs after it, into the buffer written only; zeroes
+// *umax_zero.
+void launch_advect(const VelBufs &v, int srcx, int srcy, const StepScalars *sc, cudaStream_t st,
+                   bool edges = false, Bcs bc = Bcs{}, unsigned int *umax_zero = nullptr);
 // Divergence into f (simulation.cpp:166-171).
 void launch_divergence(const VelBufs &v, int fx, int fy, float *f, const StepScalars *sc,
                        cudaStream_t st);
@@ -139,8 +145,11 @@ void launch_pbc(float *p, int pitch, int W, int H, Bcs bc, cudaStream_t st);
 // Pressure-gradient update (simulation.cpp:196-207); if umax_bits is set,
 // max(|u|) of the updated interior faces is folded into it (atomicMax on
 // the float bits).
-void launch_gradient(const VelBufs &v, int fx, int fy, const float *p, const StepScalars *sc,
-                     unsigned int *umax_bits, cudaStream_t st);
+// edges: with setPBC before it and the setVBCs after it (both buffers, the
+// edges' values folded into max|u| too).
+void launch_gradient(const VelBufs &v, int fx, int fy, float *p, const StepScalars *sc,
+                     unsigned int *umax_bits, cudaStream_t st, bool edges = false,
+                     Bcs bc = Bcs{});
 // max(|vx|, |vy|) over the front buffers -> dt = cfl*h/max (extension) and
 // the derived scalars.  With umax_ready the maximum left in *umax_bits by
 // the previous step's gradient and boundary kernels is used as is.
@@ -193,6 +202,15 @@ __device__ __forceinline__ float div_rn(float x, float d, float r) {
   return x / d;
 }
 
+// Unsigned bits of v without the sign, less one: its division by div_rn's
+// correction is exact when v is 0 (all ones) or the key is at least kDivKeyLo
+// (2^-100) and |v| at most 2^100.
+__device__ __forceinline__ unsigned div_key(float v) {
+  const unsigned u = __float_as_uint(v);
+  return u + u - 1u;
+}
+constexpr unsigned kDivKeyLo = 2u * 0x0d800000u - 1u;
+
 // Compares div_rn(x[i], d, RN(1/d)) with x[i] / d bit for bit on the device
 // (NaNs compare equal); host arrays.
 int selftest_div_rn(const float *x, int n, float d, unsigned *mismatches);
@@ -214,23 +232,20 @@ void launch_shift_map(VelBufs &v, int fx, int fy, const float *p_in, float *p_ou
 // and each block runs the single-simulation kernel body on its member's
 // arguments.  Arguments live in a device table built by the host.
 enum MultiKind {
-  MK_VBC = 0, MK_DIFFUSE, MK_ADVECT, MK_DIVERGENCE, MK_PBC, MK_GRADIENT, MK_CFL, MK_MG, MK_TAIL
-};
-struct VbcM {
-  VelBufs v;
-  int fx, fy, do_vx, do_vy;
-  Bcs bc;
-  unsigned int *umax;
+  MK_DIFFUSE = 0, MK_ADVECT, MK_DIVERGENCE, MK_GRADIENT, MK_CFL, MK_MG, MK_TAIL
 };
 struct DiffuseM {
   VelBufs v;
-  int srcx, srcy, comps, gx, gy;
+  int srcx, srcy, edges, gx;
   const StepScalars *sc;
+  Bcs bc;
 };
 struct AdvectM {
   VelBufs v;
   int srcx, srcy, gx;
   const StepScalars *sc;
+  Bcs bc;
+  unsigned int *umax_zero;
 };
 struct DivergenceM {
   const float *vx, *vy;
@@ -238,18 +253,13 @@ struct DivergenceM {
   int P, W, H, gx;
   const StepScalars *sc;
 };
-struct PbcM {
-  float *p;
-  int P, W, H;
-  Bcs bc;
-  unsigned int *umax_zero;  // zeroed by the member's first thread (next: gradient)
-};
 struct GradientM {
   VelBufs v;
   int fx, fy, gx;
-  const float *p;
+  float *p;
   const StepScalars *sc;
   unsigned int *umax;
+  Bcs bc;
 };
 struct CflM {
   const unsigned int *umax;
@@ -294,11 +304,9 @@ struct MultiSlot {
   std::vector<int> bs;
 };
 // Blocks a member needs for each kind (and fills the grid width fields).
-int multi_blocks_vbc(const VbcM &a);
 int multi_blocks_diffuse(DiffuseM &a);
 int multi_blocks_advect(AdvectM &a);
 int multi_blocks_divergence(DivergenceM &a);
-int multi_blocks_pbc(const PbcM &a);
 int multi_blocks_gradient(GradientM &a);
 // Launches over n members (device tables args, bs; total blocks).
 void launch_multi_step(int kind, const void *args, const int *bs, int n, int blocks,
