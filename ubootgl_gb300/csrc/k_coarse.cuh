@@ -409,6 +409,7 @@ __device__ __forceinline__ void run(const Args<S> &args, unsigned char *smem) {
   for (int v = 0; v < 2 * a.nlev - 1; v++) {
     const bool up = v >= a.nlev;
     const int t = up ? 2 * a.nlev - 2 - v : v;
+    if (v == 2 * a.nlev - 2) griddep_launch();
     if (wid < a.L[t].warps) visit<S>(a, t, up, smem);
     // the next level's warps read what these wrote
     __syncthreads();

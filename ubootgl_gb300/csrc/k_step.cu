@@ -422,6 +422,7 @@ __global__ void __launch_bounds__(256) k_diffuse(VelBufs v, int srcx, int srcy,
                                                  Bcs bc) {
   griddep_wait();
   k_diffuse_body<EDGES>(v, srcx, srcy, sc, comps, bc, blockIdx.x, blockIdx.y);
+  griddep_launch();
 }
 
 // ----------------------------------------------------------------- advect
@@ -658,6 +659,7 @@ __device__ __forceinline__ void k_advect_body(const VelBufs &v, int srcx, int sr
       }
     }
   }
+  griddep_launch();
   if (!EDGES) return;
   // setVBCs: the edge cells next to the tile's faces, once those are written
   if (X0 > 1 && X0 + AD_TX <= W - 3 && Y0 > 1 && Y0 + AD_TY <= H - 3) return;
@@ -724,6 +726,7 @@ __global__ void __launch_bounds__(256) k_divergence(const float *__restrict__ vx
                                                     const StepScalars *__restrict__ sc) {
   griddep_wait();
   k_divergence_body(vx, vy, f, P, W, H, sc, blockIdx.x, blockIdx.y, blockIdx.z);
+  griddep_launch();
 }
 
 __global__ void k_sinks(float *f, int P, const SinkCell *cells, int n) {
@@ -859,6 +862,7 @@ __global__ void __launch_bounds__(256, 6) k_gradient(VelBufs v, int fx, int fy, 
                                                   unsigned int *umax_bits, Bcs bc) {
   griddep_wait();
   k_gradient_body<EDGES>(v, fx, fy, p, sc, umax_bits, bc, blockIdx.x, blockIdx.y);
+  griddep_launch();
 }
 
 // ------------------------------------------------------ staged host I/O

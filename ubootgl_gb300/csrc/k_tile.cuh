@@ -457,6 +457,7 @@ __device__ __forceinline__ void run(const MgArgsT<S, SC> &a, const int region,
   else
     sweeps(std::integral_constant<int, 1>{});
 
+  griddep_launch();
   // ---- store (ya and yb are multiples of R: all of a warp's rows or none)
   if (inner) {
     if (mine && y >= ya && y < yb) {
