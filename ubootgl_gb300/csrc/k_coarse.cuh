@@ -62,7 +62,7 @@ constexpr int kArgs = 0, kArgsBytes = 1024, kXch = kArgs + kArgsBytes,
 // A level's registers: two rows, columns (0, 2) and (1, 3).
 struct Regs {
   float2 A[2], B[2], FA[2], FB[2];     // e and f h^2
-  float2 sA[2], cA[2], sB[2], cB[2];  // factors (tile::scaled2)
+  float2 sA[2], sB[2];                 // factors (tile::scaled2)
   unsigned cw[2];
 };
 // Where a lane is in its level.
@@ -123,9 +123,9 @@ __device__ __forceinline__ void half(Regs &q, const Place &pl, float2 *xch, cons
     }
     const float2 we = make_float2(W.x + E.x, W.y + E.y);
     const float2 v = tile::add2(tile::add2(tile::add2(we, S), N), onB ? q.FB[r] : q.FA[r]);
-    const float2 s = onB ? q.sB[r] : q.sA[r], c = onB ? q.cB[r] : q.cA[r];
-    r2[r] = CAREFUL ? make_float2(tile::scaled_any(v.x, s.x, c.x), tile::scaled_any(v.y, s.y, c.y))
-                    : tile::scaled2(v, s, c);
+    const float2 s = onB ? q.sB[r] : q.sA[r];
+    r2[r] = CAREFUL ? make_float2(tile::scaled_any(v.x, s.x), tile::scaled_any(v.y, s.y))
+                    : tile::scaled2(v, s);
   }
   (RED ? q.B[0] : q.A[0]) = r2[0];
   (RED ? q.A[1] : q.B[1]) = r2[1];
@@ -224,21 +224,19 @@ __device__ __forceinline__ void visit(const Args<S> &a, const int t, const bool 
     }
     float p[4] = {p4.x, p4.y, p4.z, p4.w};
     float F[4] = {fv.x * hh * hh, fv.y * hh * hh, fv.z * hh * hh, fv.w * hh * hh};
-    float2 s[4];
+    float s[4];
 #pragma unroll
     for (int b = 0; b < 4; b++) {
       if (up) p[b] = p[b] + u[r][b];
       if (!((c >> (8 * b)) & C_CENTER)) p[b] = F[b] = 0.0f;
-      s[b] = lut[(c >> (8 * b)) & 0x1fu];
+      s[b] = reinterpret_cast<const float *>(lut)[(c >> (8 * b)) & 0x1fu];
     }
     q.A[r] = make_float2(p[0], p[2]);
     q.B[r] = make_float2(p[1], p[3]);
     q.FA[r] = make_float2(F[0], F[2]);
     q.FB[r] = make_float2(F[1], F[3]);
-    q.sA[r] = make_float2(s[0].x, s[2].x);
-    q.cA[r] = make_float2(s[0].y, s[2].y);
-    q.sB[r] = make_float2(s[1].x, s[3].x);
-    q.cB[r] = make_float2(s[1].y, s[3].y);
+    q.sA[r] = make_float2(s[0], s[2]);
+    q.sB[r] = make_float2(s[1], s[3]);
     q.cw[r] = c;
     sq = f2_fma(q.FB[r], q.FB[r], f2_fma(q.FA[r], q.FA[r], sq));
     sq = f2_fma(q.B[r], q.B[r], f2_fma(q.A[r], q.A[r], sq));

@@ -11,9 +11,8 @@
 //
 // A solid cell holds 0, so a sum needs no flag tests: the flags only decide
 // what it is divided by.  A warp whose cells and all their neighbours are
-// fluid takes val / 4; any other reads two factors per cell (s = 1/n and its
-// correction for n = 3) from shared memory, where the block put them when it
-// loaded the codes.
+// fluid takes val / 4; any other reads a factor per cell (1/n) from shared
+// memory, where the block put them when it loaded the codes.
 //
 // After half sweep i, the cells within i of the region's edge are no longer
 // exact, so regions overlap by 16 columns and rows and store what is 8 or
@@ -22,12 +21,14 @@
 // What bounds it: instruction issue and the FP32 pipe on large levels, the
 // latency of loads, six barriers and one pass through the code on small ones.
 // Against tiles in shared memory (red/black-split, 112 x 50 and 48 x 16
-// cells), ncu: level 0 of 4096x2048 56 us (89 with the residual, 98 with the
-// prolongation), 2048x1024 18 us (33, 38), 1024x512 8 us (18, 20), 256x128
-// 6 us.  Of those 56 us, bounds checks outside the blocks that need them, the
+// cells), ncu: level 0 of 4096x2048 52-55 us (89 with the residual, 98 with
+// the prolongation), 2048x1024 17 us (33, 38), 1024x512 8 us (18, 20), 256x128
+// 6 us.  Of the gain, bounds checks outside the blocks that need them, the
 // packed magnitude check and W + E as scalar additions (no register moves)
-// are 2 us (32.4 -> 25.5 M warp instructions).  Regions of 8 rows per warp
-// (8 warps), and of 128 x 32 cells, are slower there (58-60, 65 us).
+// are 2 us (32.4 -> 25.5 M warp instructions), f kept in shared memory for
+// the residual and one factor per cell another 2 (4096x2048 steps 660 ->
+// 647 us).  Regions of 8 rows per warp (8 warps), and of 128 x 32 cells, are
+// slower there (58-60, 65 us).
 #pragma once
 
 namespace ubg {
@@ -43,10 +44,10 @@ constexpr unsigned kFull = 0x1f1f1f1fu;
 __host__ __device__ constexpr int regions(int c, int n) {
   return c <= n ? 1 : (c - 2 * kHalo + n - 2 * kHalo - 1) / (n - 2 * kHalo);
 }
-// Shared memory: factors (16 bytes per pair), exchanged rows of each warp
+// Shared memory: f and factors of each row (512 bytes each), exchanged rows of each warp
 // (and of one below and one above: zeros), restriction rows, table of factors
 // by code and of the prolongation's weight sums.
-constexpr int kLutBytes = (64 + 5) * 8;
+constexpr int kLutBytes = 64 * 4 + 5 * 8;
 template <int R, int NW>
 struct Mem {
   static constexpr int fac = 0, xch = fac + R * NW * 1024, res = xch + 2 * (NW + 2) * 512,
@@ -90,26 +91,27 @@ __device__ __forceinline__ float2 rnd2(float2 v) {
 }
 
 // val / n of a pair: s = 1/n (the rounded third for n = 3; 0 for a solid cell
-// or one without fluid neighbours), c = s for n = 3, else 0.  n = 1, 2, 4
-// are exact products; n = 3 is Markstein's correction, whose remainder
-// v - 3 q is exact for every finite v, subnormal results included (3 has two
-// bits).  For finite sums only: 0 * infinity would be NaN.
-__device__ __forceinline__ float2 scaled2(float2 v, float2 s, float2 c) {
+// or one without fluid neighbours).  n = 1, 2, 4 are exact products; n = 3 is
+// Markstein's correction, whose remainder v - 3 q is exact for every finite v,
+// subnormal results included (3 has two bits).  For finite sums only: 0 *
+// infinity would be NaN.
+__device__ __forceinline__ float2 scaled2(float2 v, float2 s) {
+  const float2 c = make_float2(s.x == kThird ? kThird : 0.0f, s.y == kThird ? kThird : 0.0f);
   const float2 q = f2_mul(v, s);
   return f2_fma(f2_fma(q, f2(-3.0f), v), c, q);
 }
 // The same for any v (a solid cell is 0 whatever its sum).
-__device__ __forceinline__ float scaled_any(float v, float s, float c) {
+__device__ __forceinline__ float scaled_any(float v, float s) {
   const float q = v * s;
-  const float q3 = __fmaf_rn(__fmaf_rn(-q, 3.0f, v), c, q);
-  const float n = (c != 0.0f && fabsf(v) < __int_as_float(0x7f800000)) ? q3 : q;
+  const float q3 = __fmaf_rn(__fmaf_rn(-q, 3.0f, v), s, q);
+  const float n = (s == kThird && fabsf(v) < __int_as_float(0x7f800000)) ? q3 : q;
   return s != 0.0f ? n : 0.0f;
 }
 // Bound of the sum of squares of what a lane holds under which six (ten)
 // half sweeps stay finite.
 constexpr float kBigSq = 0x1p+120f;
 
-// Fills the table: factors (s, c) by code, 32 + code for a cell that is not
+// Fills the table: factors by code, 32 + code for a cell that is not
 // smoothed; then the weight sums of the prolongation and their reciprocals.
 __device__ __forceinline__ void fill_lut(float2 *lut, int i, const float *wsum,
                                          const float *rwsum) {
@@ -117,9 +119,9 @@ __device__ __forceinline__ void fill_lut(float2 *lut, int i, const float *wsum,
     const int n = __popc((i >> 1) & 15);
     float s = n == 4 ? 0.25f : (n == 3 ? kThird : (n == 2 ? 0.5f : (n == 1 ? 1.0f : 0.0f)));
     if (!(i & (int)C_CENTER) || i >= 32) s = 0.0f;
-    lut[i] = make_float2(s, s == kThird ? s : 0.0f);
+    reinterpret_cast<float *>(lut)[i] = s;
   } else if (i < 69) {
-    lut[i] = make_float2(wsum[i - 64], rwsum[i - 64]);
+    lut[i - 32] = make_float2(wsum[i - 64], rwsum[i - 64]);
   }
 }
 
@@ -137,17 +139,17 @@ __device__ __forceinline__ void prolongate2(const float (&e)[3], const float (&f
                       ((e[1] + f[2]) + e[2]) + f[1]};
   float2 d[6];
   if (__all_sync(0xffffffffu, (g & g1) == 0x010101u)) {
-    const float2 d2 = lut[66], d4 = lut[68];
+    const float2 d2 = lut[34], d4 = lut[36];
 #pragma unroll
     for (int i = 0; i < 6; i++) d[i] = i == 3 || i == 5 ? d4 : d2;
   } else {
     const unsigned t = g + g1;  // flag sums of the column pairs, a byte each
-    d[0] = lut[64 + (g & 1u) + ((g >> 8) & 1u)];
-    d[1] = lut[64 + ((g >> 8) & 1u) + (g >> 16)];
-    d[2] = lut[64 + (t & 0xffu)];
-    d[3] = lut[64 + (t & 0xffu) + ((t >> 8) & 0xffu)];
-    d[4] = lut[64 + ((t >> 8) & 0xffu)];
-    d[5] = lut[64 + ((t >> 8) & 0xffu) + (t >> 16)];
+    d[0] = lut[32 + (g & 1u) + ((g >> 8) & 1u)];
+    d[1] = lut[32 + ((g >> 8) & 1u) + (g >> 16)];
+    d[2] = lut[32 + (t & 0xffu)];
+    d[3] = lut[32 + (t & 0xffu) + ((t >> 8) & 0xffu)];
+    d[4] = lut[32 + ((t >> 8) & 0xffu)];
+    d[5] = lut[32 + ((t >> 8) & 0xffu) + (t >> 16)];
   }
   float q[6];
   unsigned lo = ~0u;
@@ -214,17 +216,23 @@ __device__ __forceinline__ void run(const MgArgsT<S, SC> &a, const int region,
   // stored columns and rows
   const bool mine = (lane >= 2 || first) && (lane < 30 || sx == nsx - 1);
   const int ya = sy == 0 ? 0 : y0 + kHalo, yb = sy == nsy - 1 ? y0 + RY : y0 + RY - kHalo;
-  float4 *const fac = reinterpret_cast<float4 *>(smem + M::fac) + (R * wid) * 64 + lane;
+  // a row's f (16 or 8 bytes per lane), then its factors: pairs (0, 2), (1, 3)
+  unsigned char *const rowm = smem + M::fac + R * wid * 1024;
+  auto frow = [&](int r) { return reinterpret_cast<S *>(rowm + r * 1024) + 4 * lane; };
+  auto fac = [&](int r, int pair) -> float2 & {
+    return reinterpret_cast<float2 *>(rowm + r * 1024 + 512)[32 * pair + lane];
+  };
   float2 *const xch = reinterpret_cast<float2 *>(smem + M::xch) + lane;
   float2 *const res = reinterpret_cast<float2 *>(smem + M::res) + lane;
   const float2 *const lut = reinterpret_cast<const float2 *>(smem + M::lut);
+  const float *const factor = reinterpret_cast<const float *>(lut);
   // exchanged rows: buffer (half sweep parity), warp, its first or last row
   auto slot = [&](int buf, int wd, int lastrow) -> float2 & {
     return xch[((buf * (NW + 2) + 1 + wd) * 2 + lastrow) * 32];
   };
 
-  // ---- loads: all in flight together; f is copied to where the lane's
-  // factors will be (16 registers less while the rest arrives)
+  // ---- loads: all in flight together; f is copied to shared memory (16
+  // registers less while the rest arrives, and there for the residual)
   const bool inner = !first && !has_east && y0 > 0 && y0 + RY < h - 1;  // no bounds to check
   const bool colok = X < w;
   const size_t o0 = (size_t)y * P + X;
@@ -233,7 +241,7 @@ __device__ __forceinline__ void run(const MgArgsT<S, SC> &a, const int region,
   unsigned inmask = ~0u;  // columns that are smoothed
   if (inner) {
 #pragma unroll
-    for (int r = 0; r < R; r++) copy_async<4 * (int)sizeof(S)>(fac + r * 64, a.rhs + o0 + r * P, true);
+    for (int r = 0; r < R; r++) copy_async<4 * (int)sizeof(S)>(frow(r), a.rhs + o0 + r * P, true);
     if (!a.zero_init) {
 #pragma unroll
       for (int r = 0; r < R; r++) pv[r] = St::ldg4(a.in + o0 + r * P);
@@ -255,7 +263,7 @@ __device__ __forceinline__ void run(const MgArgsT<S, SC> &a, const int region,
 #pragma unroll
     for (int r = 0; r < R; r++) {
       const bool ok = colok && y + r < h;
-      copy_async<4 * (int)sizeof(S)>(fac + r * 64, a.rhs + (ok ? o0 + r * P : 0), ok);
+      copy_async<4 * (int)sizeof(S)>(frow(r), a.rhs + (ok ? o0 + r * P : 0), ok);
       pv[r] = make_float4(0.f, 0.f, 0.f, 0.f);
       cw[r] = 0u;
       if (ok) {
@@ -345,7 +353,7 @@ __device__ __forceinline__ void run(const MgArgsT<S, SC> &a, const int region,
 #pragma unroll
   for (int r = 0; r < R; r++) {
     float *p = &pv[r].x;
-    const float4 fv = St::lds4(reinterpret_cast<const S *>(fac + r * 64));
+    const float4 fv = St::lds4(frow(r));
     float F[4] = {fv.x * hh * hh, fv.y * hh * hh, fv.z * hh * hh, fv.w * hh * hh};
     if (!full) {
       const bool brow = y + r == 0 || y + r == h - 1;
@@ -355,11 +363,11 @@ __device__ __forceinline__ void run(const MgArgsT<S, SC> &a, const int region,
 #pragma unroll
       for (int b = 0; b < 4; b++)
         if (!((c >> (8 * b)) & C_CENTER)) p[b] = F[b] = 0.0f;
-      float2 s[4];
+      float s[4];
 #pragma unroll
-      for (int b = 0; b < 4; b++) s[b] = lut[(c >> (8 * b)) & 0x3fu];
-      fac[r * 64] = make_float4(s[0].x, s[2].x, s[0].y, s[2].y);
-      fac[r * 64 + 32] = make_float4(s[1].x, s[3].x, s[1].y, s[3].y);
+      for (int b = 0; b < 4; b++) s[b] = factor[(c >> (8 * b)) & 0x3fu];
+      fac(r, 0) = make_float2(s[0], s[2]);
+      fac(r, 1) = make_float2(s[1], s[3]);
     }
     A[r] = make_float2(p[0], p[2]);
     B[r] = make_float2(p[1], p[3]);
@@ -420,11 +428,11 @@ __device__ __forceinline__ void run(const MgArgsT<S, SC> &a, const int region,
       if (MODE == 0) {
         n = make_float2(v.x * 0.25f, v.y * 0.25f);
       } else {
-        const float4 s = fac[r * 64 + (onB ? 32 : 0)];
+        const float2 s = fac(r, onB ? 1 : 0);
         if (MODE == 3)
-          n = make_float2(scaled_any(v.x, s.x, s.z), scaled_any(v.y, s.y, s.w));
+          n = make_float2(scaled_any(v.x, s.x), scaled_any(v.y, s.y));
         else
-          n = scaled2(v, make_float2(s.x, s.y), make_float2(s.z, s.w));
+          n = scaled2(v, s);
       }
       n = rnd2<S>(n);
       if (EDGE) {  // cells on the domain's edge keep their values
@@ -530,16 +538,6 @@ __device__ __forceinline__ void run(const MgArgsT<S, SC> &a, const int region,
     // ---- residual (calculateResidualField, pressure_solver.cpp:91-116) of
     // every row, restricted (pressure_solver.cpp:118-132): a lane holds the
     // columns over coarse columns X/2 and X/2 + 1
-    float4 fr[R];  // f: where it was copied to, unless factors took the place
-#pragma unroll
-    for (int r = 0; r < R; r++) {
-      if (full) {
-        fr[r] = St::lds4(reinterpret_cast<const S *>(fac + r * 64));
-      } else {
-        fr[r] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (colok && y + r < h) fr[r] = St::ldg4(a.rhs + (size_t)(y + r) * P + X);
-      }
-    }
     // rows below and above: (0, 2) and (1, 3) from the two buffers
     const float2 bA = slot(1, wid - 1, 1), bB = slot(0, wid - 1, 1);
     const float2 tA = slot(0, wid + 1, 0), tB = slot(1, wid + 1, 0);
@@ -552,7 +550,8 @@ __device__ __forceinline__ void run(const MgArgsT<S, SC> &a, const int region,
       const float l = __shfl_up_sync(0xffffffffu, B[r].y, 1);
       const float rr = __shfl_down_sync(0xffffffffu, A[r].x, 1);
       const float C4[4] = {A[r].x, B[r].x, A[r].y, B[r].y};
-      const float F4[4] = {fr[r].x, fr[r].y, fr[r].z, fr[r].w};
+      const float4 fv = St::lds4(frow(r));
+      const float F4[4] = {fv.x, fv.y, fv.z, fv.w};
       float q[4];
       if (full) {
         const float2 va = add2(add2(make_float2(l + B[r].x, B[r].x + B[r].y), SA), NA);
