@@ -52,10 +52,6 @@ constexpr int BX = 32, BY = 8;
 __device__ __forceinline__ float ld(const float *p, int pitch, int x, int y) {
   return __ldg(p + (size_t)y * pitch + x);
 }
-__device__ __forceinline__ float fl(const uint8_t *f, int pitch, int x, int y) {
-  return (float)__ldg(f + (size_t)y * pitch + x);
-}
-
 // VBCPar / VBCPer / singlePBC, simulation.cpp:22-78.
 __device__ __forceinline__ float vbc_par(int bc, float a, float b) {
   if (bc == UBG_BC_INFLOW) return b;
@@ -434,23 +430,11 @@ __global__ void __launch_bounds__(256) k_diffuse(VelBufs v, int srcx, int srcy,
 struct CrW {
   float a, b, c, d;
 };
-__device__ __forceinline__ CrW cr_weights(float t) {
-  float t2 = t * t;
-  CrW w;
-  w.a = t * __fmaf_rn(t, __fmaf_rn(-0.5f, t, 1.0f), -0.5f);
-  w.b = __fmaf_rn(t2, __fmaf_rn(1.5f, t, -2.5f), 1.0f);
-  w.c = t * __fmaf_rn(t, __fmaf_rn(-1.5f, t, 2.0f), 0.5f);
-  w.d = t2 * __fmaf_rn(0.5f, t, -0.5f);
-  return w;
-}
 __device__ __forceinline__ float cr_dot(const CrW &w, float A, float B, float C, float D) {
   return __fmaf_rn(w.d, D, __fmaf_rn(w.c, C, __fmaf_rn(w.b, B, w.a * A)));
 }
 
-
-
-// The two weight sets of one sample at once: lane x for t.x, lane y for t.y
-// (the operations of cr_weights, lane by lane).
+// Two weight sets at once, lane by lane.
 struct CrW2 {
   float2 a, b, c, d;
 };
@@ -462,6 +446,9 @@ __device__ __forceinline__ CrW2 cr_weights2(float2 t) {
   w.c = f2_mul(t, f2_fma(t, f2_fma(f2(-1.5f), t, f2(2.0f)), f2(0.5f)));
   w.d = f2_mul(t2, f2_fma(f2(0.5f), t, f2(-0.5f)));
   return w;
+}
+__device__ __forceinline__ float2 cr_dot2(const CrW2 &w, float2 A, float2 B, float2 C, float2 D) {
+  return f2_fma(w.d, D, f2_fma(w.c, C, f2_fma(w.b, B, f2_mul(w.a, A))));
 }
 
 // Catmull-Rom sample from 16 values (rows r0..r3 of a 4x4 stencil): the
@@ -483,6 +470,19 @@ __device__ __forceinline__ float bicubic16(const float *b, int stride, float sx,
   return cr_dot(wx, col[0].x, col[0].y, col[1].x, col[1].y);
 }
 
+// Shared memory by 32-bit address (kept in a register over a loop, where a
+// pointer's window base would be formed again for each access).
+__device__ __forceinline__ float lds(unsigned a) {
+  float f;
+  asm("ld.shared.f32 %0, [%1];" : "=f"(f) : "r"(a));
+  return f;
+}
+__device__ __forceinline__ unsigned lds8(unsigned a) {
+  unsigned r;
+  asm("ld.shared.u8 %0, [%1];" : "=r"(r) : "r"(a));
+  return r;
+}
+
 // A staged window of one staggered component: region [sx0, sx0+SW) x
 // [sy0, sy0+SH) of the grid in shared memory.
 struct Win {
@@ -490,29 +490,101 @@ struct Win {
   int sx0, sy0;
 };
 
-// bicubicSample (interpolators.hpp:92-206) reading the 4x4 stencil from the
-// shared-memory window when it lies inside, else from global memory.
-template <int SW, int SH>
-__device__ __forceinline__ float bicubic_win(const Win &wn, const float *__restrict__ g, int P,
-                                             int gw, int gh, float cx, float cy) {
-  float hx = (float)gw - 3.0f, hy = (float)gh - 3.0f;
-  cx = cx < hx ? cx : hx;
-  cx = cx > 3.0f ? cx : 3.0f;
-  cy = cy < hy ? cy : hy;
-  cy = cy > 3.0f ? cy : 3.0f;
-  int ix = (int)cx, iy = (int)cy;
-  float sx = cx - (float)ix, sy = cy - (float)iy;
-  int lx = ix - 1 - wn.sx0, ly = iy - 1 - wn.sy0;
-  if (lx >= 0 && lx + 3 < SW && ly >= 0 && ly + 3 < SH)
-    return bicubic16(wn.s + ly * SW + lx, SW, sx, sy);
-  return bicubic16(g + (size_t)(iy - 1) * P + (ix - 1), P, sx, sy);
+// bicubicSample (interpolators.hpp:92-206) with the stencil in global memory.
+__device__ __noinline__ float bicubic_global(const float *__restrict__ g, int P, float hx, float hy,
+                                             float cx, float cy) {
+  cx = fmaxf(fminf(cx, hx), 3.0f);
+  cy = fmaxf(fminf(cy, hy), 3.0f);
+  const int ix = (int)cx, iy = (int)cy;
+  return bicubic16(g + (size_t)(iy - 1) * P + (ix - 1), P, cx - (float)ix, cy - (float)iy);
 }
+
+// Two bicubic samples at once, lane x of vx at (cx.x, cy.x) and lane y of vy
+// at (cx.y, cy.y), the stencils from the shared-memory windows when both lie
+// inside, else from global memory.  The coordinates are clamped to [3, h] as
+// the reference clamps them (fminf and fmaxf give a NaN the same bounds), so
+// c + 2^23 rounded down holds the integer part in its low bits, for grids of
+// up to 2^23 cells a side; for wider ones the caller's offsets ox, oy (2^23's
+// bits and the window's corner) leave every stencil outside.
+struct Pair {
+  const float *sx, *sy, *gx, *gy;
+  float hxx, hxy, hyx, hyy;  // upper bounds: of vx's grid in x, y, of vy's
+  unsigned ox, oy;
+  int P;
+};
+template <int SW, int SH, int SS>
+__device__ __forceinline__ float2 bicubic_pair(const Pair &q, float2 cx, float2 cy) {
+  const float2 x = make_float2(fmaxf(fminf(cx.x, q.hxx), 3.0f), fmaxf(fminf(cx.y, q.hyx), 3.0f));
+  const float2 y = make_float2(fmaxf(fminf(cy.x, q.hxy), 3.0f), fmaxf(fminf(cy.y, q.hyy), 3.0f));
+  const float2 tx = f2_add_rm(x, f2(0x1p23f)), ty = f2_add_rm(y, f2(0x1p23f));
+  const unsigned ax = __float_as_uint(tx.x) - q.ox, bx = __float_as_uint(tx.y) - q.ox;
+  const unsigned ay = __float_as_uint(ty.x) - q.oy, by = __float_as_uint(ty.y) - q.oy;
+  if (max(ax, bx) <= SW - 4 && max(ay, by) <= SH - 4) {
+    const CrW2 wx = cr_weights2(f2_fma(f2_add_rm(tx, f2(-0x1p23f)), f2(-1.0f), x));
+    const CrW2 wy = cr_weights2(f2_fma(f2_add_rm(ty, f2(-0x1p23f)), f2(-1.0f), y));
+    const float *a = q.sx + (ay * SS + ax), *b = q.sy + (by * SS + bx);
+    float2 col[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+      col[j] = cr_dot2(wy, make_float2(a[j], b[j]), make_float2(a[SS + j], b[SS + j]),
+                       make_float2(a[2 * SS + j], b[2 * SS + j]),
+                       make_float2(a[3 * SS + j], b[3 * SS + j]));
+    return cr_dot2(wx, col[0], col[1], col[2], col[3]);
+  }
+  return make_float2(bicubic_global(q.gx, q.P, q.hxx, q.hxy, cx.x, cy.x),
+                     bicubic_global(q.gy, q.P, q.hyx, q.hyy, cx.y, cy.y));
+}
+
+// The same where every stencil lies in the windows, in two parts: the stencils'
+// places and weights, and the values; addresses are 32-bit ones of shared
+// memory, with 2^23's bits and the window's corner taken off the bases.
+template <int SS, int DY>  // vy's window is DY bytes after vx's
+struct Near {
+  float hxx, hxy, hyx, hyy;
+  unsigned base;
+  struct At {
+    CrW2 wx, wy;
+    unsigned a, b;
+  };
+  // CLAMP: false where no trace of the block reaches the domain's edge
+  template <bool CLAMP>
+  __device__ __forceinline__ At at(float2 x, float2 y) const {
+    if (CLAMP) {
+      x = make_float2(fmaxf(fminf(x.x, hxx), 3.0f), fmaxf(fminf(x.y, hyx), 3.0f));
+      y = make_float2(fmaxf(fminf(y.x, hxy), 3.0f), fmaxf(fminf(y.y, hyy), 3.0f));
+    }
+    const float2 tx = f2_add_rm(x, f2(0x1p23f)), ty = f2_add_rm(y, f2(0x1p23f));
+    At r;
+    r.wx = cr_weights2(f2_fma(f2_add_rm(tx, f2(-0x1p23f)), f2(-1.0f), x));
+    r.wy = cr_weights2(f2_fma(f2_add_rm(ty, f2(-0x1p23f)), f2(-1.0f), y));
+    r.a = base + 4u * (__float_as_uint(ty.x) * SS + __float_as_uint(tx.x));
+    r.b = base + 4u * (__float_as_uint(ty.y) * SS + __float_as_uint(tx.y));
+    return r;
+  }
+  template <int LANE>
+  static __device__ __forceinline__ void load(unsigned at, float2 (&v)[16]) {
+#pragma unroll
+    for (int k = 0; k < 16; k++) {
+      const float f = lds(at + 4u * ((k / 4) * SS + k % 4) + (LANE ? DY : 0));
+      if (LANE == 0)
+        v[k].x = f;
+      else
+        v[k].y = f;
+    }
+  }
+  static __device__ __forceinline__ float2 value(const At &r, const float2 (&v)[16]) {
+    float2 col[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) col[j] = cr_dot2(r.wy, v[j], v[4 + j], v[8 + j], v[12 + j]);
+    return cr_dot2(r.wx, col[0], col[1], col[2], col[3]);
+  }
+};
 
 // bilinearSample (interpolators.hpp:11-27) for the advection option: clamp
 // to [0, size - 1.1] (glm::clamp = min(max(c, lo), hi)), truncate,
 // interpolate along x, then along y; the four values from the shared-memory
 // window when they lie inside, else from global memory.
-template <int SW, int SH>
+template <int SW, int SH, int SS>
 __device__ __forceinline__ float bilinear_win(const Win &wn, const float *__restrict__ g, int P,
                                               int gw, int gh, float cx, float cy) {
   const float hx = (float)gw - 1.1f, hy = (float)gh - 1.1f;
@@ -525,11 +597,11 @@ __device__ __forceinline__ float bilinear_win(const Win &wn, const float *__rest
   const int lx = ix - wn.sx0, ly = iy - wn.sy0;
   float v1, v2, v3, v4;
   if (lx >= 0 && lx + 1 < SW && ly >= 0 && ly + 1 < SH) {
-    const float *b = wn.s + ly * SW + lx;
+    const float *b = wn.s + ly * SS + lx;
     v1 = b[0];
     v2 = b[1];
-    v3 = b[SW];
-    v4 = b[SW + 1];
+    v3 = b[SS];
+    v4 = b[SS + 1];
   } else {
     const float *b = g + (size_t)iy * P + ix;
     v1 = b[0];
@@ -543,31 +615,66 @@ __device__ __forceinline__ float bilinear_win(const Win &wn, const float *__rest
 }
 
 // advect, simulation.cpp:241-354.  A block handles the vx and vy faces of a
-// 64 x 16 tile of cells; both velocity components are staged in shared
-// memory with a 4-cell halo, which holds every stencil of a back-trace that
-// moves up to about one cell (the CFL-0.5 step moves at most half a cell);
-// longer traces read from global memory.
-constexpr int AD_TX = 64, AD_TY = 16, AD_H = 4;
-constexpr int AD_SW = AD_TX + 2 * AD_H, AD_SH = AD_TY + 2 * AD_H;
+// 64 x TY tile of cells; both velocity components are staged in shared
+// memory with a 4-cell halo.
+//
+// What bounds it: issue (400 warp instructions per 32 cells, of which the
+// interpolation is 200) and the FP32 pipe (two operations in each packed
+// one), not memory: 124 us at 4096x2048, where 151 MB take 22 us.  It was
+// 153 us with each sample by itself.  The steps from there (warp instructions
+// per 32 cells, 2048x1024): two samples at once in packed arithmetic, 511; no
+// window tests where the staging saw that no value moves far, the end's
+// stencil reused from the middle's where it is the same one (mostly: the
+// trace bends little in half a step), 492; no clamps away from the domain's
+// edge, 441; shared memory by address in a register, 399.  Rows of 96 floats
+// instead of 72 took the bank conflicts from 2.0 M to 0.1 M of 8.7 M
+// wavefronts.
+//
+// Tiles of 64 x 4 where 64 x 16 ones would not fill the chip (608 blocks fit
+// at once): 256x128 14 -> 6.4 us, 512x256 14 -> 8.5, 1024x512 20.5 -> 17;
+// from 2048x1024 on the taller tile stages less (42 against 46 us, 4096x2048
+// 124 against 163).  Tiles of 64 x 32 give 47 and 126 us, three blocks per SM
+// instead of four 42 and 130.
+constexpr int AD_TX = 64, AD_TY = 16, AD_LOW = 4, AD_H = 4;
+constexpr unsigned kLowTiles = 608;
+// Cells that the fastest value of a window may travel in a step for every
+// stencil to lie in it: a sample is at most 1.25^2 times the largest value
+// (the sum of the weights' magnitudes), and 1.25^2 * 1.28 = 2 cells plus the
+// stencil's own reach stay inside the halo of 4.  (A step at CFL 0.5 moves at
+// most half a cell.)
+constexpr float kReach = 1.28f;
+constexpr int AD_SW = AD_TX + 2 * AD_H;
+// Row stride in shared memory: with a multiple of 32, a sample's bank is its
+// column, and the lanes of a warp (consecutive faces) read different columns
+// whatever rows they fall in.
+constexpr int AD_SS = 96;
 
 // BIL: the advection option's bilinearSample instead of bicubicSample.
 // EDGES: with the setVBCs that follows in a step, into the buffer written.
-template <bool BIL, bool EDGES>
+template <bool BIL, bool EDGES, int TY>
 __device__ __forceinline__ void k_advect_body(const VelBufs &v, int srcx, int srcy,
                                               const StepScalars *__restrict__ sc, Bcs bc,
                                               const int bx, const int by) {
-  __shared__ __align__(16) float sxv[AD_SH * AD_SW];
-  __shared__ __align__(16) float syv[AD_SH * AD_SW];
-  __shared__ __align__(16) uint8_t scx[AD_TY * AD_TX], scy[AD_TY * AD_TX];
+  constexpr int AD_SH = TY + 2 * AD_H;
+  // both windows, and both components' codes
+  constexpr int kWin = AD_SH * AD_SS, kCodes = TY * AD_TX;
+  __shared__ __align__(16) float sv[2 * kWin];
+  __shared__ __align__(16) uint8_t codes[2 * kCodes];
+  float *const sxv = sv, *const syv = sv + kWin;
+  uint8_t *const scx = codes, *const scy = codes + kCodes;
   const int W = v.W, H = v.H, P = v.pitch;
   const float *vx = pick(v.vx, srcx);
   const float *vy = pick(v.vy, srcy);
-  const int X0 = bx * AD_TX, Y0 = by * AD_TY;
+  const int X0 = bx * AD_TX, Y0 = by * TY;
   const int sx0 = X0 - AD_H, sy0 = Y0 - AD_H;
   const int tid = threadIdx.y * BX + threadIdx.x;
   // staging: 4 entries per load (sx0 and X0 are multiples of 4, so every
   // float4 / uchar4 lies inside its row's pitch); entries outside a
   // component's extent are 0
+  const float chalf = sc->chalf, cfull = sc->cfull;
+  const bool finite = fabsf(cfull) <= 1e30f && fabsf(chalf) <= fabsf(cfull);
+  const float reach = finite ? fminf(kReach / fabsf(cfull), 1e30f) : -1.0f;
+  bool far = (W | H) > 1 << 23;
   static_assert(AD_SW % 4 == 0 && AD_H % 4 == 0 && AD_TX % 4 == 0, "vector staging");
   for (int i = tid; i < AD_SH * (AD_SW / 4); i += 256) {
     const int ry = i / (AD_SW / 4), rx = 4 * (i - ry * (AD_SW / 4));
@@ -587,10 +694,14 @@ __device__ __forceinline__ void k_advect_body(const VelBufs &v, int srcx, int sr
         b.w = 0.f;
       }
     }
-    *reinterpret_cast<float4 *>(sxv + ry * AD_SW + rx) = a;
-    *reinterpret_cast<float4 *>(syv + ry * AD_SW + rx) = b;
+    // (each value by itself: a NaN is far)
+    far |= !(fabsf(a.x) <= reach) | !(fabsf(a.y) <= reach) | !(fabsf(a.z) <= reach) |
+           !(fabsf(a.w) <= reach) | !(fabsf(b.x) <= reach) | !(fabsf(b.y) <= reach) |
+           !(fabsf(b.z) <= reach) | !(fabsf(b.w) <= reach);
+    *reinterpret_cast<float4 *>(sxv + ry * AD_SS + rx) = a;
+    *reinterpret_cast<float4 *>(syv + ry * AD_SS + rx) = b;
   }
-  for (int i = tid; i < AD_TY * (AD_TX / 4); i += 256) {
+  for (int i = tid; i < TY * (AD_TX / 4); i += 256) {
     const int ty = i / (AD_TX / 4), tx = 4 * (i - ty * (AD_TX / 4));
     const int x = X0 + tx, y = Y0 + ty;
     unsigned a = 0u, b = 0u;
@@ -601,71 +712,120 @@ __device__ __forceinline__ void k_advect_body(const VelBufs &v, int srcx, int sr
     *reinterpret_cast<unsigned *>(scx + ty * AD_TX + tx) = a;
     *reinterpret_cast<unsigned *>(scy + ty * AD_TX + tx) = b;
   }
-  __syncthreads();
+  // the values of column 0 that the faces of column W - 2 use
+  if (X0 + AD_TX > W - 2 && X0 <= W - 2 && tid <= TY)
+    far |= !(fabsf(ld(vx, P, 0, min(Y0 + tid, H - 1))) <= reach);
+  far = __syncthreads_or(far);
   const Win wx{sxv, sx0, sy0}, wy{syv, sx0, sy0};
-  const float chalf = sc->chalf, cfull = sc->cfull;
-  auto SX = [&](int x, int y) { return sxv[(y - sy0) * AD_SW + (x - sx0)]; };
-  auto SY = [&](int x, int y) { return syv[(y - sy0) * AD_SW + (x - sx0)]; };
   float *outx = pick(v.vx, 1 - srcx), *outy = pick(v.vy, 1 - srcy);
-  auto SAMPLE = [&](const Win &wn, const float *__restrict__ g, int P_, int gw, int gh, float cx,
-                    float cy) {
+  const bool wide = (W | H) > 1 << 23;
+  const Pair q{sxv,
+               syv,
+               vx,
+               vy,
+               (float)(W - 1) - 3.0f,
+               (float)H - 3.0f,
+               (float)W - 3.0f,
+               (float)(H - 1) - 3.0f,
+               wide ? 0u : 0x4b000000u + (unsigned)(sx0 + 1),
+               wide ? 0u : 0x4b000000u + (unsigned)(sy0 + 1),
+               P};
+  // vx at (cx.x, cy.x), vy at (cx.y, cy.y)
+  auto sample = [&](float2 cx, float2 cy) {
     if constexpr (BIL)
-      return bilinear_win<AD_SW, AD_SH>(wn, g, P_, gw, gh, cx, cy);
+      return make_float2(bilinear_win<AD_SW, AD_SH, AD_SS>(wx, vx, P, W - 1, H, cx.x, cy.x),
+                         bilinear_win<AD_SW, AD_SH, AD_SS>(wy, vy, P, W, H - 1, cx.y, cy.y));
     else
-      return bicubic_win<AD_SW, AD_SH>(wn, g, P_, gw, gh, cx, cy);
+      return bicubic_pair<AD_SW, AD_SH, AD_SS>(q, cx, cy);
   };
-  for (int i = tid; i < AD_TX * AD_TY; i += 256) {
-    int ty = i / AD_TX, tx = i - ty * AD_TX;
-    int x = X0 + tx, y = Y0 + ty;
-    if (y < 1 || y >= H - 1 || x < 1) continue;
-    // vx face (x, y), simulation.cpp:247-298
-    if (x < W - 2) {
-      unsigned k = scx[i];
-      if (k & FC_A) {
-        float posx = (float)x + 0.5f, posy = (float)y;
-        float vx1 = SX(x, y);
-        float vy1 = ((SY(x, y) + SY(x, y - 1)) + (SY(x + 1, y) + SY(x + 1, y - 1))) * 0.25f;
-        float midx = posx - vx1 * chalf;
-        float midy = posy - vy1 * chalf;
-        float vx2 = SAMPLE(wx, vx, P, W - 1, H, midx - 0.5f, midy);
-        float vy2 = SAMPLE(wy, vy, P, W, H - 1, midx, midy - 0.5f);
-        float endx = posx - vx2 * cfull;
-        float endy = posy - vy2 * cfull;
-        float r = SAMPLE(wx, vx, P, W - 1, H, endx - 0.5f, endy);
-        outx[(size_t)y * P + x] = (k & FC_M) ? r : 0.0f;
+  // (after the barrier: what is read through these is read after it)
+  unsigned vbase, cbase;
+  asm volatile("mov.u32 %0, %1;" : "=r"(vbase) : "r"((unsigned)__cvta_generic_to_shared(sv)) : "memory");
+  asm volatile("mov.u32 %0, %1;" : "=r"(cbase) : "r"((unsigned)__cvta_generic_to_shared(codes)) : "memory");
+  const Near<AD_SS, 4 * kWin> near{q.hxx, q.hxy, q.hyx, q.hyy,
+                                   vbase - 4u * (q.oy * AD_SS + q.ox)};
+  // PATH 0: any trace; 1: every stencil in the windows; 2: and no face or
+  // trace of the block near the domain's edge
+  auto faces = [&](auto path) {
+    constexpr int PATH = decltype(path)::value;
+    const int tx = tid % AD_TX, x = X0 + tx;
+    const float fx = (float)x;
+    float fy = (float)(Y0 + tid / AD_TX);
+    int y = Y0 + tid / AD_TX;
+    unsigned at0 = vbase + 4u * ((AD_H + tid / AD_TX) * AD_SS + AD_H + tx), ac = cbase + tid;
+    // vx and vy in this row and the one below, at this column and the next
+    auto px = [&](int dx, int dy) { return lds(at0 + 4u * (dy * AD_SS + dx)); };
+    auto py = [&](int dx, int dy) { return lds(at0 + 4u * (kWin + dy * AD_SS + dx)); };
+#pragma unroll 1
+    for (int n = 0; n < TY * AD_TX / 256; n++, y += 256 / AD_TX, fy += 256 / AD_TX,
+             at0 += 4u * (256 / AD_TX) * AD_SS, ac += 256) {
+      if (PATH < 2 && (y < 1 || y >= H - 1 || x < 1 || x >= W - 1)) continue;
+      const unsigned kx = PATH == 2 || x < W - 2 ? lds8(ac) : 0u, ky = lds8(ac + kCodes);
+      if (!((kx | ky) & FC_A)) continue;
+      const float vxc = px(0, 0), vxs = px(0, -1), vyc = py(0, 0), vys = py(0, -1);
+      // vx face (x, y), simulation.cpp:247-298
+      const float pxx = fx + 0.5f, pxy = fy;
+      const float vy1 = ((vyc + vys) + (py(1, 0) + py(1, -1))) * 0.25f;
+      const float mxx = pxx - vxc * chalf, mxy = pxy - vy1 * chalf;
+      // vy face (x, y), simulation.cpp:300-347 (rows 1..H-2 of the vx loop).
+      // The reference reads vx at flat index x+1+y*(W-1): for x = W-2 that is
+      // element 0 of the next row.
+      const float pyx = fx, pyy = fy + 0.5f;
+      const bool own = PATH == 2 || x + 1 < W - 1;
+      const float a2 = own ? px(1, 0) : ld(vx, P, 0, y + 1);
+      const float a3 = own ? px(1, -1) : ld(vx, P, 0, y);
+      const float vx1 = ((vxc + vxs) + (a2 + a3)) * 0.25f;
+      const float myx = pyx - vx1 * chalf, myy = pyy - vyc * chalf;
+      // u: vx at the vx face's middle, vy at the vy face's; w: vx at the vy
+      // face's middle, vy at the vx face's; r: the ends of both traces
+      const float2 ux = make_float2(mxx - 0.5f, myx), uy = make_float2(mxy, myy - 0.5f);
+      const float2 wx = make_float2(myx - 0.5f, mxx), wy = make_float2(myy, mxy - 0.5f);
+      float2 r;
+      auto end_x = [&](float2 u, float2 w) {
+        return make_float2((pxx - u.x * cfull) - 0.5f, pyx - w.x * cfull);
+      };
+      auto end_y = [&](float2 u, float2 w) {
+        return make_float2(pxy - w.y * cfull, (pyy - u.y * cfull) - 0.5f);
+      };
+      if constexpr (PATH > 0) {
+        float2 s[16];
+        auto at = near.template at<PATH == 1>(wx, wy);
+        near.template load<0>(at.a, s);
+        near.template load<1>(at.b, s);
+        const float2 w = near.value(at, s);
+        at = near.template at<PATH == 1>(ux, uy);
+        const unsigned a = at.a, b = at.b;
+        near.template load<0>(a, s);
+        near.template load<1>(b, s);
+        const float2 u = near.value(at, s);
+        // the ends mostly lie in the stencils just read
+        at = near.template at<PATH == 1>(end_x(u, w), end_y(u, w));
+        if (at.a != a) near.template load<0>(at.a, s);
+        if (at.b != b) near.template load<1>(at.b, s);
+        r = near.value(at, s);
+      } else {
+        const float2 w = sample(wx, wy), u = sample(ux, uy);
+        r = sample(end_x(u, w), end_y(u, w));
       }
+      if (kx & FC_A) outx[(size_t)y * P + x] = (kx & FC_M) ? r.x : 0.0f;
+      // (row H-2 is vy's northern edge: kept only where setVBCs keeps it)
+      if ((ky & FC_A) && (!EDGES || PATH == 2 || y < H - 2 || bc.n == UBG_BC_INFLOW))
+        outy[(size_t)y * P + x] = (ky & FC_M) ? r.y : 0.0f;
     }
-    // vy face (x, y), simulation.cpp:300-347 (rows 1..H-2 of the vx loop)
-    if (x < W - 1) {
-      unsigned k = scy[i];
-      if (k & FC_A) {
-        float posx = (float)x, posy = (float)y + 0.5f;
-        float vy1 = SY(x, y);
-        // The reference reads vx at flat index x+1+y*(W-1): for x = W-2 that
-        // is element 0 of the next row.
-        float a2 = (x + 1 < W - 1) ? SX(x + 1, y) : ld(vx, P, 0, y + 1);
-        float a3 = (x + 1 < W - 1) ? SX(x + 1, y - 1) : ld(vx, P, 0, y);
-        float vx1 = ((SX(x, y) + SX(x, y - 1)) + (a2 + a3)) * 0.25f;
-        float midx = posx - vx1 * chalf;
-        float midy = posy - vy1 * chalf;
-        float vx2 = SAMPLE(wx, vx, P, W - 1, H, midx - 0.5f, midy);
-        float vy2 = SAMPLE(wy, vy, P, W, H - 1, midx, midy - 0.5f);
-        float endx = posx - vx2 * cfull;
-        float endy = posy - vy2 * cfull;
-        float r = SAMPLE(wy, vy, P, W, H - 1, endx, endy - 0.5f);
-        r = (k & FC_M) ? r : 0.0f;
-        // (row H-2 is vy's northern edge: kept only where setVBCs keeps it)
-        if (!EDGES || y < H - 2 || bc.n == UBG_BC_INFLOW) outy[(size_t)y * P + x] = r;
-      }
-    }
-  }
+  };
+  if (BIL || far)
+    faces(std::integral_constant<int, 0>{});
+  else if (X0 > 4 && Y0 >= 8 && X0 + AD_TX + 8 <= W && Y0 + TY + 8 <= H)
+    faces(std::integral_constant<int, 2>{});
+  else
+    faces(std::integral_constant<int, 1>{});
   griddep_launch();
   if (!EDGES) return;
   // setVBCs: the edge cells next to the tile's faces, once those are written
-  if (X0 > 1 && X0 + AD_TX <= W - 3 && Y0 > 1 && Y0 + AD_TY <= H - 3) return;
+  if (X0 > 1 && X0 + AD_TX <= W - 3 && Y0 > 1 && Y0 + TY <= H - 3) return;
   __syncthreads();
 #pragma unroll 1
-  for (int i = tid; i < AD_TX * AD_TY; i += 256) {
+  for (int i = tid; i < AD_TX * TY; i += 256) {
     const int ty = i / AD_TX, x = X0 + i - ty * AD_TX, y = Y0 + ty;
     if (y < 1 || y >= H - 1 || x < 1 || x > W - 2) continue;
     if (x <= W - 3 && (x == 1 || x == W - 3 || y == 1 || y == H - 2))
@@ -693,13 +853,13 @@ __device__ __forceinline__ void k_advect_body(const VelBufs &v, int srcx, int sr
 }
 // umax_zero: max|u|, zeroed for the step's gradient kernel to accumulate (the
 // step's dt has been formed from it).
-template <bool BIL, bool EDGES>
-__global__ void __launch_bounds__(256) k_advect(VelBufs v, int srcx, int srcy,
+template <bool BIL, bool EDGES, int TY>
+__global__ void __launch_bounds__(256, 4) k_advect(VelBufs v, int srcx, int srcy,
                                                 const StepScalars *__restrict__ sc, Bcs bc,
                                                 unsigned int *umax_zero) {
   griddep_wait();
   if (EDGES && (blockIdx.x | blockIdx.y | threadIdx.x | threadIdx.y) == 0) *umax_zero = 0u;
-  k_advect_body<BIL, EDGES>(v, srcx, srcy, sc, bc, blockIdx.x, blockIdx.y);
+  k_advect_body<BIL, EDGES, TY>(v, srcx, srcy, sc, bc, blockIdx.x, blockIdx.y);
 }
 
 // ------------------------------------------------------------- divergence
@@ -979,7 +1139,7 @@ __global__ void __launch_bounds__(256) k_diffuse_m(const DiffuseM *__restrict__ 
   else
     k_diffuse_body<2>(a.v, a.srcx, a.srcy, a.sc, 3, a.bc, l % a.gx, l / a.gx);
 }
-__global__ void __launch_bounds__(256, 6) k_advect_m(const AdvectM *__restrict__ A, const int *__restrict__ bs, int n,
+__global__ void __launch_bounds__(256, 4) k_advect_m(const AdvectM *__restrict__ A, const int *__restrict__ bs, int n,
            unsigned tag, unsigned *err) {
   griddep_wait();
   if (!table_ok(bs, n, tag, err)) return;
@@ -988,7 +1148,7 @@ __global__ void __launch_bounds__(256, 6) k_advect_m(const AdvectM *__restrict__
   const int l = (int)blockIdx.x - __ldg(bs + m);
   if (l == 0 && (threadIdx.x | threadIdx.y) == 0) *a.umax_zero = 0u;
   // fused members advect bicubically (the bilinear option is not fused)
-  k_advect_body<false, true>(a.v, a.srcx, a.srcy, a.sc, a.bc, l % a.gx, l / a.gx);
+  k_advect_body<false, true, AD_TY>(a.v, a.srcx, a.srcy, a.sc, a.bc, l % a.gx, l / a.gx);
 }
 __global__ void __launch_bounds__(256) k_divergence_m(const DivergenceM *__restrict__ A, const int *__restrict__ bs, int n,
                unsigned tag, unsigned *err) {
@@ -1054,8 +1214,16 @@ void launch_advect(const VelBufs &v, int srcx, int srcy, const StepScalars *sc, 
                    bool edges, Bcs bc, unsigned int *umax_zero) {
   ProfScope ps_(KC_ADVECT, st);
   dim3 grid((v.W + AD_TX - 1) / AD_TX, (v.H + AD_TY - 1) / AD_TY);
-  auto *k = v.advect_bilinear ? (edges ? k_advect<true, true> : k_advect<true, false>)
-                              : (edges ? k_advect<false, true> : k_advect<false, false>);
+  auto pick_ty = [&](auto ty) {
+    constexpr int T = decltype(ty)::value;
+    return v.advect_bilinear ? (edges ? k_advect<true, true, T> : k_advect<true, false, T>)
+                             : (edges ? k_advect<false, true, T> : k_advect<false, false, T>);
+  };
+  auto *k = pick_ty(std::integral_constant<int, AD_TY>{});
+  if (grid.x * grid.y < kLowTiles) {
+    k = pick_ty(std::integral_constant<int, AD_LOW>{});
+    grid.y = (v.H + AD_LOW - 1) / AD_LOW;
+  }
   launch_pdl(k, grid, dim3(BX, BY), 0, st, v, srcx, srcy, sc, bc, umax_zero);
   UBG_LAUNCH_CHECK();
   g_stats.launches++;
