@@ -13,7 +13,10 @@
 // inner neighbour, whose own value then stands for them.
 //
 // What bounds it: latency, a few hundred dependent instructions per visit.
-// 64x32 and down: 13.6 us (ncu).  With 4 columns x 2 rows per lane but always
+// 64x32 and down: 10.4 us (ncu).  It was 13.6 with the codes read level by
+// level (a memory latency each) and the tolerance hierarchy's edges behind a
+// uniform branch in every half sweep (132 against 80 cycles per half sweep of
+// one warp).  Before, with 4 columns x 2 rows per lane but always
 // 32 lanes per row, all 32 warps and a block barrier per half sweep, 128x64 and
 // down took 32 us: small levels waited for barriers of idle warps.  128x64 in
 // the block instead of two smoothing launches (5 us each in a step): 43
@@ -26,6 +29,7 @@ namespace coarse {
 
 constexpr int kMaxLevels = 12;
 constexpr int kWarps = 16;
+constexpr int kItems = 4, kMaxGroups = kItems * 32 * kWarps;  // groups of four cells, all levels
 
 struct Level {
   int w, h, lsh, warps;   // lanes per row 1 << lsh; warps that hold its rows
@@ -87,7 +91,7 @@ __device__ __forceinline__ void sync_level(int warps) {
 
 // One half sweep (red or black).  MULTI: the level takes several warps.
 // grad: the edge cells have their inner neighbour's value.
-template <bool MULTI, bool CAREFUL, int RED>
+template <bool MULTI, bool CAREFUL, bool EXT, int RED>
 __device__ __forceinline__ void half(Regs &q, const Place &pl, float2 *xch, const int w,
                                      const int h, const bool grad) {
   auto slot = [&](int buf, int wd, int lastrow) -> float2 & {
@@ -113,7 +117,7 @@ __device__ __forceinline__ void half(Regs &q, const Place &pl, float2 *xch, cons
       E = q.B[r];
     }
     float2 S = r ? (onB ? q.B[0] : q.A[0]) : below, N = r ? above : (onB ? q.B[1] : q.A[1]);
-    if (grad) {
+    if (EXT && grad) {
       const unsigned c0 = q.cw[r] >> (onB ? 8 : 0), c1 = c0 >> 16;
       if (onB && pl.X == 0) W.x = (c0 & C_W) ? own.x : 0.0f;
       if (xe == (onB ? 1 : 0)) E.x = (c0 & C_E) ? own.x : 0.0f;
@@ -135,20 +139,20 @@ __device__ __forceinline__ void half(Regs &q, const Place &pl, float2 *xch, cons
     sync_level(pl.warps);
   }
 }
-template <bool MULTI, bool CAREFUL>
+template <bool MULTI, bool CAREFUL, bool EXT>
 __device__ __forceinline__ void sweeps(Regs &q, const Place &pl, float2 *xch, const int w,
-                                       const int h, const int n, const bool ext, const bool up) {
+                                       const int h, const int n, const bool up) {
 #pragma unroll 1
   for (int s = 0; s < n; s++) {
-    half<MULTI, CAREFUL, 1>(q, pl, xch, w, h, ext && (up || s > 0));
-    half<MULTI, CAREFUL, 0>(q, pl, xch, w, h, ext && (up || s > 0));
+    half<MULTI, CAREFUL, EXT, 1>(q, pl, xch, w, h, up || s > 0);
+    half<MULTI, CAREFUL, EXT, 0>(q, pl, xch, w, h, up || s > 0);
   }
 }
 
 // One visit of level t by its warps: down (e = 0; sweeps, and unless it is the
 // coarsest level residual and restriction to level t+1) or up (prolongation
 // and correction from level t+1, sweeps).
-template <class S>
+template <class S, bool EXT>
 __device__ __forceinline__ void visit(const Args<S> &a, const int t, const bool up,
                                       unsigned char *smem) {
   using St = Sto<S>;
@@ -164,7 +168,7 @@ __device__ __forceinline__ void visit(const Args<S> &a, const int t, const bool 
   pl.X = 4 * pl.l;
   pl.y = 2 * (pl.wid * pl.groups + pl.sub);
   const int w = L.w, h = L.h, X = pl.X, y = pl.y, n = 1 << pl.lsh, stride = 4 * n;
-  const bool ext = a.ext != 0, last = t == a.nlev - 1;
+  const bool last = t == a.nlev - 1;
   float *const e = reinterpret_cast<float *>(smem + L.oe) + y * stride + X;
   const float *const f = reinterpret_cast<const float *>(smem + L.of) + y * stride + X;
   const uint8_t *const code = smem + L.oc + y * stride + X;
@@ -201,7 +205,7 @@ __device__ __forceinline__ void visit(const Args<S> &a, const int t, const bool 
     g0 |= (__shfl_down_sync(0xffffffffu, g0, 1) & 1u) << 16;
     g1 |= (__shfl_down_sync(0xffffffffu, g1, 1) & 1u) << 16;
     tile::prolongate2(e3, f3, g0, g1, lut, u);
-    if (!ext) {  // no coarse cell beyond
+    if (!EXT) {  // no coarse cell beyond
 #pragma unroll
       for (int b = 0; b < 4; b++) {
         if ((b & 1) && X + b >= w - 2) u[0][b] = u[1][b] = 0.0f;
@@ -259,16 +263,16 @@ __device__ __forceinline__ void visit(const Args<S> &a, const int t, const bool 
                  : "memory");
     careful = any != 0;
   }
-  const int ns = last ? (ext ? a.ncoarse : 5) : 3;
+  const int ns = last ? (EXT ? a.ncoarse : 5) : 3;
   if (careful) {
     if (multi)
-      sweeps<true, true>(q, pl, xch, w, h, ns, ext, up);
+      sweeps<true, true, EXT>(q, pl, xch, w, h, ns, up);
     else
-      sweeps<false, true>(q, pl, xch, w, h, ns, ext, up);
+      sweeps<false, true, EXT>(q, pl, xch, w, h, ns, up);
   } else if (multi) {
-    sweeps<true, false>(q, pl, xch, w, h, ns, ext, up);
+    sweeps<true, false, EXT>(q, pl, xch, w, h, ns, up);
   } else {
-    sweeps<false, false>(q, pl, xch, w, h, ns, ext, up);
+    sweeps<false, false, EXT>(q, pl, xch, w, h, ns, up);
   }
 
   // ---- e to shared memory, or the result to the top level's array.  Edge
@@ -278,7 +282,7 @@ __device__ __forceinline__ void visit(const Args<S> &a, const int t, const bool 
   for (int r = 0; r < 2; r++) {
     const int yy = y + r;
     float o[4] = {q.A[r].x, q.B[r].x, q.A[r].y, q.B[r].y};
-    if (ext) {
+    if (EXT) {
       const float left = __shfl_up_sync(0xffffffffu, q.B[r].y, 1);
       const float inner[4] = {left, o[0], o[1], o[2]};
       if (X == 0) o[0] = o[1];
@@ -301,9 +305,9 @@ __device__ __forceinline__ void visit(const Args<S> &a, const int t, const bool 
         *reinterpret_cast<float4 *>(e + (ye - y) * stride) = make_float4(o[0], o[1], o[2], o[3]);
       }
     };
-    if (!ext || (yy >= 1 && yy < h - 1)) put(yy);
-    if (ext && yy == 1) put(0);
-    if (ext && yy == h - 2) put(h - 1);
+    if (!EXT || (yy >= 1 && yy < h - 1)) put(yy);
+    if (EXT && yy == 1) put(0);
+    if (EXT && yy == h - 2) put(h - 1);
   }
   if (up || last) return;
 
@@ -332,7 +336,7 @@ __device__ __forceinline__ void visit(const Args<S> &a, const int t, const bool 
     const float F4[4] = {fv.x, fv.y, fv.z, fv.w};
     float W4[4] = {l, q.A[r].x, q.B[r].x, q.A[r].y}, E4[4] = {q.B[r].x, q.A[r].y, q.B[r].y, rr};
     float S4[4] = {SA.x, SB.x, SA.y, SB.y}, N4[4] = {NA.x, NB.x, NA.y, NB.y};
-    if (ext) {  // the edge cells have this cell's value
+    if (EXT) {  // the edge cells have this cell's value
 #pragma unroll
       for (int b = 0; b < 4; b++) {
         if (X + b == 1) W4[b] = C4[b];
@@ -369,9 +373,10 @@ __device__ __forceinline__ void visit(const Args<S> &a, const int t, const bool 
         make_float2(v0, v1);
 }
 
+// What needs no other kernel's results: arguments and zero rows to shared
+// memory.
 template <class S>
-__device__ __forceinline__ void run(const Args<S> &args, unsigned char *smem) {
-  using St = Sto<S>;
+__device__ __forceinline__ void init(const Args<S> &args, unsigned char *smem) {
   static_assert(sizeof(Args<S>) <= kArgsBytes && sizeof(Args<S>) % 4 == 0, "arguments");
   if (threadIdx.x < sizeof(Args<S>) / 4)
     reinterpret_cast<unsigned *>(smem + kArgs)[threadIdx.x] =
@@ -381,25 +386,55 @@ __device__ __forceinline__ void run(const Args<S> &args, unsigned char *smem) {
   if (threadIdx.x < 128) xch[(threadIdx.x >> 6) * (kWarps + 2) * 64 + (threadIdx.x & 63)] = make_float2(0.f, 0.f);
   if (threadIdx.x < 32) reinterpret_cast<float2 *>(smem + kRes)[threadIdx.x] = make_float2(0.f, 0.f);
   __syncthreads();
+}
+
+template <class S, bool EXT>
+__device__ __forceinline__ void run(unsigned char *smem) {
+  using St = Sto<S>;
   const Args<S> &a = *reinterpret_cast<const Args<S> *>(smem + kArgs);
-  // codes of every level, the top level's right-hand side (columns past the
-  // width: 0)
+  // Codes of every level, the top level's right-hand side (columns past the
+  // width: 0).  The levels' groups of four cells are numbered through, at
+  // most kItems per thread (128 x 32 cells, or 16 x 256, and the levels below:
+  // fewer than 2048 groups), and all their loads are in flight together.
+  const uint8_t *src[kItems];
+  unsigned mask[kItems], dst[kItems], c[kItems];
+  int left[kItems];
+#pragma unroll
+  for (int k = 0; k < kItems; k++) {
+    left[k] = threadIdx.x + 32 * kWarps * k;
+    src[k] = nullptr;
+    mask[k] = dst[k] = c[k] = 0u;
+  }
+  const Level &T = a.L[0];
+  const int nt = T.h << T.lsh, n1 = (1 << T.lsh) - 1;
+#pragma unroll 1
   for (int t = 0; t < a.nlev; t++) {
     const Level &L = a.L[t];
-    const int stride = 4 << L.lsh;
-    for (int i = threadIdx.x; i < L.h << L.lsh; i += 32 * kWarps) {
-      const int y = i >> L.lsh, X = 4 * (i & ((1 << L.lsh) - 1));
-      unsigned m = 0u, c = 0u;
-      float4 fv = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int n = L.h << L.lsh;
 #pragma unroll
-      for (int b = 0; b < 4; b++) m |= X + b < L.w ? 0xffu << (8 * b) : 0u;
-      if (X < L.w) {
-        c = __ldg(reinterpret_cast<const unsigned *>(L.code + (size_t)y * L.code_pitch + X)) & m;
-        if (t == 0) fv = St::ldg4(a.rhs_top + (size_t)y * a.rhs_pitch + X);
-      }
-      *reinterpret_cast<unsigned *>(smem + L.oc + y * stride + X) = c;
-      if (t == 0) *reinterpret_cast<float4 *>(smem + L.of + (y * stride + X) * 4) = fv;
+    for (int k = 0; k < kItems; k++) {
+      const int i = left[k], X = 4 * (i & ((1 << L.lsh) - 1));
+      left[k] -= n;
+      if (i < 0 || i >= n) continue;
+      dst[k] = L.oc + 4 * i;
+      if (X >= L.w) continue;
+      src[k] = L.code + (size_t)(i >> L.lsh) * L.code_pitch + X;
+      mask[k] = 0xffffffffu >> (8 * max(0, X + 4 - L.w));
     }
+  }
+  float4 fv[kItems];
+#pragma unroll
+  for (int k = 0; k < kItems; k++) {
+    if (src[k]) c[k] = __ldg(reinterpret_cast<const unsigned *>(src[k])) & mask[k];
+    const int i = threadIdx.x + 32 * kWarps * k, X = 4 * (i & n1);
+    fv[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (i < nt && X < T.w) fv[k] = St::ldg4(a.rhs_top + (size_t)(i >> T.lsh) * a.rhs_pitch + X);
+  }
+#pragma unroll
+  for (int k = 0; k < kItems; k++) {
+    if (dst[k]) *reinterpret_cast<unsigned *>(smem + dst[k]) = c[k];
+    const int i = threadIdx.x + 32 * kWarps * k;
+    if (i < nt) *reinterpret_cast<float4 *>(smem + T.of + 16 * i) = fv[k];
   }
   __syncthreads();
   const int wid = threadIdx.x >> 5;
@@ -408,7 +443,7 @@ __device__ __forceinline__ void run(const Args<S> &args, unsigned char *smem) {
     const bool up = v >= a.nlev;
     const int t = up ? 2 * a.nlev - 2 - v : v;
     if (v == 2 * a.nlev - 2) griddep_launch();
-    if (wid < a.L[t].warps) visit<S>(a, t, up, smem);
+    if (wid < a.L[t].warps) visit<S, EXT>(a, t, up, smem);
     // the next level's warps read what these wrote
     __syncthreads();
   }

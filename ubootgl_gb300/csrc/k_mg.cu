@@ -308,13 +308,14 @@ __global__ void __launch_bounds__(32 * NW, 1024 / (32 * NW))
   tile::run<float, float, false, PRE, R, NW>(a, (int)blockIdx.x - __ldg(bs + m), smem_raw);
 }
 
-template <class S>
+template <class S, bool EXT>
 __global__ void __launch_bounds__(32 * coarse::kWarps, 1)
     k_coarse(const __grid_constant__ coarse::Args<S> a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   tile::fill_lut(reinterpret_cast<float2 *>(smem_raw + coarse::kLut), threadIdx.x, a.wsum, a.rwsum);
+  coarse::init<S>(a, smem_raw);
   griddep_wait();
-  coarse::run<S>(a, smem_raw);
+  coarse::run<S, EXT>(smem_raw);
 }
 // One block per member of a batch (FP32).
 __global__ void __launch_bounds__(32 * coarse::kWarps, 1)
@@ -325,7 +326,8 @@ __global__ void __launch_bounds__(32 * coarse::kWarps, 1)
   if (!table_ok(bs, n, tag, err)) return;
   const coarse::Args<float> &a = A[blockIdx.x];
   tile::fill_lut(reinterpret_cast<float2 *>(smem_raw + coarse::kLut), threadIdx.x, a.wsum, a.rwsum);
-  coarse::run<float>(a, smem_raw);
+  coarse::init<float>(a, smem_raw);
+  coarse::run<float, false>(smem_raw);
 }
 
 template <int TX, int TY, int HALO>
@@ -991,9 +993,12 @@ static void set_all_kernel_attributes() {
   set_smem_attr(k_mg<40, 8, 12, true, 256, __half>, Tile<40, 8, 12>::smem(2));
   set_smem_attr(k_mg<40, 8, 12, true, 256, __nv_bfloat16>, Tile<40, 8, 12>::smem(2));
   set_smem_attr(k_mg<56, 24, 4, false, 256, float>, Tile<56, 24, 4>::smem(4));
-  set_smem_attr(k_coarse<float>, kCoarseSmemMax);
-  set_smem_attr(k_coarse<__half>, kCoarseSmemMax);
-  set_smem_attr(k_coarse<__nv_bfloat16>, kCoarseSmemMax);
+  set_smem_attr(k_coarse<float, true>, kCoarseSmemMax);
+  set_smem_attr(k_coarse<float, false>, kCoarseSmemMax);
+  set_smem_attr(k_coarse<__half, true>, kCoarseSmemMax);
+  set_smem_attr(k_coarse<__half, false>, kCoarseSmemMax);
+  set_smem_attr(k_coarse<__nv_bfloat16, true>, kCoarseSmemMax);
+  set_smem_attr(k_coarse<__nv_bfloat16, false>, kCoarseSmemMax);
   set_smem_attr(k_coarse_m, kCoarseSmemMax);
   set_smem_attr(k_mg_tail<float, float>, TAIL_SMEM_MAX);
   set_smem_attr(k_mg_tail<__half, float>, TAIL_SMEM_MAX);
@@ -1170,7 +1175,7 @@ coarse::Args<S> coarse_args(MgHier &mg, int lt, const S *rhs_top, S *e_top, cons
   a.nlev = nl;
   a.ext = mg.ext ? 1 : 0;
   a.ncoarse = mg.ncoarse;
-  size_t off = coarse::kLevels;
+  size_t off = coarse::kLevels, groups = 0;
   for (int t = 0; t < nl; t++) {
     MgLevel &L = mg.lv[lt + t];
     coarse::Level &C = a.L[t];
@@ -1182,6 +1187,7 @@ coarse::Args<S> coarse_args(MgHier &mg, int lt, const S *rhs_top, S *e_top, cons
     C.ihsq = rfac ? 1.0f : 1.0f / L.hh / L.hh;
     C.rfac = rfac ? rfac[lt + t] : 1.0f / 16.0f;
     const size_t n = (size_t)C.h << C.lsh;
+    groups += n;
     C.oe = (int)off;
     C.of = (int)(off + 16 * n);
     C.oc = (int)(off + 32 * n);
@@ -1189,7 +1195,8 @@ coarse::Args<S> coarse_args(MgHier &mg, int lt, const S *rhs_top, S *e_top, cons
     C.code = L.code;
     C.code_pitch = L.pitch;
   }
-  if (off > kCoarseSmemMax) throw ArgError("coarse levels exceed the shared memory of a block");
+  if (off > kCoarseSmemMax || groups > coarse::kMaxGroups)
+    throw ArgError("coarse levels exceed one block");
   MgLevel &top = mg.lv[lt];
   a.rhs_top = rhs_top;
   a.rhs_pitch = top.pitch;
@@ -1213,7 +1220,8 @@ void run_coarse(MgHier &mg, int lt, const S *rhs_top, S *e_top, const float *rfa
   ProfScope ps_(KC_TAIL, st);
   size_t smem = 0;
   const coarse::Args<S> a = coarse_args<S>(mg, lt, rhs_top, e_top, rfac, &smem);
-  launch_pdl(k_coarse<S>, dim3(1), dim3(32 * coarse::kWarps), smem, st, a);
+  launch_pdl(a.ext ? k_coarse<S, true> : k_coarse<S, false>, dim3(1), dim3(32 * coarse::kWarps),
+             smem, st, a);
   UBG_LAUNCH_CHECK();
   g_stats.launches++;
 }
