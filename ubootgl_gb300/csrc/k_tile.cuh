@@ -111,14 +111,15 @@ __device__ __forceinline__ float scaled_any(float v, float s) {
 // half sweeps stay finite.
 constexpr float kBigSq = 0x1p+120f;
 
-// Fills the table: factors by code, 32 + code for a cell that is not
-// smoothed; then the weight sums of the prolongation and their reciprocals.
+// Fills the table: factors by code, 32 + flag for a cell on the domain's
+// edge; then the weight sums of the prolongation and their reciprocals.
 __device__ __forceinline__ void fill_lut(float2 *lut, int i, const float *wsum,
                                          const float *rwsum) {
   if (i < 64) {
     const int n = __popc((i >> 1) & 15);
     float s = n == 4 ? 0.25f : (n == 3 ? kThird : (n == 2 ? 0.5f : (n == 1 ? 1.0f : 0.0f)));
-    if (!(i & (int)C_CENTER) || i >= 32) s = 0.0f;
+    if (!(i & (int)C_CENTER)) s = 0.0f;
+    if (i >= 32) s = i & (int)C_CENTER ? -1.0f : -0.0f;
     reinterpret_cast<float *>(lut)[i] = s;
   } else if (i < 69) {
     lut[i - 32] = make_float2(wsum[i - 64], rwsum[i - 64]);
@@ -273,23 +274,12 @@ __device__ __forceinline__ void run(const MgArgsT<S, SC> &a, const int region,
     }
   }
   copy_commit();
-  unsigned all = cw[0];
-#pragma unroll
-  for (int r = 1; r < R; r++) all &= cw[r];
-  // the warp's rows or columns touch the domain's edge (rows 1 and h-2 too:
-  // their neighbours on the edge follow them); where the edge cells are 0 and
-  // stay so, the factor 0 does it
-  const bool rim = first || has_east || y <= 1 || y + R >= h - 1;
-  const bool wedge = rim && !a.zero_edges;
-  const bool full = __all_sync(0xffffffffu, all == kFull) && !rim;
-
+  // the coarse level's values and flags under these rows
+  constexpr int RC = PRE ? 1 : R / 2 + 1;
+  float2 ev[RC];
+  unsigned fl[RC];
   if constexpr (!PRE) {
-    // ---- prolongate (pressure_solver.cpp:134-172) + correct: an even row
-    // lies over one coarse row, an odd row between two
-    constexpr int RC = R / 2 + 1;
     const int c0 = X >> 1, cy = y >> 1;
-    float2 ev[RC];
-    unsigned fl[RC];
 #pragma unroll
     for (int k = 0; k < RC; k++) {
       const size_t o = (size_t)(cy + k) * a.cpitch + c0;
@@ -304,6 +294,22 @@ __device__ __forceinline__ void run(const MgArgsT<S, SC> &a, const int region,
         }
       }
     }
+  }
+  unsigned all = cw[0];
+#pragma unroll
+  for (int r = 1; r < R; r++) all &= cw[r];
+  // the warp's rows or columns touch the domain's edge (rows 1 and h-2 too:
+  // their neighbours on the edge follow them); where the edge cells are 0 and
+  // stay so, the factor 0 does it
+  const bool rim = first || has_east || y <= 1 || y + R >= h - 1;
+  const bool wedge = rim && !a.zero_edges;
+  const bool west = first && lane == 0;  // column 0 is the lane's first
+  const int pe = w - 1 - X;              // place of column w-1 in the lane
+  const bool full = __all_sync(0xffffffffu, all == kFull) && !rim;
+
+  if constexpr (!PRE) {
+    // ---- prolongate (pressure_solver.cpp:134-172) + correct: an even row
+    // lies over one coarse row, an odd row between two
     float ecmul = 1.0f;
     if (EXT && a.scale_bits) coarse_scale(a.scale_bits, a.scale_h1sq, a.scale_kexp, &ecmul);
     float e[3] = {ev[0].x, ev[0].y, __shfl_down_sync(0xffffffffu, ev[0].x, 1)};
@@ -358,8 +364,9 @@ __device__ __forceinline__ void run(const MgArgsT<S, SC> &a, const int region,
     if (!full) {
       const bool brow = y + r == 0 || y + r == h - 1;
       const unsigned in = brow ? 0u : inmask;
-      // codes, 32 + flag where the cell keeps its value
-      const unsigned c = (cw[r] & in & 0x1f1f1f1fu) | (~in & ((cw[r] & 0x01010101u) | 0x20202020u));
+      // codes; 32 + flag on the domain's edge (32 where it is and stays 0)
+      const unsigned c = (cw[r] & in & 0x1f1f1f1fu) |
+                         (~in & (a.zero_edges ? 0x20202020u : (cw[r] & 0x01010101u) | 0x20202020u));
 #pragma unroll
       for (int b = 0; b < 4; b++)
         if (!((c >> (8 * b)) & C_CENTER)) p[b] = F[b] = 0.0f;
@@ -375,7 +382,33 @@ __device__ __forceinline__ void run(const MgArgsT<S, SC> &a, const int region,
     FB[r] = make_float2(F[1], F[3]);
     sq = f2_fma(FB[r], FB[r], f2_fma(FA[r], FA[r], f2_fma(B[r], B[r], f2_fma(A[r], A[r], sq))));
   }
-  slot(0, wid, 0) = A[0];
+  if (!PRE && wedge && zg) {  // edge cells: their inner neighbours' values
+    auto flag = [&](unsigned c, int b, float v) { return (c >> (8 * b)) & C_CENTER ? v : 0.0f; };
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+      const float left = __shfl_up_sync(0xffffffffu, B[r].y, 1);
+      const unsigned c = cw[r];
+      if (west) A[r].x = flag(c, 0, B[r].x);
+      if (pe == 0) A[r].x = flag(c, 0, left);
+      if (pe == 1) B[r].x = flag(c, 1, A[r].x);
+      if (pe == 2) A[r].y = flag(c, 2, B[r].x);
+      if (pe == 3) B[r].y = flag(c, 3, A[r].y);
+    }
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+      const unsigned c = cw[r];
+      if ((r == 0 && y == 0) || (r > 0 && y + r == h - 1)) {
+        const int i = r == 0 ? 1 : r - 1;
+        A[r] = make_float2(flag(c, 0, A[i].x), flag(c, 2, A[i].y));
+        B[r] = make_float2(flag(c, 1, B[i].x), flag(c, 3, B[i].y));
+      }
+    }
+  }
+  // (row h-1 as a warp's first row is written by the warp below it)
+  if (!(!PRE && wedge && zg && wid > 0 && y == h - 1)) slot(0, wid, 0) = A[0];
+  if (!PRE && wedge && zg && wid < NW - 1 && y + R == h - 1)
+    slot(0, wid + 1, 0) = make_float2((cw[R - 1] & C_N) ? A[R - 1].x : 0.0f,
+                                      ((cw[R - 1] >> 16) & C_N) ? A[R - 1].y : 0.0f);
   slot(0, wid, 1) = B[R - 1];
   if (wid == 0)
     slot(0, -1, 1) = slot(1, -1, 1) = slot(0, NW, 0) = slot(1, NW, 0) = res[0] =
@@ -388,12 +421,14 @@ __device__ __forceinline__ void run(const MgArgsT<S, SC> &a, const int region,
   // ---- three sweeps.  Red updates the pair (1, 3) of even rows and (0, 2)
   // of odd rows, black the others; what a warp reads of its neighbours' rows
   // was updated in the half sweep before.
-  // At the domain's edge a cell's neighbour on the edge holds the cell's own
-  // value of the sweep before (zero gradient; 0 if the edge cell is solid).
-  const int xe = w - 2 - X;  // place of column w-2 in the lane
+  // A cell on the domain's edge (factor -1, -0 if solid) takes its inner
+  // neighbour's value when its colour is updated (follow), which is then that
+  // neighbour's value of the sweep before until the neighbour itself is
+  // updated, as the reference's zero-gradient copy between sweeps gives it; or
+  // it keeps its own.
   // MODE 0: an all-fluid warp, 1: any flags, 2: and the domain's edge, 3: and
   // sums that may not be finite.
-  auto half = [&](auto modec, auto redc, const bool grad) {
+  auto half = [&](auto modec, auto redc, const bool follow) {
     constexpr int MODE = decltype(modec)::value;
     constexpr int RED = decltype(redc)::value;
     constexpr bool EDGE = MODE >= 2;
@@ -411,36 +446,30 @@ __device__ __forceinline__ void run(const MgArgsT<S, SC> &a, const int region,
         W = make_float2(__shfl_up_sync(0xffffffffu, B[r].y, 1), B[r].x);
         E = B[r];
       }
-      float2 Sv = r > 0 ? (onB ? B[r > 0 ? r - 1 : 0] : A[r > 0 ? r - 1 : 0]) : below;
-      float2 Nv = r < R - 1 ? (onB ? B[r < R - 1 ? r + 1 : 0] : A[r < R - 1 ? r + 1 : 0]) : above;
-      if (EDGE && grad) {
-        const unsigned c0 = cw[r] >> (onB ? 8 : 0), c1 = c0 >> 16;
-        if (onB && first && lane == 0) W.x = (c0 & C_W) ? own.x : 0.0f;
-        if (xe == (onB ? 1 : 0)) E.x = (c0 & C_E) ? own.x : 0.0f;
-        if (xe == (onB ? 3 : 2)) E.y = (c1 & C_E) ? own.y : 0.0f;
-        if (y + r == 1) Sv = make_float2((c0 & C_S) ? own.x : 0.0f, (c1 & C_S) ? own.y : 0.0f);
-        if (y + r == h - 2) Nv = make_float2((c0 & C_N) ? own.x : 0.0f, (c1 & C_N) ? own.y : 0.0f);
-      }
+      const float2 Sv = r > 0 ? (onB ? B[r > 0 ? r - 1 : 0] : A[r > 0 ? r - 1 : 0]) : below;
+      const float2 Nv = r < R - 1 ? (onB ? B[r < R - 1 ? r + 1 : 0] : A[r < R - 1 ? r + 1 : 0]) : above;
       // (W + E needs no pair of its own: scalar additions, without moves)
       const float2 we = make_float2(W.x + E.x, W.y + E.y);
-      const float2 v = add2(add2(add2(we, Sv), Nv), onB ? FB[r] : FA[r]);
+      float2 v = add2(add2(add2(we, Sv), Nv), onB ? FB[r] : FA[r]);
       float2 n;
       if (MODE == 0) {
         n = make_float2(v.x * 0.25f, v.y * 0.25f);
       } else {
         const float2 s = fac(r, onB ? 1 : 0);
+        if (EDGE) {
+          float2 t = make_float2(!onB && west ? E.x : W.x, W.y);
+          if (r == 0 && y == 0) t = Nv;
+          if (y + r == h - 1) t = Sv;
+          if (!follow) t = own;
+          if (__float_as_int(s.x) < 0) v.x = -t.x;
+          if (__float_as_int(s.y) < 0) v.y = -t.y;
+        }
         if (MODE == 3)
           n = make_float2(scaled_any(v.x, s.x), scaled_any(v.y, s.y));
         else
           n = scaled2(v, s);
       }
       n = rnd2<S>(n);
-      if (EDGE) {  // cells on the domain's edge keep their values
-        if (y + r == 0 || y + r == h - 1) n = own;
-        if (!onB && first && lane == 0) n.x = own.x;
-        if (xe + 1 == (onB ? 1 : 0)) n.x = own.x;
-        if (xe + 1 == (onB ? 3 : 2)) n.y = own.y;
-      }
       own = n;
     }
     slot(buf ^ 1, wid, 0) = RED ? B[0] : A[0];
@@ -453,14 +482,14 @@ __device__ __forceinline__ void run(const MgArgsT<S, SC> &a, const int region,
 #pragma unroll 1
     for (int s = 0; s < 3; s++) {
       half(modec, red, zg && (!PRE || s > 0));
-      half(modec, black, zg && (!PRE || s > 0));
+      half(modec, black, zg);
     }
   };
   if (full)
     sweeps(std::integral_constant<int, 0>{});
   else if (careful)
     sweeps(std::integral_constant<int, 3>{});
-  else if (wedge)
+  else if (wedge && (first || has_east || y == 0 || y + R >= h))
     sweeps(std::integral_constant<int, 2>{});
   else
     sweeps(std::integral_constant<int, 1>{});
@@ -487,49 +516,54 @@ __device__ __forceinline__ void run(const MgArgsT<S, SC> &a, const int region,
         }
       }
   } else {
-    auto old = [&](int xx, int yy) {
-      return a.zero_init ? 0.0f : St::ldg1(a.in + (size_t)yy * P + xx);
-    };
-    auto store = [&](int yy, const float (&o)[4]) {
+    // columns 0 and w-1, rows 0 and h-1 (stored with rows 1 and h-2): the
+    // inner neighbour's value, or as they were (corners of the reference's
+    // hierarchy always)
+    auto store = [&](int yy, const float (&o)[4], bool corners) {
       if (!mine || X >= w || yy < ya || yy >= yb) return;
       S *dst = a.out + (size_t)yy * P + X;
-      if (X + 3 < w) {
+      if (X + 3 < w && (corners || !(west || pe == 3))) {
         St::st4(dst, make_float4(o[0], o[1], o[2], o[3]));
       } else {
 #pragma unroll
-        for (int b = 0; b < 3; b++)
-          if (X + b < w) dst[b] = St::fromf(o[b]);
+        for (int b = 0; b < 4; b++)
+          if (X + b < w && (corners || !((b == 0 && west) || b == pe))) dst[b] = St::fromf(o[b]);
       }
+    };
+    auto old = [&](int xx, int yy) {
+      return a.zero_init ? 0.0f : St::ldg1(a.in + (size_t)yy * P + xx);
     };
 #pragma unroll
     for (int r = 0; r < R; r++) {
       const int yy = y + r;
       if (yy >= h) break;
       float o[4] = {A[r].x, B[r].x, A[r].y, B[r].y};
-      // columns 0 and w-1: the inner neighbour's value, or as they were
-      const float left = __shfl_up_sync(0xffffffffu, B[r].y, 1);
-      const float in[4] = {left, A[r].x, B[r].x, A[r].y};
-      if (yy == 0 || yy == h - 1) {
-        if (zg) continue;  // written with rows 1 and h-2
+      const float in[4] = {__shfl_up_sync(0xffffffffu, B[r].y, 1), o[0], o[1], o[2]};
+      if (zg) {
+        if (west) o[0] = o[1];
 #pragma unroll
-        for (int b = 0; b < 4; b++) o[b] = X + b < w ? old(X + b, yy) : 0.0f;
-        store(yy, o);
-        continue;
+        for (int b = 0; b < 4; b++)
+          if (b == pe) o[b] = in[b];
+        if (yy >= 1 && yy < h - 1) store(yy, o, true);
+        if (yy == 1) store(0, o, ext);
+        if (yy == h - 2) store(h - 1, o, ext);
+      } else {
+#pragma unroll
+        for (int b = 0; b < 4; b++)
+          if (X + b < w && (yy == 0 || yy == h - 1 || (b == 0 && west) || b == pe))
+            o[b] = old(X + b, yy);
+        store(yy, o, true);
       }
-      if (first && lane == 0) o[0] = zg ? o[1] : old(0, yy);
+    }
+    // corners that hold what was there before
+    if (zg && !ext && a.in != a.out && mine && (west || (pe >= 0 && pe < 4))) {
 #pragma unroll
-      for (int b = 0; b < 4; b++)
-        if (X + b == w - 1) o[b] = zg ? in[b] : old(w - 1, yy);
-      store(yy, o);
-      if (zg && (yy == 1 || yy == h - 2)) {
-        const int ye = yy == 1 ? 0 : h - 1;
-        if (!ext) {  // corner cells are left as they were
-          if (first && lane == 0) o[0] = old(0, ye);
-#pragma unroll
-          for (int b = 0; b < 4; b++)
-            if (X + b == w - 1) o[b] = old(w - 1, ye);
-        }
-        store(ye, o);
+      for (int r = 0; r < R; r++) {
+        const int yy = y + r;
+        if ((yy != 0 && yy != h - 1) || yy < ya || yy >= yb) continue;
+        S *dst = a.out + (size_t)yy * P;
+        if (west) dst[0] = St::fromf(old(0, yy));
+        if (pe >= 0 && pe < 4) dst[w - 1] = St::fromf(old(w - 1, yy));
       }
     }
   }
