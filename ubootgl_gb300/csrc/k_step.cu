@@ -48,6 +48,7 @@ Profiler::~Profiler() {
 namespace {
 
 constexpr int BX = 32, BY = 8;
+constexpr int VX = 64, VY = 4;  // row-vector kernels: 4 faces per thread
 
 __device__ __forceinline__ float ld(const float *p, int pitch, int x, int y) {
   return __ldg(p + (size_t)y * pitch + x);
@@ -127,37 +128,73 @@ __device__ void vbc_component(const float *s, float *b0, float *b1, int pitch, i
   }
 }
 
-// The same boundary values from the thread that has just computed interior
+// The same boundary values from a thread that knows the value v of interior
 // face (x, y): the cells of the edge next to it and, next to two edges, the
 // corner.  In the step this replaces six launches of edge cells only (setVBCs
-// five times, setPBC), 2 to 3 us each: 107 -> 97 us per step at 256x128.  old(x, y): the edge's value before; put(x, y, value) stores.  Each
-// edge cell's old value is read by this thread alone, and before it is
-// overwritten.
+// five times, setPBC), 2 to 3 us each: 107 -> 97 us per step at 256x128.
+// old(x, y): the edge's value before, which only an inflow keeps; put(x, y,
+// value) stores.  Each edge cell's old value is read by this thread alone, and
+// before it is overwritten.
 template <bool XPAR, class Old, class Put>
 __device__ __forceinline__ void edge_cells(int x, int y, float v, int w, int h, Bcs bc, Old &&old,
                                            Put &&put) {
-  auto edge_x = [&](int side, float a, float b) {
-    return XPAR ? vbc_par(side, a, b) : vbc_per(side, a, b);
+  auto edge_x = [&](int side, float a, auto &&b) {
+    if (side == UBG_BC_INFLOW) return b();
+    return XPAR ? vbc_par(side, a, 0.0f) : vbc_per(side, a, 0.0f);
   };
-  auto edge_y = [&](int side, float a, float b) {
-    return XPAR ? vbc_per(side, a, b) : vbc_par(side, a, b);
+  auto edge_y = [&](int side, float a, auto &&b) {
+    if (side == UBG_BC_INFLOW) return b();
+    return XPAR ? vbc_per(side, a, 0.0f) : vbc_par(side, a, 0.0f);
   };
   const bool W = x == 1, E = x == w - 2, S = y == 1, N = y == h - 2;
   float l = 0.0f, r = 0.0f;
-  if (W) l = edge_x(bc.w, v, old(0, y));
-  if (E) r = edge_x(bc.e, v, old(w - 1, y));
+  if (W) l = edge_x(bc.w, v, [&] { return old(0, y); });
+  if (E) r = edge_x(bc.e, v, [&] { return old(w - 1, y); });
 #pragma unroll 1
   for (int k = 0; k < 2; k++) {
     if (!(k ? N : S)) continue;
     const int ye = k ? h - 1 : 0, side = k ? bc.n : bc.s;
-    const float o = old(x, ye);
-    if (W) put(0, ye, edge_y(side, l, edge_x(bc.w, o, old(0, ye))));
-    if (E) put(w - 1, ye, edge_y(side, r, edge_x(bc.e, o, old(w - 1, ye))));
-    put(x, ye, edge_y(side, v, o));
+    if (W)
+      put(0, ye, edge_y(side, l, [&] {
+            return edge_x(bc.w, old(x, ye), [&] { return old(0, ye); });
+          }));
+    if (E)
+      put(w - 1, ye, edge_y(side, r, [&] {
+            return edge_x(bc.e, old(x, ye), [&] { return old(w - 1, ye); });
+          }));
+    put(x, ye, edge_y(side, v, [&] { return old(x, ye); }));
   }
   if (W) put(0, y, l);
   if (E) put(w - 1, y, r);
 }
+// Calls fn(x, y) for the faces of a block (4 VX x VY cells) that have an edge
+// of vx, vy or p next to them, a face per thread, once the block's faces are
+// written (fn reads them back).  As four faces in turn by the thread that wrote
+// them, with the old values of every kind of edge read, each of the three
+// kernels that do this took 4 us more than without (256x128).
+template <class F>
+__device__ __forceinline__ void edge_faces(const int bx, const int by, const int W, const int H,
+                                           F &&fn) {
+  const int x0 = bx * 4 * VX, y0 = by * VY, tid = threadIdx.y * VX + threadIdx.x;
+  const bool cols = x0 <= 1 || x0 + 4 * VX > W - 3;
+  if (!cols && y0 > 1 && y0 + VY <= H - 3) return;
+  __syncthreads();
+  // rows 1, H-3 and H-2, then columns 1, W-3 and W-2 of the other rows
+#pragma unroll 1
+  for (int k = 0; k < 4; k++) {
+    int x, y;
+    if (k < 3) {
+      x = x0 + tid;
+      y = k == 0 ? 1 : H - 4 + k;
+    } else {
+      x = tid / VY == 0 ? 1 : W - 4 + tid / VY;
+      y = y0 + tid % VY;
+      if (tid >= 3 * VY || x < x0 || x >= x0 + 4 * VX || y <= 1 || y >= H - 3) continue;
+    }
+    if (y >= y0 && y < y0 + VY && x >= 1 && x <= W - 2) fn(x, y);
+  }
+}
+
 // Whether faces x .. x + 3 of row y have one next to an edge.
 __device__ __forceinline__ bool near_edge(int x, int y, int w, int h) {
   return x <= 1 || x + 3 >= w - 2 || y == 1 || y == h - 2;
@@ -265,7 +302,6 @@ __global__ void k_face_codes(const uint8_t *__restrict__ flag, uint8_t *cx, uint
 // Row-vector access: a thread handles 4 consecutive faces of one row with
 // float4 loads (x is a multiple of 4 and rows are 128-byte aligned); a block
 // of 64 x 4 threads covers 256 x 4 faces.
-constexpr int VX = 64, VY = 4;
 __device__ __forceinline__ float4 ld4(const float *p, int P, int x, int y) {
   return __ldg(reinterpret_cast<const float4 *>(p + (size_t)y * P + x));
 }
@@ -389,28 +425,22 @@ __device__ __forceinline__ void k_diffuse_body(const VelBufs &v, int srcx, int s
     diffuse4(K, c, ss, n, e, w, a, den, rden, o);
     st4_masked(pick(v.vy, 1 - srcy) + (size_t)y * P, x, 1, W - 2, o);
   }
-  // edges, after both components' loads and stores; not unrolled and with the
-  // values read back: few threads come here, and the others should not pay
-  // registers for it
-  if (EDGES && y >= 1 && y < H - 1 && x <= W - 2 &&
-      (near_edge(x, y, W - 1, H) || near_edge(x, y, W, H - 1))) {
-    const float *sx = pick(v.vx, srcx), *sy = pick(v.vy, srcy);
-    float *dx = pick(v.vx, 1 - srcx), *dy = pick(v.vy, 1 - srcy);
-    const float *ex = EDGES == 1 ? dx : sx;
-#pragma unroll 1
-    for (int xx = max(x, 1); xx <= min(x + 3, W - 2); xx++) {
-      if (xx <= W - 3)
-        edge_cells<true>(
-            xx, y, dx[(size_t)y * P + xx], W - 1, H, bc,
-            [&](int a, int b) { return ex[(size_t)b * P + a]; },
-            [&](int a, int b, float q) { dx[(size_t)b * P + a] = q; });
-      if (y <= H - 3)
-        edge_cells<false>(
-            xx, y, dy[(size_t)y * P + xx], W, H - 1, bc,
-            [&](int a, int b) { return sy[(size_t)b * P + a]; },
-            [&](int a, int b, float q) { dy[(size_t)b * P + a] = q; });
-    }
-  }
+  if (!EDGES) return;
+  const float *sx = pick(v.vx, srcx), *sy = pick(v.vy, srcy);
+  float *dx = pick(v.vx, 1 - srcx), *dy = pick(v.vy, 1 - srcy);
+  const float *ex = EDGES == 1 ? dx : sx;
+  edge_faces(bx, by, W, H, [&](int fx, int fy) {
+    if (fx <= W - 3)
+      edge_cells<true>(
+          fx, fy, dx[(size_t)fy * P + fx], W - 1, H, bc,
+          [&](int a, int b) { return ex[(size_t)b * P + a]; },
+          [&](int a, int b, float q) { dx[(size_t)b * P + a] = q; });
+    if (fy <= H - 3)
+      edge_cells<false>(
+          fx, fy, dy[(size_t)fy * P + fx], W, H - 1, bc,
+          [&](int a, int b) { return sy[(size_t)b * P + a]; },
+          [&](int a, int b, float q) { dy[(size_t)b * P + a] = q; });
+  });
 }
 template <int EDGES>
 __global__ void __launch_bounds__(256) k_diffuse(VelBufs v, int srcx, int srcy,
@@ -967,41 +997,41 @@ __device__ __forceinline__ void k_gradient_body(const VelBufs &v, int fx, int fy
     }
     st4_masked(vx + (size_t)y * P, x, 1, W - 3, ox);
     if (y <= H - 3) st4_masked(vy + (size_t)y * P, x, 1, W - 2, oy);
-    if (EDGES && (near_edge(x, y, W - 1, H) || y >= H - 3)) {
-      float *bx_ = pick(v.vx, 1 - fx), *by_ = pick(v.vy, 1 - fy);
-#pragma unroll 1
-      for (int xx = max(x, 1); xx <= min(x + 3, W - 2); xx++) {
-        if (xx <= W - 3)
-          edge_cells<true>(
-              xx, y, vx[(size_t)y * P + xx], W - 1, H, bc, [&](int a, int b) { return vx[(size_t)b * P + a]; },
-              [&](int a, int b, float q) {
-                vx[(size_t)b * P + a] = bx_[(size_t)b * P + a] = q;
-                m = fmaxf(m, fabsf(q));
-              });
-        if (y <= H - 3)
-          edge_cells<false>(
-              xx, y, vy[(size_t)y * P + xx], W, H - 1, bc, [&](int a, int b) { return vy[(size_t)b * P + a]; },
-              [&](int a, int b, float q) {
-                vy[(size_t)b * P + a] = by_[(size_t)b * P + a] = q;
-                m = fmaxf(m, fabsf(q));
-              });
-        // setPBC, x edges first (so a corner is two of them)
-        const float pc = p[(size_t)y * P + xx];
-        const bool w1 = xx == 1, e1 = xx == W - 2;
-        const float l = single_pbc(bc.w, pc), r = single_pbc(bc.e, pc);
-        if (w1) p[(size_t)y * P] = l;
-        if (e1) p[(size_t)y * P + W - 1] = r;
-#pragma unroll 1
-        for (int k = 0; k < 2; k++) {
-          if (y != (k ? H - 2 : 1)) continue;
-          float *row = p + (size_t)(k ? H - 1 : 0) * P;
-          const int side = k ? bc.n : bc.s;
-          row[xx] = single_pbc(side, pc);
-          if (w1) row[0] = single_pbc(side, l);
-          if (e1) row[W - 1] = single_pbc(side, r);
-        }
+  }
+  if (EDGES) {
+    float *vx = pick(v.vx, fx), *vy = pick(v.vy, fy);
+    float *ox = pick(v.vx, 1 - fx), *oy = pick(v.vy, 1 - fy);
+    edge_faces(bx, by, W, H, [&](int xx, int yy) {
+      if (xx <= W - 3)
+        edge_cells<true>(
+            xx, yy, vx[(size_t)yy * P + xx], W - 1, H, bc,
+            [&](int a, int b) { return vx[(size_t)b * P + a]; },
+            [&](int a, int b, float q) {
+              vx[(size_t)b * P + a] = ox[(size_t)b * P + a] = q;
+              m = fmaxf(m, fabsf(q));
+            });
+      if (yy <= H - 3)
+        edge_cells<false>(
+            xx, yy, vy[(size_t)yy * P + xx], W, H - 1, bc,
+            [&](int a, int b) { return vy[(size_t)b * P + a]; },
+            [&](int a, int b, float q) {
+              vy[(size_t)b * P + a] = oy[(size_t)b * P + a] = q;
+              m = fmaxf(m, fabsf(q));
+            });
+      // setPBC, x edges first (so a corner is two of them)
+      const float pc = p[(size_t)yy * P + xx];
+      const bool w1 = xx == 1, e1 = xx == W - 2;
+      const float l = single_pbc(bc.w, pc), r = single_pbc(bc.e, pc);
+      if (w1) p[(size_t)yy * P] = l;
+      if (e1) p[(size_t)yy * P + W - 1] = r;
+      if (yy == 1 || yy == H - 2) {
+        float *row = p + (size_t)(yy == 1 ? 0 : H - 1) * P;
+        const int side = yy == 1 ? bc.s : bc.n;
+        row[xx] = single_pbc(side, pc);
+        if (w1) row[0] = single_pbc(side, l);
+        if (e1) row[W - 1] = single_pbc(side, r);
       }
-    }
+    });
   }
   if (umax_bits) {
     // one atomic per block: per-warp atomics on one address serialise
