@@ -430,24 +430,28 @@ __device__ __forceinline__ void k_diffuse_body(const VelBufs &v, int srcx, int s
   float *dx = pick(v.vx, 1 - srcx), *dy = pick(v.vy, 1 - srcy);
   const float *ex = EDGES == 1 ? dx : sx;
   edge_faces(bx, by, W, H, [&](int fx, int fy) {
-    if (fx <= W - 3)
+    if ((comps & 1) && fx <= W - 3)
       edge_cells<true>(
           fx, fy, dx[(size_t)fy * P + fx], W - 1, H, bc,
           [&](int a, int b) { return ex[(size_t)b * P + a]; },
           [&](int a, int b, float q) { dx[(size_t)b * P + a] = q; });
-    if (fy <= H - 3)
+    if ((comps & 2) && fy <= H - 3)
       edge_cells<false>(
           fx, fy, dy[(size_t)fy * P + fx], W, H - 1, bc,
           [&](int a, int b) { return sy[(size_t)b * P + a]; },
           [&](int a, int b, float q) { dy[(size_t)b * P + a] = q; });
   });
 }
+// A block takes one component of the velocity (blockIdx.z): 256x128 74.9 ->
+// 70.9 us per step, 4096x2048 600 -> 594, against both one after the other.
+// The members of a batch fill the chip as they are and take both (16 served
+// simulations: 9.09 against 9.16 ms).
 template <int EDGES>
 __global__ void __launch_bounds__(256) k_diffuse(VelBufs v, int srcx, int srcy,
                                                  const StepScalars *__restrict__ sc, int comps,
                                                  Bcs bc) {
   griddep_wait();
-  k_diffuse_body<EDGES>(v, srcx, srcy, sc, comps, bc, blockIdx.x, blockIdx.y);
+  k_diffuse_body<EDGES>(v, srcx, srcy, sc, comps & (1 << blockIdx.z), bc, blockIdx.x, blockIdx.y);
   griddep_launch();
 }
 
@@ -1235,7 +1239,7 @@ void launch_diffuse_sweep(const VelBufs &v, int srcx, int srcy, const StepScalar
                           cudaStream_t st, int edges, Bcs bc) {
   ProfScope ps_(KC_DIFFUSE, st);
   auto *k = edges == 0 ? k_diffuse<0> : (edges == 1 ? k_diffuse<1> : k_diffuse<2>);
-  launch_pdl(k, grid_vec(v.W, v.H), dim3(VX, VY), 0, st, v, srcx, srcy, sc, comps, bc);
+  launch_pdl(k, grid_vec(v.W, v.H, 2), dim3(VX, VY), 0, st, v, srcx, srcy, sc, comps, bc);
   UBG_LAUNCH_CHECK();
   g_stats.launches++;
 }
