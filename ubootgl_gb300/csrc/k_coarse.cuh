@@ -66,7 +66,7 @@ constexpr int kArgs = 0, kArgsBytes = 1024, kXch = kArgs + kArgsBytes,
 // A level's registers: two rows, columns (0, 2) and (1, 3).
 struct Regs {
   float2 A[2], B[2], FA[2], FB[2];     // e and f h^2
-  float2 sA[2], sB[2];                 // factors (tile::scaled2)
+  float2 sA[2], sB[2], cA[2], cB[2];   // factors (tile::scaled2)
   unsigned cw[2];
 };
 // Where a lane is in its level.
@@ -129,7 +129,7 @@ __device__ __forceinline__ void half(Regs &q, const Place &pl, float2 *xch, cons
     const float2 v = tile::add2(tile::add2(tile::add2(we, S), N), onB ? q.FB[r] : q.FA[r]);
     const float2 s = onB ? q.sB[r] : q.sA[r];
     r2[r] = CAREFUL ? make_float2(tile::scaled_any(v.x, s.x), tile::scaled_any(v.y, s.y))
-                    : tile::scaled2(v, s);
+                    : tile::scaled2(v, s, onB ? q.cB[r] : q.cA[r]);
   }
   (RED ? q.B[0] : q.A[0]) = r2[0];
   (RED ? q.A[1] : q.B[1]) = r2[1];
@@ -241,6 +241,8 @@ __device__ __forceinline__ void visit(const Args<S> &a, const int t, const bool 
     q.FB[r] = make_float2(F[1], F[3]);
     q.sA[r] = make_float2(s[0], s[2]);
     q.sB[r] = make_float2(s[1], s[3]);
+    q.cA[r] = tile::third2(q.sA[r]);
+    q.cB[r] = tile::third2(q.sB[r]);
     q.cw[r] = c;
     sq = f2_fma(q.FB[r], q.FB[r], f2_fma(q.FA[r], q.FA[r], sq));
     sq = f2_fma(q.B[r], q.B[r], f2_fma(q.A[r], q.A[r], sq));

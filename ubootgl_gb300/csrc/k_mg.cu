@@ -289,7 +289,6 @@ __global__ void __launch_bounds__(32 * NW, 1024 / (32 * NW)) k_tile(MgArgsT<S, S
   tile::fill_lut(reinterpret_cast<float2 *>(smem_raw + tile::Mem<R, NW>::lut), threadIdx.x, a.wsum,
                  a.rwsum);
   __syncthreads();
-  griddep_wait();
   tile::run<S, SC, EXT, PRE, R, NW>(a, (int)blockIdx.x, smem_raw);
 }
 // One launch over the members of a batch (FP32): block -> member -> region.

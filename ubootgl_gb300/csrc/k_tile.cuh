@@ -94,9 +94,11 @@ __device__ __forceinline__ float2 rnd2(float2 v) {
 // or one without fluid neighbours).  n = 1, 2, 4 are exact products; n = 3 is
 // Markstein's correction, whose remainder v - 3 q is exact for every finite v,
 // subnormal results included (3 has two bits).  For finite sums only: 0 *
-// infinity would be NaN.
-__device__ __forceinline__ float2 scaled2(float2 v, float2 s) {
-  const float2 c = make_float2(s.x == kThird ? kThird : 0.0f, s.y == kThird ? kThird : 0.0f);
+// infinity would be NaN.  c: third2(s).
+__device__ __forceinline__ float2 third2(float2 s) {
+  return make_float2(s.x == kThird ? kThird : 0.0f, s.y == kThird ? kThird : 0.0f);
+}
+__device__ __forceinline__ float2 scaled2(float2 v, float2 s, float2 c) {
   const float2 q = f2_mul(v, s);
   return f2_fma(f2_fma(q, f2(-3.0f), v), c, q);
 }
@@ -235,6 +237,7 @@ __device__ __forceinline__ void run(const MgArgsT<S, SC> &a, const int region,
   // ---- loads: all in flight together; f is copied to shared memory (16
   // registers less while the rest arrives, and there for the residual)
   const bool inner = !first && !has_east && y0 > 0 && y0 + RY < h - 1;  // no bounds to check
+  griddep_wait();
   const bool colok = X < w;
   const size_t o0 = (size_t)y * P + X;
   float4 pv[R];
@@ -351,8 +354,11 @@ __device__ __forceinline__ void run(const MgArgsT<S, SC> &a, const int region,
     }
   }
 
-  // ---- registers: pairs of p (0 in solid cells) and of f h^2; factors
-  float2 A[R], B[R], FA[R], FB[R];
+  // ---- registers: pairs of p (0 in solid cells) and of f h^2; factors, with
+  // two rows in registers too
+  constexpr bool KEEP = R == 2;
+  float2 A[R], B[R], FA[R], FB[R], sA[KEEP ? R : 1], sB[KEEP ? R : 1], cA[KEEP ? R : 1],
+      cB[KEEP ? R : 1];
   const float hh = a.hh;
   copy_wait();
   float2 sq = make_float2(0.f, 0.f);  // sums of squares of p and f h^2
@@ -373,8 +379,15 @@ __device__ __forceinline__ void run(const MgArgsT<S, SC> &a, const int region,
       float s[4];
 #pragma unroll
       for (int b = 0; b < 4; b++) s[b] = factor[(c >> (8 * b)) & 0x3fu];
-      fac(r, 0) = make_float2(s[0], s[2]);
-      fac(r, 1) = make_float2(s[1], s[3]);
+      if constexpr (KEEP) {
+        sA[r] = make_float2(s[0], s[2]);
+        sB[r] = make_float2(s[1], s[3]);
+        cA[r] = third2(sA[r]);
+        cB[r] = third2(sB[r]);
+      } else {
+        fac(r, 0) = make_float2(s[0], s[2]);
+        fac(r, 1) = make_float2(s[1], s[3]);
+      }
     }
     A[r] = make_float2(p[0], p[2]);
     B[r] = make_float2(p[1], p[3]);
@@ -455,7 +468,14 @@ __device__ __forceinline__ void run(const MgArgsT<S, SC> &a, const int region,
       if (MODE == 0) {
         n = make_float2(v.x * 0.25f, v.y * 0.25f);
       } else {
-        const float2 s = fac(r, onB ? 1 : 0);
+        float2 s, c;
+        if constexpr (KEEP) {
+          s = onB ? sB[r] : sA[r];
+          c = onB ? cB[r] : cA[r];
+        } else {
+          s = fac(r, onB ? 1 : 0);
+          c = third2(s);
+        }
         if (EDGE) {
           float2 t = make_float2(!onB && west ? E.x : W.x, W.y);
           if (r == 0 && y == 0) t = Nv;
@@ -467,7 +487,7 @@ __device__ __forceinline__ void run(const MgArgsT<S, SC> &a, const int region,
         if (MODE == 3)
           n = make_float2(scaled_any(v.x, s.x), scaled_any(v.y, s.y));
         else
-          n = scaled2(v, s);
+          n = scaled2(v, s, c);
       }
       n = rnd2<S>(n);
       own = n;
