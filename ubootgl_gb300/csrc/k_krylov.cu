@@ -90,44 +90,63 @@ __device__ __forceinline__ void df_axpy(float &h, float &l, float a, float d) {
   l = t - (h - s);
 }
 
-// Reduction of up to three sums and a max over the grid, in a fixed order:
-// each block reduces its threads (warp shuffles, then its warps in order)
-// and writes its partials; the last block to finish (a ticket counter)
-// adds the partials of all blocks in block order and stores the results
-// (dst[k] = sum; *mdst = max), then resets the ticket.  The results are the
-// same bits on every run, and no same-address atomics pile up (FP64 atomics
-// to one address from 8192 blocks cost ~90 us per kernel).
+// Sums of a block's 256 values of each v[k] and the maximum of its mx: the
+// sum of v[k] is left in the lanes of warp k, the maximum in those of warp 0.
+// The order is that of a butterfly over each warp followed by the warps in
+// turn; with FP64 additions at 2 lanes per clock and SM, one warp does it for
+// all eight (17 additions instead of 48 per sum).
 template <int N>
-__device__ __forceinline__ void block_reduce(double (&v)[N], unsigned mx, double *const (&dst)[N],
-                                             unsigned *mdst, FcgPartials *pr) {
-  const int tid = threadIdx.y * BX + threadIdx.x;
+__device__ __forceinline__ void block_sum(const double (&v)[N], unsigned mx, double *sum,
+                                          unsigned *m) {
+  __shared__ double part[N][BX * BY];
+  __shared__ unsigned partm[BY];
+  const int lane = threadIdx.x, wid = threadIdx.y;
 #pragma unroll
-  for (int k = 0; k < N; k++)
-    for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+  for (int k = 0; k < N; k++) part[k][wid * 32 + lane] = v[k];
   mx = __reduce_max_sync(0xffffffffu, mx);
-  __shared__ double red[N][BY];
-  __shared__ unsigned redm[BY];
+  if (lane == 0) partm[wid] = mx;
+  __syncthreads();
+  if (wid < N) {
+    const double *a = &part[wid][(lane >> 2) * 32 + (lane & 3)];
+    double t = ((a[0] + a[16]) + (a[8] + a[24])) + ((a[4] + a[20]) + (a[12] + a[28]));
+    t += __shfl_xor_sync(0xffffffffu, t, 2);
+    t += __shfl_xor_sync(0xffffffffu, t, 1);
+    *sum = 0.0;
+    for (int w = 0; w < BY; w++) *sum += __shfl_sync(0xffffffffu, t, 4 * w);
+    *m = partm[0];
+    for (int w = 1; w < BY; w++) *m = max(*m, partm[w]);
+  }
+  __syncthreads();
+}
+
+// Reduction of up to three sums and a max over the grid, in a fixed order:
+// each block writes its partials; the last block to finish (a ticket
+// counter) adds the partials of all blocks in block order, stores the results
+// (dst[k] = sum; *mdst = max), resets the ticket and calls done() in one
+// thread.  The results are the same bits on every run, and no same-address
+// atomics pile up (FP64 atomics to one address from 8192 blocks cost ~90 us
+// per kernel).  done() forms what the next kernel needs of the sums: a
+// quotient in FP64 takes a warp some 150 clocks of the SM's FP64 pipe, and
+// formed by every thread it was about 2 us of each kernel.  With that, the
+// sums above and launches that overlap, a step at 1024x512 (19 iterations)
+// went from 1348 to 1133 us.
+template <int N, class F>
+__device__ __forceinline__ void block_reduce(double (&v)[N], unsigned mx, double *const (&dst)[N],
+                                             unsigned *mdst, FcgPartials *pr, F &&done) {
+  const int tid = threadIdx.y * BX + threadIdx.x, wid = threadIdx.y;
   __shared__ bool last;
-  if ((tid & 31) == 0) {
-#pragma unroll
-    for (int k = 0; k < N; k++) red[k][tid >> 5] = v[k];
-    redm[tid >> 5] = mx;
-  }
-  __syncthreads();
-  if (tid == 0) {
-#pragma unroll
-    for (int k = 0; k < N; k++) {
-      double t = 0.0;
-      for (int i = 0; i < BY; i++) t += red[k][i];
-      pr->v[blockIdx.x][k] = t;
-    }
-    unsigned m = 0;
-    for (int i = 0; i < BY; i++) m = max(m, redm[i]);
-    pr->m[blockIdx.x] = m;
+  double sum = 0.0;
+  unsigned m = 0u;
+  block_sum<N>(v, mx, &sum, &m);
+  if (threadIdx.x == 0 && wid < N) {
+    pr->v[blockIdx.x][wid] = sum;
+    if (wid == 0) pr->m[blockIdx.x] = m;
     __threadfence();
-    last = atomicAdd(&pr->ticket, 1u) == gridDim.x - 1;
   }
   __syncthreads();
+  if (tid == 0) last = atomicAdd(&pr->ticket, 1u) == gridDim.x - 1;
+  __syncthreads();
+  griddep_launch();
   if (!last) return;
   __threadfence();
   // the last block: every thread adds the partials of blocks tid, tid + 256,
@@ -135,7 +154,7 @@ __device__ __forceinline__ void block_reduce(double (&v)[N], unsigned mx, double
   // fixed order as above
   const int nb = (int)gridDim.x;
   double t[N];
-  unsigned m = 0;
+  m = 0u;
 #pragma unroll
   for (int k = 0; k < N; k++) t[k] = 0.0;
   for (int b = tid; b < nb; b += BX * BY) {
@@ -143,29 +162,23 @@ __device__ __forceinline__ void block_reduce(double (&v)[N], unsigned mx, double
     for (int k = 0; k < N; k++) t[k] += __ldcg(&pr->v[b][k]);
     m = max(m, __ldcg(&pr->m[b]));
   }
+  block_sum<N>(t, m, &sum, &m);
+  if (threadIdx.x == 0 && wid < N) {
 #pragma unroll
-  for (int k = 0; k < N; k++)
-    for (int o = 16; o > 0; o >>= 1) t[k] += __shfl_xor_sync(0xffffffffu, t[k], o);
-  m = __reduce_max_sync(0xffffffffu, m);
-  __syncthreads();  // red / redm are reused
-  if ((tid & 31) == 0) {
-#pragma unroll
-    for (int k = 0; k < N; k++) red[k][tid >> 5] = t[k];
-    redm[tid >> 5] = m;
+    for (int k = 0; k < N; k++)
+      if (k == wid && dst[k]) *dst[k] = sum;
+    if (wid == 0 && mdst) *mdst = m;
   }
   __syncthreads();
   if (tid == 0) {
-#pragma unroll
-    for (int k = 0; k < N; k++) {
-      double sum = 0.0;
-      for (int i = 0; i < BY; i++) sum += red[k][i];
-      if (dst[k]) *dst[k] = sum;
-    }
-    unsigned mm = 0;
-    for (int i = 0; i < BY; i++) mm = max(mm, redm[i]);
-    if (mdst) *mdst = mm;
+    pr->ticket = 0u;
+    done();
   }
-  if (tid == 0) pr->ticket = 0u;
+}
+template <int N>
+__device__ __forceinline__ void block_reduce(double (&v)[N], unsigned mx, double *const (&dst)[N],
+                                             unsigned *mdst, FcgPartials *pr) {
+  block_reduce<N>(v, mx, dst, mdst, pr, [] {});
 }
 
 // Sum of f over the interior fluid cells, the fluid cells of the outflow
@@ -199,16 +212,13 @@ __global__ void __launch_bounds__(BX *BY) k_fcg_fsum(const float *__restrict__ f
   }
   double v[3] = {(double)s, (double)ne, (double)nf};
   double *const dst[3] = {&sc->fsum, &sc->neast, &sc->nfluid};
-  block_reduce<3>(v, 0u, dst, nullptr, pr);
-}
-
-// The compatibility correction: (on the outflow column, everywhere else)
-// in FP32, formed once per launch.
-__device__ __forceinline__ float2 compat_corr(const FcgScalars *sc) {
-  const double ne = sc->neast, nf = sc->nfluid;
-  if (ne > 0.0) return make_float2((float)(sc->fsum / ne), 0.0f);
-  const float a = nf > 0.0 ? (float)(sc->fsum / nf) : 0.0f;
-  return make_float2(a, a);
+  // the compatibility correction: on the outflow column, everywhere else
+  block_reduce<3>(v, 0u, dst, nullptr, pr, [&] {
+    const double ne = sc->neast, nf = sc->nfluid;
+    const float a = nf > 0.0 ? (float)(sc->fsum / nf) : 0.0f;
+    sc->corr[0] = ne > 0.0 ? (float)(sc->fsum / ne) : a;
+    sc->corr[1] = ne > 0.0 ? 0.0f : a;
+  });
 }
 
 // r = f_c + ihsq * sum_n flag_n (x_n - x) on the interior fluid cells (0
@@ -224,7 +234,7 @@ __global__ void __launch_bounds__(BX *BY) k_fcg_resid(const float *__restrict__ 
   griddep_wait();
   float ff = 0.0f, rr = 0.0f;
   unsigned mx = 0;
-  const float2 corr = compat_corr(sc);
+  const float2 corr = make_float2(sc->corr[0], sc->corr[1]);
   // grid-stride over tiles of 128 x 8 cells: a few blocks per SM, so few
   // partial sums to combine
   const int tiles_x = (W + 4 * BX - 1) / (4 * BX), ntiles = tiles_x * ((H + BY - 1) / BY);
@@ -358,25 +368,19 @@ __global__ void __launch_bounds__(BX *BY) k_fcg_zsum(const float *__restrict__ z
   }
   double v[1] = {(double)s};
   double *const dst[1] = {&sc->zsum};
-  block_reduce<1>(v, 0u, dst, nullptr, pr);
+  block_reduce<1>(v, 0u, dst, nullptr, pr, [&] {
+    sc->zmean = sc->nfluid > 0.0 ? (float)(sc->zsum / sc->nfluid) : 0.0f;
+  });
 }
 
-__device__ __forceinline__ float z_mean(const FcgScalars *sc) {
-  return sc->nfluid > 0.0 ? (float)(sc->zsum / sc->nfluid) : 0.0f;
-}
-
-// zq = (z - zm, q_prev), zm the mean of z over the interior fluid cells;
-// zeroes the accumulators of k_fcg_dir.
+// zq = (z - zm, q_prev), zm the mean of z over the interior fluid cells, and
+// beta = -zq / dq_prev.
 __global__ void __launch_bounds__(BX *BY) k_fcg_zq(const float *__restrict__ z,
                                                    const float *__restrict__ q, int W, int H,
                                                    int P, FcgScalars *sc, int slot,
                                                    FcgPartials *pr) {
   griddep_wait();
-  const float zm = z_mean(sc);
-  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && threadIdx.y == 0) {
-    sc->dq[slot] = 0.0;
-    sc->dr = 0.0;
-  }
+  const float zm = sc->zmean;
   float s = 0.0f;
   // grid-stride over tiles of 128 x 8 cells, four tiles per pass with
   // their loads issued together
@@ -405,14 +409,14 @@ __global__ void __launch_bounds__(BX *BY) k_fcg_zq(const float *__restrict__ z,
   }
   double v[1] = {(double)s};
   double *const dst[1] = {&sc->zq};
-  block_reduce<1>(v, 0u, dst, nullptr, pr);
+  block_reduce<1>(v, 0u, dst, nullptr, pr,
+                  [&] { sc->beta = (float)(-sc->zq / sc->dq[slot ^ 1]); });
 }
 
-// d = (z - zm) + beta d_old (beta = -zq / dq_prev; 0 on the first
-// iteration) on the interior fluid cells and the edges, d = 0 on the
+// d = (z - zm) + beta d_old (beta 0 on the first iteration) on the interior fluid cells and the edges, d = 0 on the
 // interior solid cells (where z and d_old are 0), q = A d = -ihsq * sum_n
 // flag_n (d_n - d) on the interior fluid cells (0 elsewhere), (d, q) and
-// (d, r); zeroes the accumulators of k_fcg_update.  The shift by zm is
+// (d, r), and alpha = dr / dq.  The shift by zm is
 // applied to every value read, so q sees the stored d of each fluid cell;
 // the values of solid neighbours never enter q.
 __global__ void __launch_bounds__(BX *BY) k_fcg_dir(const float *__restrict__ z,
@@ -422,12 +426,8 @@ __global__ void __launch_bounds__(BX *BY) k_fcg_dir(const float *__restrict__ z,
                                                     int H, int P, float ihsq, FcgScalars *sc,
                                                     int first, int slot, FcgPartials *pr) {
   griddep_wait();
-  const float beta = first ? 0.0f : (float)(-sc->zq / sc->dq[slot ^ 1]);
-  const float zm = z_mean(sc);
-  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && threadIdx.y == 0) {
-    sc->rr = 0.0;
-    sc->maxbits = 0u;
-  }
+  const float beta = first ? 0.0f : sc->beta;
+  const float zm = sc->zmean;
   float dq = 0.0f, dr = 0.0f;
   // grid-stride over tiles of 128 x 8 cells: a few blocks per SM, so few
   // same-address atomics in the final reduction
@@ -515,20 +515,20 @@ __global__ void __launch_bounds__(BX *BY) k_fcg_dir(const float *__restrict__ z,
   }
   double v[2] = {(double)dq, (double)dr};
   double *const dst[2] = {&sc->dq[slot], &sc->dr};
-  block_reduce<2>(v, 0u, dst, nullptr, pr);
+  block_reduce<2>(v, 0u, dst, nullptr, pr, [&] {
+    const double dq = sc->dq[slot];
+    sc->alpha = (float)(dq != 0.0 ? sc->dr / dq : 0.0);
+  });
 }
 
-// alpha = dr / dq; x += alpha d (double-float, the product exact); r -=
-// alpha q; ||r||^2 and max|r|; zeroes the accumulator of the next k_fcg_zq.
+// x += alpha d (double-float, the product exact); r -= alpha q; ||r||^2 and
+// max|r|.
 __global__ void __launch_bounds__(BX *BY) k_fcg_update(float *xh, float *xl,
                                                        const float *__restrict__ d, float *r,
                                                        const float *__restrict__ q, int W, int H,
-                                                       int P, FcgScalars *sc, int slot,
-                                                       FcgPartials *pr) {
+                                                       int P, FcgScalars *sc, FcgPartials *pr) {
   griddep_wait();
-  const double dqv = sc->dq[slot];
-  const float af = (float)(dqv != 0.0 ? sc->dr / dqv : 0.0);
-  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && threadIdx.y == 0) sc->zq = 0.0;
+  const float af = sc->alpha;
   float rr = 0.0f;
   unsigned mx = 0;
   const int tiles_x = (W + 4 * BX - 1) / (4 * BX), ntiles = tiles_x * ((H + BY - 1) / BY);
@@ -770,18 +770,18 @@ int fcg_solve(FcgSolver &fs, const uint8_t *flag, const float *f, float *p, doub
   UBG_CUDA(cudaMemsetAsync(fs.dev, 0, sizeof(FcgScalars), st));
   {
     ProfScope ps_(KC_KRYLOV, st);
-    k_fcg_load<<<grid, blk, 0, st>>>(p, fs.xh, fs.xl, W, H, P);
+    launch_pdl(k_fcg_load, grid, blk, 0, st, p, fs.xh, fs.xl, W, H, P);
   }
   UBG_LAUNCH_CHECK();
   {
     ProfScope ps_(KC_KRYLOV, st);
-    k_fcg_fsum<<<g_fsum, blk, 0, st>>>(f, L0.code, W, H, P, fs.dev, fs.part);
+    launch_pdl(k_fcg_fsum, g_fsum, blk, 0, st, f, L0.code, W, H, P, fs.dev, fs.part);
   }
   UBG_LAUNCH_CHECK();
   {
     ProfScope ps_(KC_KRYLOV, st);
-    k_fcg_resid<<<g_resid, blk, 0, st>>>(fs.xh, fs.xl, f, L0.code, W, H, P, ihsq, r, fs.dev, 1,
-                                       fs.part);
+    launch_pdl(k_fcg_resid, g_resid, blk, 0, st, fs.xh, fs.xl, f, L0.code, W, H, P, ihsq, r, fs.dev,
+               1, fs.part);
   }
   UBG_LAUNCH_CHECK();
   g_stats.launches += 3;
@@ -811,8 +811,8 @@ int fcg_solve(FcgSolver &fs, const uint8_t *flag, const float *f, float *p, doub
     UBG_CUDA(cudaMemsetAsync(&fs.dev->maxbits, 0, sizeof(unsigned), st));
     {
       ProfScope ps_(KC_KRYLOV, st);
-      k_fcg_resid<<<g_resid, blk, 0, st>>>(fs.xh, fs.xl, f, L0.code, W, H, P, ihsq, r, fs.dev, 0,
-                                         fs.part);
+      launch_pdl(k_fcg_resid, g_resid, blk, 0, st, fs.xh, fs.xl, f, L0.code, W, H, P, ihsq, r,
+                 fs.dev, 0, fs.part);
     }
     UBG_LAUNCH_CHECK();
     g_stats.launches++;
@@ -839,29 +839,29 @@ int fcg_solve(FcgSolver &fs, const uint8_t *flag, const float *f, float *p, doub
     const int slot = it & 1;
     {
       ProfScope ps_(KC_KRYLOV, st);
-      k_fcg_zsum<<<g_zsum, blk, 0, st>>>(z, L0.code, W, H, P, fs.dev, fs.part);
+      launch_pdl(k_fcg_zsum, g_zsum, blk, 0, st, z, L0.code, W, H, P, fs.dev, fs.part);
     }
     UBG_LAUNCH_CHECK();
     g_stats.launches++;
     if (it > 0) {  // (also zeroes the accumulators of k_fcg_dir)
       {
         ProfScope ps_(KC_KRYLOV, st);
-        k_fcg_zq<<<g_zq, blk, 0, st>>>(z, fs.q, W, H, P, fs.dev, slot, fs.part);
+        launch_pdl(k_fcg_zq, g_zq, blk, 0, st, z, fs.q, W, H, P, fs.dev, slot, fs.part);
       }
       UBG_LAUNCH_CHECK();
       g_stats.launches++;
     }
     {
       ProfScope ps_(KC_KRYLOV, st);
-      k_fcg_dir<<<g_dir, blk, 0, st>>>(z, fs.d[cur_d], fs.d[cur_d ^ 1], fs.q, r, L0.code, W, H, P,
-                                      ihsq, fs.dev, first ? 1 : 0, slot, fs.part);
+      launch_pdl(k_fcg_dir, g_dir, blk, 0, st, z, fs.d[cur_d], fs.d[cur_d ^ 1], fs.q, r, L0.code, W,
+                 H, P, ihsq, fs.dev, first ? 1 : 0, slot, fs.part);
     }
     UBG_LAUNCH_CHECK();
     cur_d ^= 1;
     {
       ProfScope ps_(KC_KRYLOV, st);
-      k_fcg_update<<<g_update, blk, 0, st>>>(fs.xh, fs.xl, fs.d[cur_d], r, fs.q, W, H, P, fs.dev, slot,
-                                            fs.part);
+      launch_pdl(k_fcg_update, g_update, blk, 0, st, fs.xh, fs.xl, fs.d[cur_d], r, fs.q, W, H, P,
+                 fs.dev, fs.part);
     }
     UBG_LAUNCH_CHECK();
     g_stats.launches += 2;
@@ -878,7 +878,7 @@ int fcg_solve(FcgSolver &fs, const uint8_t *flag, const float *f, float *p, doub
   if (diverged || rr > start_rr) {
     {
       ProfScope ps_(KC_KRYLOV, st);
-      k_fcg_load<<<grid, blk, 0, st>>>(p, fs.xh, fs.xl, W, H, P);
+      launch_pdl(k_fcg_load, grid, blk, 0, st, p, fs.xh, fs.xl, W, H, P);
     }
     UBG_LAUNCH_CHECK();
     g_stats.launches++;
@@ -886,7 +886,7 @@ int fcg_solve(FcgSolver &fs, const uint8_t *flag, const float *f, float *p, doub
   } else {
     {
       ProfScope ps_(KC_KRYLOV, st);
-      k_fcg_store<<<grid, blk, 0, st>>>(fs.xh, fs.xl, p, W, H, P);
+      launch_pdl(k_fcg_store, grid, blk, 0, st, fs.xh, fs.xl, p, W, H, P);
     }
     UBG_LAUNCH_CHECK();
     g_stats.launches++;
@@ -899,8 +899,8 @@ void launch_gradient_df(const VelBufs &v, int fx, int fy, const float *xh, const
                         const StepScalars *sc, unsigned *umax_bits, cudaStream_t st) {
   ProfScope ps_(KC_GRADIENT, st);
   const dim3 grid((v.W + 4 * BX - 1) / (4 * BX), (v.H + BY - 1) / BY);
-  k_gradient_df<<<grid, dim3(BX, BY), 0, st>>>(fx ? v.vx[1] : v.vx[0], fy ? v.vy[1] : v.vy[0], v.cx,
-                                                v.cy, xh, xl, v.W, v.H, v.pitch, sc, umax_bits);
+  launch_pdl(k_gradient_df, grid, dim3(BX, BY), 0, st, fx ? v.vx[1] : v.vx[0],
+             fy ? v.vy[1] : v.vy[0], v.cx, v.cy, xh, xl, v.W, v.H, v.pitch, sc, umax_bits);
   UBG_LAUNCH_CHECK();
   g_stats.launches++;
 }

@@ -467,7 +467,10 @@ struct FcgScalars {
   double nfluid;   // interior fluid cells
   double zsum;     // sum of the preconditioned residual z over the interior fluid cells
   unsigned maxbits;  // max|r| as float bits
-  unsigned pad;
+  float zmean;       // zsum / nfluid
+  float beta;        // -zq / dq of the previous iteration
+  float alpha;       // dr / dq
+  float corr[2];     // f_c - f on the outflow column and elsewhere
 };
 
 // Per-block partial sums of the Krylov reductions (summed in block order by
