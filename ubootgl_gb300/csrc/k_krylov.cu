@@ -175,10 +175,12 @@ __device__ __forceinline__ void block_reduce(double (&v)[N], unsigned mx, double
     done();
   }
 }
-template <int N>
-__device__ __forceinline__ void block_reduce(double (&v)[N], unsigned mx, double *const (&dst)[N],
-                                             unsigned *mdst, FcgPartials *pr) {
-  block_reduce<N>(v, mx, dst, mdst, pr, [] {});
+// The residual's norm to the host, which waits for the number (fcg_solve).
+__device__ __forceinline__ void publish(const FcgScalars *sc, FcgResult *out, unsigned seq) {
+  out->ff = sc->ff;
+  out->rr = sc->rr;
+  __threadfence_system();
+  *reinterpret_cast<volatile unsigned *>(&out->seq) = seq;
 }
 
 // Sum of f over the interior fluid cells, the fluid cells of the outflow
@@ -230,7 +232,8 @@ __global__ void __launch_bounds__(BX *BY) k_fcg_resid(const float *__restrict__ 
                                                       const float *__restrict__ f,
                                                       const uint8_t *__restrict__ code, int W,
                                                       int H, int P, float ihsq, float *r,
-                                                      FcgScalars *sc, int want_ff, FcgPartials *pr) {
+                                                      FcgScalars *sc, int want_ff, FcgPartials *pr,
+                                                      FcgResult *out, unsigned seq) {
   griddep_wait();
   float ff = 0.0f, rr = 0.0f;
   unsigned mx = 0;
@@ -313,7 +316,7 @@ __global__ void __launch_bounds__(BX *BY) k_fcg_resid(const float *__restrict__ 
   }
   double v[2] = {(double)ff, (double)rr};
   double *const dst[2] = {want_ff ? &sc->ff : nullptr, &sc->rr};
-  block_reduce<2>(v, mx, dst, &sc->maxbits, pr);
+  block_reduce<2>(v, mx, dst, &sc->maxbits, pr, [&] { publish(sc, out, seq); });
 }
 
 // Sum of z over the interior fluid cells.  A maps a constant on a fluid
@@ -526,7 +529,8 @@ __global__ void __launch_bounds__(BX *BY) k_fcg_dir(const float *__restrict__ z,
 __global__ void __launch_bounds__(BX *BY) k_fcg_update(float *xh, float *xl,
                                                        const float *__restrict__ d, float *r,
                                                        const float *__restrict__ q, int W, int H,
-                                                       int P, FcgScalars *sc, FcgPartials *pr) {
+                                                       int P, FcgScalars *sc, FcgPartials *pr,
+                                                       FcgResult *out, unsigned seq) {
   griddep_wait();
   const float af = sc->alpha;
   float rr = 0.0f;
@@ -575,7 +579,7 @@ __global__ void __launch_bounds__(BX *BY) k_fcg_update(float *xh, float *xl,
   }
   double v[1] = {(double)rr};
   double *const dst[1] = {&sc->rr};
-  block_reduce<1>(v, mx, dst, &sc->maxbits, pr);
+  block_reduce<1>(v, mx, dst, &sc->maxbits, pr, [&] { publish(sc, out, seq); });
 }
 
 // x = p on every cell (warm start from the current pressure; tail 0).
@@ -681,7 +685,7 @@ void fcg_alloc(FcgSolver &fs, int W, int H, int P, float h) {
   UBG_CUDA(cudaMemsetAsync(arena, 0, total, cudaStreamLegacy));
   UBG_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
   void *host = nullptr;
-  if (cudaHostAlloc(&host, sizeof(FcgScalars), cudaHostAllocDefault) != cudaSuccess) {
+  if (cudaHostAlloc(&host, sizeof(FcgResult), cudaHostAllocMapped) != cudaSuccess) {
     cudaGetLastError();
     cudaFree(arena);
     fcg_free(fs);
@@ -702,7 +706,9 @@ void fcg_alloc(FcgSolver &fs, int W, int H, int P, float h) {
   p += a256(n * 4);
   fs.q = (float *)p;
   fs.arena = arena;
-  fs.host = (FcgScalars *)host;
+  fs.host = (FcgResult *)host;
+  fs.host->seq = 0;
+  fs.seq = 0;
   fs.W = W;
   fs.H = H;
   fs.P = P;
@@ -766,6 +772,20 @@ int fcg_solve(FcgSolver &fs, const uint8_t *flag, const float *f, float *p, doub
   const dim3 g_fsum = wave(k_fcg_fsum), g_resid = wave(k_fcg_resid), g_zq = wave(k_fcg_zq),
              g_zsum = wave(k_fcg_zsum),
              g_dir = wave(k_fcg_dir), g_update = wave(k_fcg_update);
+  // Waits for the norm that the last launch of k_fcg_resid or k_fcg_update
+  // writes to host memory, instead of a copy and a synchronisation after it.
+  FcgResult *out = nullptr;
+  UBG_CUDA(cudaHostGetDevicePointer((void **)&out, fs.host, 0));
+  auto read = [&]() {
+    auto arrived = [&] { return __atomic_load_n(&fs.host->seq, __ATOMIC_ACQUIRE) == fs.seq; };
+    for (unsigned i = 1; !arrived(); i++) {
+      if (i % 4096) continue;
+      const cudaError_t e = cudaStreamQuery(st);
+      if (e == cudaErrorNotReady) continue;
+      UBG_CUDA(e);
+      if (!arrived()) throw CudaError("tolerance solver: no residual from the device");
+    }
+  };
   float *r = L0.rhs;  // the V-cycle's level-0 right-hand side is the residual
   UBG_CUDA(cudaMemsetAsync(fs.dev, 0, sizeof(FcgScalars), st));
   {
@@ -781,14 +801,10 @@ int fcg_solve(FcgSolver &fs, const uint8_t *flag, const float *f, float *p, doub
   {
     ProfScope ps_(KC_KRYLOV, st);
     launch_pdl(k_fcg_resid, g_resid, blk, 0, st, fs.xh, fs.xl, f, L0.code, W, H, P, ihsq, r, fs.dev,
-               1, fs.part);
+               1, fs.part, out, ++fs.seq);
   }
   UBG_LAUNCH_CHECK();
   g_stats.launches += 3;
-  auto read = [&]() {
-    UBG_CUDA(cudaMemcpyAsync(fs.host, fs.dev, sizeof(FcgScalars), cudaMemcpyDeviceToHost, st));
-    UBG_CUDA(cudaStreamSynchronize(st));
-  };
   read();
   const double ff = fs.host->ff, target2 = tol * tol * ff;
   // The recurrence r -= alpha q drifts from f_c + L x by FP32 rounding; when
@@ -812,7 +828,7 @@ int fcg_solve(FcgSolver &fs, const uint8_t *flag, const float *f, float *p, doub
     {
       ProfScope ps_(KC_KRYLOV, st);
       launch_pdl(k_fcg_resid, g_resid, blk, 0, st, fs.xh, fs.xl, f, L0.code, W, H, P, ihsq, r,
-                 fs.dev, 0, fs.part);
+                 fs.dev, 0, fs.part, out, ++fs.seq);
     }
     UBG_LAUNCH_CHECK();
     g_stats.launches++;
@@ -861,7 +877,7 @@ int fcg_solve(FcgSolver &fs, const uint8_t *flag, const float *f, float *p, doub
     {
       ProfScope ps_(KC_KRYLOV, st);
       launch_pdl(k_fcg_update, g_update, blk, 0, st, fs.xh, fs.xl, fs.d[cur_d], r, fs.q, W, H, P,
-                 fs.dev, fs.part);
+                 fs.dev, fs.part, out, ++fs.seq);
     }
     UBG_LAUNCH_CHECK();
     g_stats.launches += 2;

@@ -473,6 +473,12 @@ struct FcgScalars {
   float corr[2];     // f_c - f on the outflow column and elsewhere
 };
 
+// What the host reads of them (in host memory, written by the device).
+struct FcgResult {
+  double ff, rr;
+  unsigned seq;  // number of the launch that wrote it
+};
+
 // Per-block partial sums of the Krylov reductions (summed in block order by
 // the last block of each launch) and the ticket that finds that block.
 constexpr int kFcgMaxBlocks = 2048;
@@ -488,7 +494,9 @@ struct FcgSolver {
   int prec = UBG_FP32;
   float *xh = nullptr, *xl = nullptr;  // double-float pressure iterate, pitched like the fields
   float *d[2] = {nullptr, nullptr}, *q = nullptr;
-  FcgScalars *dev = nullptr, *host = nullptr;
+  FcgScalars *dev = nullptr;
+  FcgResult *host = nullptr;  // mapped
+  unsigned seq = 0;           // launches that write it so far
   FcgPartials *part = nullptr;  // zeroed at allocation (ticket 0)
   void *arena = nullptr;
   bool dirty = true;  // the flag changed since the coarse flags were built
@@ -501,7 +509,7 @@ size_t fcg_bytes(int W, int H, int P, int prec);
 void fcg_set_precision(FcgSolver &fs, int prec);
 // Solves the zero-gradient system for p (warm start: p as given; result:
 // p's interior cells, and fs.xh + fs.xl as a double-float) until ||r|| <= tol ||f_c||, at most
-// max_iter iterations (one V-cycle each).  Synchronises once per
+// max_iter iterations (one V-cycle each).  Waits for the device once per
 // iteration.  Returns the iterations run; *rel = ||f_c + L x|| / ||f_c||
 // of the final x.
 int fcg_solve(FcgSolver &fs, const uint8_t *flag, const float *f, float *p, double tol,
