@@ -10,7 +10,7 @@
 // side lie in shared memory (rows of 4 n columns).  Edge cells of the
 // reference's coarse levels are 0 and never updated; a solid cell and an edge
 // cell have the factor 0.  The tolerance hierarchy's edge cells follow their
-// inner neighbour, whose own value then stands for them.
+// inner neighbour (factor -1, as in k_tile.cuh).
 //
 // What bounds it: latency, a few hundred dependent instructions per visit.
 // 64x32 and down: 10.4 us (ncu).  It was 13.6 with the codes read level by
@@ -89,15 +89,15 @@ __device__ __forceinline__ void sync_level(int warps) {
     __syncwarp();
 }
 
-// One half sweep (red or black).  MULTI: the level takes several warps.
-// grad: the edge cells have their inner neighbour's value.
+// One half sweep (red or black).  MULTI: the level takes several warps.  EXT:
+// the edge cells take their inner neighbour's value (follow) or keep theirs.
 template <bool MULTI, bool CAREFUL, bool EXT, int RED>
 __device__ __forceinline__ void half(Regs &q, const Place &pl, float2 *xch, const int w,
-                                     const int h, const bool grad) {
+                                     const int h, const bool follow) {
   auto slot = [&](int buf, int wd, int lastrow) -> float2 & {
     return xch[((buf * (kWarps + 2) + 1 + wd) * 2 + lastrow) * 32];
   };
-  const int n = 1 << pl.lsh, buf = RED ? 0 : 1, xe = w - 2 - pl.X;
+  const int n = 1 << pl.lsh, buf = RED ? 0 : 1;
   // pair updated in row 0: (1, 3) in a red half sweep, (0, 2) in a black one;
   // row 1 the other pair
   float2 below = shfl2_up(RED ? q.B[1] : q.A[1], n), above = shfl2_down(RED ? q.A[0] : q.B[0], n);
@@ -107,7 +107,6 @@ __device__ __forceinline__ void half(Regs &q, const Place &pl, float2 *xch, cons
 #pragma unroll
   for (int r = 0; r < 2; r++) {
     const bool onB = (r ^ RED) != 0;
-    const float2 own = onB ? q.B[r] : q.A[r];
     float2 W, E;
     if (onB) {
       W = q.A[r];
@@ -116,18 +115,18 @@ __device__ __forceinline__ void half(Regs &q, const Place &pl, float2 *xch, cons
       W = make_float2(__shfl_up_sync(0xffffffffu, q.B[r].y, 1), q.B[r].x);
       E = q.B[r];
     }
-    float2 S = r ? (onB ? q.B[0] : q.A[0]) : below, N = r ? above : (onB ? q.B[1] : q.A[1]);
-    if (EXT && grad) {
-      const unsigned c0 = q.cw[r] >> (onB ? 8 : 0), c1 = c0 >> 16;
-      if (onB && pl.X == 0) W.x = (c0 & C_W) ? own.x : 0.0f;
-      if (xe == (onB ? 1 : 0)) E.x = (c0 & C_E) ? own.x : 0.0f;
-      if (xe == (onB ? 3 : 2)) E.y = (c1 & C_E) ? own.y : 0.0f;
-      if (pl.y + r == 1) S = make_float2((c0 & C_S) ? own.x : 0.0f, (c1 & C_S) ? own.y : 0.0f);
-      if (pl.y + r == h - 2) N = make_float2((c0 & C_N) ? own.x : 0.0f, (c1 & C_N) ? own.y : 0.0f);
-    }
+    const float2 S = r ? (onB ? q.B[0] : q.A[0]) : below, N = r ? above : (onB ? q.B[1] : q.A[1]);
     const float2 we = make_float2(W.x + E.x, W.y + E.y);
-    const float2 v = tile::add2(tile::add2(tile::add2(we, S), N), onB ? q.FB[r] : q.FA[r]);
+    float2 v = tile::add2(tile::add2(tile::add2(we, S), N), onB ? q.FB[r] : q.FA[r]);
     const float2 s = onB ? q.sB[r] : q.sA[r];
+    if (EXT) {  // as in k_tile.cuh
+      float2 t = make_float2(!onB && pl.X == 0 ? E.x : W.x, W.y);
+      if (r == 0 && pl.y == 0) t = N;
+      if (pl.y + r == h - 1) t = S;
+      if (!follow) t = onB ? q.B[r] : q.A[r];
+      if (__float_as_int(s.x) < 0) v.x = -t.x;
+      if (__float_as_int(s.y) < 0) v.y = -t.y;
+    }
     r2[r] = CAREFUL ? make_float2(tile::scaled_any(v.x, s.x), tile::scaled_any(v.y, s.y))
                     : tile::scaled2(v, s, onB ? q.cB[r] : q.cA[r]);
   }
@@ -145,7 +144,7 @@ __device__ __forceinline__ void sweeps(Regs &q, const Place &pl, float2 *xch, co
 #pragma unroll 1
   for (int s = 0; s < n; s++) {
     half<MULTI, CAREFUL, EXT, 1>(q, pl, xch, w, h, up || s > 0);
-    half<MULTI, CAREFUL, EXT, 0>(q, pl, xch, w, h, up || s > 0);
+    half<MULTI, CAREFUL, EXT, 0>(q, pl, xch, w, h, true);
   }
 }
 
@@ -215,16 +214,22 @@ __device__ __forceinline__ void visit(const Args<S> &a, const int t, const bool 
   }
   const float hh = L.hh;
   float2 sq = make_float2(0.f, 0.f);
+  unsigned ef[2] = {0u, 0u};  // flags of the edge cells (EXT)
 #pragma unroll
   for (int r = 0; r < 2; r++) {
     const int yy = y + r;
     float4 p4 = make_float4(0.f, 0.f, 0.f, 0.f), fv = p4;
-    unsigned c = 0u;  // smoothed cells' codes, 0 elsewhere
+    unsigned c = 0u;   // smoothed cells' codes, 0 elsewhere
+    unsigned ci = 0u;  // the table's index of each factor
     if (yy < h) {
       fv = *reinterpret_cast<const float4 *>(f + r * stride);
       if (up) p4 = *reinterpret_cast<const float4 *>(e + r * stride);
-      if (yy >= 1 && yy < h - 1)
-        c = *reinterpret_cast<const unsigned *>(code + r * stride) & inmask;
+      const unsigned raw = *reinterpret_cast<const unsigned *>(code + r * stride);
+      const unsigned in = yy >= 1 && yy < h - 1 ? inmask : 0u;
+      c = raw & in;
+      ci = c & 0x1f1f1f1fu;
+      if (EXT) ci |= ~in & ((raw & 0x01010101u) | 0x20202020u);
+      if (EXT) ef[r] = raw & 0x01010101u & ~in;
     }
     float p[4] = {p4.x, p4.y, p4.z, p4.w};
     float F[4] = {fv.x * hh * hh, fv.y * hh * hh, fv.z * hh * hh, fv.w * hh * hh};
@@ -233,7 +238,7 @@ __device__ __forceinline__ void visit(const Args<S> &a, const int t, const bool 
     for (int b = 0; b < 4; b++) {
       if (up) p[b] = p[b] + u[r][b];
       if (!((c >> (8 * b)) & C_CENTER)) p[b] = F[b] = 0.0f;
-      s[b] = reinterpret_cast<const float *>(lut)[(c >> (8 * b)) & 0x1fu];
+      s[b] = reinterpret_cast<const float *>(lut)[(ci >> (8 * b)) & 0x3fu];
     }
     q.A[r] = make_float2(p[0], p[2]);
     q.B[r] = make_float2(p[1], p[3]);
@@ -247,12 +252,39 @@ __device__ __forceinline__ void visit(const Args<S> &a, const int t, const bool 
     sq = f2_fma(q.FB[r], q.FB[r], f2_fma(q.FA[r], q.FA[r], sq));
     sq = f2_fma(q.B[r], q.B[r], f2_fma(q.A[r], q.A[r], sq));
   }
+  if (EXT && up) {  // edge cells: their inner neighbours' corrected values
+    const int pe = w - 1 - X;
+    auto flag = [&](int r, int b, float v) { return (ef[r] >> (8 * b)) & 1u ? v : 0.0f; };
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+      const float left = __shfl_up_sync(0xffffffffu, q.B[r].y, 1);
+      if (X == 0) q.A[r].x = flag(r, 0, q.B[r].x);
+      if (pe == 0) q.A[r].x = flag(r, 0, left);
+      if (pe == 1) q.B[r].x = flag(r, 1, q.A[r].x);
+      if (pe == 2) q.A[r].y = flag(r, 2, q.B[r].x);
+      if (pe == 3) q.B[r].y = flag(r, 3, q.A[r].y);
+    }
+    // rows 0 and h-1 (of the row below for a lane's first row, by shuffle; a
+    // warp's first row is written by the warp below it, further down)
+    const float2 bA = shfl2_up(q.A[1], n), bB = shfl2_up(q.B[1], n);
+    auto row = [&](int r, float2 a, float2 b) {
+      q.A[r] = make_float2(flag(r, 0, a.x), flag(r, 2, a.y));
+      q.B[r] = make_float2(flag(r, 1, b.x), flag(r, 3, b.y));
+    };
+    if (y == 0) row(0, q.A[1], q.B[1]);
+    if (y == h - 1) row(0, bA, bB);
+    if (y + 1 == h - 1) row(1, q.A[0], q.B[0]);
+  }
   // sums that may not stay finite (false for infinities and NaNs too): a warp
   // alone decides for itself, several agree through shared memory
   bool careful = __any_sync(0xffffffffu, !(sq.x + sq.y < tile::kBigSq)) != 0;
   const bool multi = pl.warps > 1;
   if (multi) {
-    if (pl.sub == 0) slot(0, pl.wid, 0) = q.A[0];
+    const bool init = EXT && up;
+    if (pl.sub == 0 && !(init && pl.wid > 0 && y == h - 1)) slot(0, pl.wid, 0) = q.A[0];
+    if (init && pl.sub == pl.groups - 1 && pl.wid < pl.warps - 1 && y + 2 == h - 1)
+      slot(0, pl.wid + 1, 0) = make_float2((q.cw[1] & C_N) ? q.A[1].x : 0.0f,
+                                           ((q.cw[1] >> 16) & C_N) ? q.A[1].y : 0.0f);
     if (pl.sub == pl.groups - 1) slot(0, pl.wid, 1) = q.B[1];
     // the row above the last warp's: zeros
     if (pl.wid == pl.warps - 1 && pl.sub == 0)
