@@ -710,30 +710,39 @@ __device__ __forceinline__ void k_advect_body(const VelBufs &v, int srcx, int sr
   const float reach = finite ? fminf(kReach / fabsf(cfull), 1e30f) : -1.0f;
   bool far = (W | H) > 1 << 23;
   static_assert(AD_SW % 4 == 0 && AD_H % 4 == 0 && AD_TX % 4 == 0, "vector staging");
-  for (int i = tid; i < AD_SH * (AD_SW / 4); i += 256) {
-    const int ry = i / (AD_SW / 4), rx = 4 * (i - ry * (AD_SW / 4));
-    const int gx = sx0 + rx, gy = sy0 + ry;
-    float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
-    if (gx >= 0 && gy >= 0) {
-      if (gx < W - 1 && gy < H) a = *reinterpret_cast<const float4 *>(vx + (size_t)gy * P + gx);
-      if (gx < W && gy < H - 1) b = *reinterpret_cast<const float4 *>(vy + (size_t)gy * P + gx);
-      if (gx + 3 >= W - 1) {
-        if (gx + 1 >= W - 1) a.y = 0.f;
-        if (gx + 2 >= W - 1) a.z = 0.f;
-        a.w = 0.f;
-      }
-      if (gx + 3 >= W) {
-        if (gx + 1 >= W) b.y = 0.f;
-        if (gx + 2 >= W) b.z = 0.f;
-        b.w = 0.f;
-      }
+  // a warp takes every eighth row, all its loads in flight together
+  constexpr int kRows = AD_SH / 8 + (AD_SH % 8 != 0);
+  const int lane = threadIdx.x, gx = sx0 + 4 * lane;
+  const bool col = lane < AD_SW / 4 && gx >= 0;
+  float4 a[kRows], b[kRows];
+#pragma unroll
+  for (int k = 0; k < kRows; k++) {
+    const int ry = threadIdx.y + 8 * k, gy = sy0 + ry;
+    a[k] = b[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (!col || gy < 0 || (AD_SH % 8 != 0 && ry >= AD_SH)) continue;
+    const size_t o = (size_t)gy * P + gx;
+    if (gx < W - 1 && gy < H) a[k] = *reinterpret_cast<const float4 *>(vx + o);
+    if (gx < W && gy < H - 1) b[k] = *reinterpret_cast<const float4 *>(vy + o);
+  }
+#pragma unroll
+  for (int k = 0; k < kRows; k++) {
+    const int ry = threadIdx.y + 8 * k;
+    if (gx + 3 >= W - 1) {
+      if (gx + 1 >= W - 1) a[k].y = 0.f;
+      if (gx + 2 >= W - 1) a[k].z = 0.f;
+      a[k].w = 0.f;
+      if (gx + 1 >= W) b[k].y = 0.f;
+      if (gx + 2 >= W) b[k].z = 0.f;
+      if (gx + 3 >= W) b[k].w = 0.f;
     }
     // (each value by itself: a NaN is far)
-    far |= !(fabsf(a.x) <= reach) | !(fabsf(a.y) <= reach) | !(fabsf(a.z) <= reach) |
-           !(fabsf(a.w) <= reach) | !(fabsf(b.x) <= reach) | !(fabsf(b.y) <= reach) |
-           !(fabsf(b.z) <= reach) | !(fabsf(b.w) <= reach);
-    *reinterpret_cast<float4 *>(sxv + ry * AD_SS + rx) = a;
-    *reinterpret_cast<float4 *>(syv + ry * AD_SS + rx) = b;
+    far |= !(fabsf(a[k].x) <= reach) | !(fabsf(a[k].y) <= reach) | !(fabsf(a[k].z) <= reach) |
+           !(fabsf(a[k].w) <= reach) | !(fabsf(b[k].x) <= reach) | !(fabsf(b[k].y) <= reach) |
+           !(fabsf(b[k].z) <= reach) | !(fabsf(b[k].w) <= reach);
+    if (lane < AD_SW / 4 && (AD_SH % 8 == 0 || ry < AD_SH)) {
+      *reinterpret_cast<float4 *>(sxv + ry * AD_SS + 4 * lane) = a[k];
+      *reinterpret_cast<float4 *>(syv + ry * AD_SS + 4 * lane) = b[k];
+    }
   }
   for (int i = tid; i < TY * (AD_TX / 4); i += 256) {
     const int ty = i / (AD_TX / 4), tx = 4 * (i - ty * (AD_TX / 4));
