@@ -1016,7 +1016,13 @@ void init_kernel_attributes() {
 // 64 cells, 112 x 48 stored), id 1 = 2 rows (128 x 32, 112 x 16).  The taller
 // region recomputes less; the shorter one gives a level of up to 1200 columns
 // more blocks, each with half the rows to go through per half sweep (512x256:
-// 8.5 against 10.0 us).  The autotuner tries both on every level.
+// 8.5 against 10.0 us).  The autotuner tries both on every level.  A level of
+// several members together is one launch (two, one per region, with the rule
+// above took 1442 us against 1260 for two steps of 20 members), of the shorter
+// region while it leaves SMs with fewer than two blocks (limits of 150 / 304 /
+// 608 / 1200 blocks: 1282, 1260, 1263, 1299 us; 16 served simulations 8.73,
+// 8.77, 8.84, 8.99 ms).
+constexpr int kTallBlocks = 304;
 constexpr int kTiles = 2;
 const char *const kTileNames[kTiles] = {"128x64", "128x32"};
 constexpr int kTileRows[kTiles] = {4, 2};
@@ -2061,6 +2067,12 @@ void mg_multi_vcycle(const std::vector<MgHier *> &mgs, std::vector<MultiSlot> &o
   }
   auto level_slots = [&](int l, bool pre) {
     std::map<int, MultiSlot> by_tile;
+    // one region for all members, so one launch
+    int blocks = 0;
+    for (auto *m : mgs)
+      if (l < m->tail_top)
+        blocks += tile::regions(m->lv[l].w, 128) * tile::regions(m->lv[l].h, 32);
+    const int common = blocks >= kTallBlocks ? 0 : 1;
     for (int i = 0; i < n; i++) {
       MgHier &mg = *mgs[i];
       if (l >= mg.tail_top) continue;
@@ -2081,7 +2093,8 @@ void mg_multi_vcycle(const std::vector<MgHier *> &mgs, std::vector<MultiSlot> &o
         a.ch = C.h;
       }
       a.zero_edges = l > 0;
-      const int id = tile_for(L.w, pre ? L.tile_pre : L.tile_post);
+      const int choice = pre ? L.tile_pre : L.tile_post;
+      const int id = choice < 0 ? common : tile_for(L.w, choice);
       MultiSlot &sl = by_tile[id];
       sl.kind = MK_MG;
       sl.tile = 2 * id + (pre ? 0 : 1);
