@@ -28,8 +28,11 @@ namespace {
 namespace coarse {
 
 constexpr int kMaxLevels = 12;
-constexpr int kWarps = 16;
-constexpr int kItems = 4, kMaxGroups = kItems * 32 * kWarps;  // groups of four cells, all levels
+// Warps of the block: the tolerance hierarchy's levels of 2^n + 1 columns and
+// rows (65x33) take one group of rows more.
+constexpr int warps_for(bool ext) { return ext ? 20 : 16; }
+constexpr int kWarps = warps_for(true);
+constexpr int kItems = 4, kMaxGroups = kItems * 32 * warps_for(false);  // groups of four cells, all levels
 
 struct Level {
   int w, h, lsh, warps;   // lanes per row 1 << lsh; warps that hold its rows
@@ -55,7 +58,7 @@ inline int warps_of(int w, int h) {
   const int rows = 2 * (32 >> lane_shift(w));
   return (h + rows - 1) / rows;
 }
-inline bool fits(int w, int h) { return w <= 128 && warps_of(w, h) <= kWarps; }
+inline bool fits(int w, int h, bool ext) { return w <= 128 && warps_of(w, h) <= warps_for(ext); }
 // Shared memory before the levels: arguments (indexed by level, which in the
 // parameter space would be a load from memory each time), exchanged rows of
 // the warps and of one below and one above (zeros), restriction rows, table.
@@ -425,6 +428,7 @@ __device__ __forceinline__ void init(const Args<S> &args, unsigned char *smem) {
 template <class S, bool EXT>
 __device__ __forceinline__ void run(unsigned char *smem) {
   using St = Sto<S>;
+  constexpr int NT = 32 * warps_for(EXT);
   const Args<S> &a = *reinterpret_cast<const Args<S> *>(smem + kArgs);
   // Codes of every level, the top level's right-hand side (columns past the
   // width: 0).  The levels' groups of four cells are numbered through, at
@@ -435,7 +439,7 @@ __device__ __forceinline__ void run(unsigned char *smem) {
   int left[kItems];
 #pragma unroll
   for (int k = 0; k < kItems; k++) {
-    left[k] = threadIdx.x + 32 * kWarps * k;
+    left[k] = threadIdx.x + NT * k;
     src[k] = nullptr;
     mask[k] = dst[k] = c[k] = 0u;
   }
@@ -460,14 +464,14 @@ __device__ __forceinline__ void run(unsigned char *smem) {
 #pragma unroll
   for (int k = 0; k < kItems; k++) {
     if (src[k]) c[k] = __ldg(reinterpret_cast<const unsigned *>(src[k])) & mask[k];
-    const int i = threadIdx.x + 32 * kWarps * k, X = 4 * (i & n1);
+    const int i = threadIdx.x + NT * k, X = 4 * (i & n1);
     fv[k] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (i < nt && X < T.w) fv[k] = St::ldg4(a.rhs_top + (size_t)(i >> T.lsh) * a.rhs_pitch + X);
   }
 #pragma unroll
   for (int k = 0; k < kItems; k++) {
     if (dst[k]) *reinterpret_cast<unsigned *>(smem + dst[k]) = c[k];
-    const int i = threadIdx.x + 32 * kWarps * k;
+    const int i = threadIdx.x + NT * k;
     if (i < nt) *reinterpret_cast<float4 *>(smem + T.of + 16 * i) = fv[k];
   }
   __syncthreads();

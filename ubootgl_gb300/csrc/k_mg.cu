@@ -308,7 +308,7 @@ __global__ void __launch_bounds__(32 * NW, 1024 / (32 * NW))
 }
 
 template <class S, bool EXT>
-__global__ void __launch_bounds__(32 * coarse::kWarps, 1)
+__global__ void __launch_bounds__(32 * coarse::warps_for(EXT), 1)
     k_coarse(const __grid_constant__ coarse::Args<S> a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   tile::fill_lut(reinterpret_cast<float2 *>(smem_raw + coarse::kLut), threadIdx.x, a.wsum, a.rwsum);
@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(32 * coarse::kWarps, 1)
   coarse::run<S, EXT>(smem_raw);
 }
 // One block per member of a batch (FP32).
-__global__ void __launch_bounds__(32 * coarse::kWarps, 1)
+__global__ void __launch_bounds__(32 * coarse::warps_for(false), 1)
     k_coarse_m(const coarse::Args<float> *__restrict__ A, const int *__restrict__ bs, int n,
                unsigned tag, unsigned *err) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1216,17 +1216,17 @@ coarse::Args<S> coarse_args(MgHier &mg, int lt, const S *rhs_top, S *e_top, cons
 }
 
 template <class S>
-void run_coarse(MgHier &mg, int lt, const S *rhs_top, S *e_top, const float *rfac,
+void run_coarse(MgHier &mg, int lt, bool wide, const S *rhs_top, S *e_top, const float *rfac,
                 cudaStream_t st) {
-  if (mg.tail_wide) {
+  if (wide) {
     run_tail_t<S, float>(mg, lt, rhs_top, e_top, rfac, st);
     return;
   }
   ProfScope ps_(KC_TAIL, st);
   size_t smem = 0;
   const coarse::Args<S> a = coarse_args<S>(mg, lt, rhs_top, e_top, rfac, &smem);
-  launch_pdl(a.ext ? k_coarse<S, true> : k_coarse<S, false>, dim3(1), dim3(32 * coarse::kWarps),
-             smem, st, a);
+  launch_pdl(a.ext ? k_coarse<S, true> : k_coarse<S, false>, dim3(1),
+             dim3(32 * coarse::warps_for(mg.ext)), smem, st, a);
   UBG_LAUNCH_CHECK();
   g_stats.launches++;
 }
@@ -1236,7 +1236,7 @@ void solve_level(MgHier &mg, std::vector<int> &cur, int l, bool zgbc, cudaStream
   bool bc = zgbc && l == 0;
   MgLevel &L = mg.lv[l];
   if (l >= 1 && l == mg.tail_top) {
-    run_coarse<float>(mg, l, L.rhs, L.e[0], nullptr, st);
+    run_coarse<float>(mg, l, mg.tail_wide, L.rhs, L.e[0], nullptr, st);
     cur[l] = 0;
     return;
   }
@@ -1632,19 +1632,26 @@ int choose_tail_any(const std::vector<MgLevel> &lv, int max_cells, size_t elem_b
 }
 // The first level from which the one-block coarse solve covers the rest, with
 // a top level of at most max_cells.
-int choose_tail(const std::vector<MgLevel> &lv, int max_cells, int last) {
+int choose_tail(const std::vector<MgLevel> &lv, int max_cells, int last, bool ext) {
   for (int lt = 1; lt <= last; lt++)
-    if (coarse::fits(lv[lt].w, lv[lt].h) && last - lt < coarse::kMaxLevels &&
+    if (coarse::fits(lv[lt].w, lv[lt].h, ext) && last - lt < coarse::kMaxLevels &&
         (size_t)lv[lt].w * lv[lt].h <= (size_t)max_cells)
       return lt;
   return -1;
 }
 // Sets the hierarchy's tail: the coarse solve in registers, or the kernel of
-// any shape for elongated levels of at most wide_cells.
+// any shape for elongated levels of at most wide_cells.  With 16-bit levels it
+// is always the first level of at most wide_cells, whatever its shape: a level
+// above the tail is rounded to 16 bits in every half sweep, one in it is not.
 void set_tail(MgHier &mg, int last, int wide_cells) {
-  mg.tail_top = choose_tail(mg.lv, mg.tail_cells, last);
+  const int any = choose_tail_any(mg.lv, wide_cells, 4, last);
+  const bool fits = any >= 1 && coarse::fits(mg.lv[any].w, mg.lv[any].h, mg.ext) &&
+                    last - any < coarse::kMaxLevels;
+  mg.tail_top = fits ? any : choose_tail(mg.lv, mg.tail_cells, last, mg.ext);
   mg.tail_wide = mg.tail_top < 1;
-  if (mg.tail_wide) mg.tail_top = choose_tail_any(mg.lv, wide_cells, 4, last);
+  if (mg.tail_wide) mg.tail_top = any;
+  mg.tail_top16 = any;
+  mg.tail_wide16 = !fits;
 }
 
 }  // namespace
@@ -1905,7 +1912,7 @@ void mg_autotune(MgHier &mg, cudaStream_t st, std::string *report) {
   const int tail_cand[] = {512, 2048, 4096};
   int best_tc = mg.tail_cells, best_lt = mg.tail_top;
   for (int tc : tail_cand) {
-    int lt = mg.tail_wide ? -1 : choose_tail(mg.lv, tc, nl - 2);
+    int lt = mg.tail_wide ? -1 : choose_tail(mg.lv, tc, nl - 2, mg.ext);
     if (lt < 1 || lt == best_lt) continue;
     int keep = mg.tail_top;
     mg.tail_top = lt;
@@ -2138,7 +2145,7 @@ void launch_multi_mg(const MultiSlot &slot, const void *dargs, const int *dbs, u
     launch_pdl(k_mg_tail_m, dim3(slot.n), dim3(32, 32), slot.smem, st,
                (const TailArgs<float> *)dargs, dbs, slot.n, tag, err);
   } else if (slot.kind == MK_TAIL) {
-    launch_pdl(k_coarse_m, dim3(slot.n), dim3(32 * coarse::kWarps), slot.smem, st,
+    launch_pdl(k_coarse_m, dim3(slot.n), dim3(32 * coarse::warps_for(false)), slot.smem, st,
                (const coarse::Args<float> *)dargs, dbs, slot.n, tag, err);
   } else {
     const MgArgs *A = (const MgArgs *)dargs;
@@ -2289,7 +2296,7 @@ MgArgsT<SC> ext_level_args(MgHier &mg, MgLow *lo, int l, int cin, int ns) {
 template <class SC>
 void ext_vcycle_t(MgHier &mg, MgLow *lo, const unsigned *scale_bits, cudaStream_t st) {
   constexpr bool scaled = !std::is_same<SC, float>::value;
-  const int T = mg.tail_top;
+  const int T = scaled ? mg.tail_top16 : mg.tail_top;
   if (T < 1) throw ArgError("tolerance hierarchy without a coarse tail");
   auto arr = [&](int l, int c) -> SC * {
     return scaled ? (SC *)lo->e[c][l] : (SC *)mg.lv[l].e[c];
@@ -2360,7 +2367,8 @@ void ext_vcycle_t(MgHier &mg, MgLow *lo, const unsigned *scale_bits, cudaStream_
   }
   {
     std::vector<float> rf(mg.levels, 0.25f);
-    run_coarse<SC>(mg, T, rhs(T), arr(T, 0), scaled ? rf.data() : nullptr, st);
+    run_coarse<SC>(mg, T, scaled ? mg.tail_wide16 : mg.tail_wide, rhs(T), arr(T, 0),
+                   scaled ? rf.data() : nullptr, st);
     cur[T] = 0;
   }
   // up
@@ -2427,7 +2435,7 @@ void ext_hier_alloc(MgHier &mg, int W, int H, float h0) {
   mg.lv = lv;
   mg.levels = (int)lv.size();
   set_tail(mg, mg.levels - 1, 4096);
-  if (mg.tail_top < 1) mg.tail_top = mg.levels - 1;
+  if (mg.tail_top < 1) mg.tail_top = mg.tail_top16 = mg.levels - 1;
   mg.tail_top_fp64 = -1;
   mg.arena = arena;
   mg.arena_bytes = total;

@@ -348,6 +348,8 @@ struct MgHier {
   int cur0 = 0;                  // which e[] of level 0 holds p
   int tail_top = -1;             // first level solved by the one-CTA tail kernel
   bool tail_wide = false;        // elongated levels: the tail kernel of any shape
+  int tail_top16 = -1;           // the same two with 16-bit levels (set_tail)
+  bool tail_wide16 = false;
   int tail_cells = 2048;         // largest top level the tail takes (autotuned)
   int tail_top_fp64 = -1;        // the same for the mixed solver's FP64 tail
   void *arena = nullptr;
