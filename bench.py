@@ -640,9 +640,9 @@ ALG_BYTES_PER_CELL = {
 
 
 def profiled_traffic(W, H):
-    """DRAM bytes (read + write) per level-0 k_mg launch from the committed
+    """DRAM bytes (read + write) per level-0 k_tile launch from the committed
     ncu summary of this workload, or None if there is none for this size."""
-    fn = os.path.join(ROOT, "profiles", "k_mg_level0_%dx%d.txt" % (W, H))
+    fn = os.path.join(ROOT, "profiles", "k_tile_level0_%dx%d.txt" % (W, H))
     try:
         for line in open(fn):
             if line.startswith("dram_bytes_per_launch:"):
@@ -785,9 +785,9 @@ def kernel_timing(sim, lib, W, H, reps=30):
     compulsory = 13.0 * cells
     achieved = alg / (ms_l / 1e3) / 1e9
     ach_c = compulsory / (ms_l / 1e3) / 1e9
-    roof = {"bound": "hbm", "kernel": "k_mg level 0 (3 red-black sweeps per launch, temporally "
-                                      "blocked in shared memory, with the residual + restriction "
-                                      "or the prolongation + correction of the level)",
+    roof = {"bound": "hbm", "kernel": "k_tile level 0 (3 red-black sweeps per launch on regions "
+                                      "in registers, with the residual + restriction or the "
+                                      "prolongation + correction of the level)",
             "alg_bytes_per_cell": ALG_BYTES_PER_CELL[dom],
             "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
             "frac": round(achieved / peak, 3), "peak_source": peak_src,

@@ -234,9 +234,9 @@ int ubg_restore(ubg_sim *sim, const void *src);
 
 /* ------------------------------------------- autotuner and batches */
 
-/* Autotuner (extension): times the candidate smoother tiles of every
+/* Autotuner (extension): times the candidate smoother regions of every
  * multigrid level (pre- and post-smoothing launches separately) and the
- * sizes of the one-CTA coarse tail on this simulation's own arrays, and
+ * sizes of the one-block coarse end on this simulation's own arrays, and
  * keeps the fastest.  The simulation's state is unchanged and results are
  * bit-identical for every choice.  report (may be NULL) receives a JSON
  * object with the per-level choices and times (truncated to len). */
@@ -247,7 +247,7 @@ int ubg_autotune(ubg_sim *sim, char *report, size_t len);
  * the FP32 fixed-mode members of at most 2^20 cells (at least two of them)
  * are fused: each kernel of the step is one launch over all of them (blocks
  * mapped to members through prefix sums, per-member arguments in a device
- * table), ~40 launches whatever their count.  The other members' own step
+ * table), 16 to 28 launches whatever their count.  The other members' own step
  * bodies run as parallel branches of the same graph.  dts: n host time
  * steps (every member then a branch), or NULL for dt = cfl * h / max|u| per
  * member on the device.  Members keep their own fields, options and

@@ -20,7 +20,10 @@
 // 32 lanes per row, all 32 warps and a block barrier per half sweep, 128x64 and
 // down took 32 us: small levels waited for barriers of idle warps.  128x64 in
 // the block instead of two smoothing launches (5 us each in a step): 43
-// against 35 us per V-cycle of 256x128, hence the limit of 2048 cells.
+// against 35 us per V-cycle of 256x128, hence the limit of 2048 cells.  The
+// tolerance hierarchy's 65x33 in the block (17 warps) instead of two launches:
+// 885 -> 871 us per step at 1024x512.  Its edge cells in registers: 374 -> 200
+// cycles per half sweep of one warp.
 #pragma once
 
 namespace ubg {

@@ -9,7 +9,8 @@
 //              restrict, pressure_solver.cpp:91-132), with the zero-gradient
 //              boundary (setZeroGradientBC, pressure_solver.cpp:183-192).
 //  k_coarse    (k_coarse.cuh) the coarse end of the V-cycle in one block, from
-//              a level of at most 128 x 64 cells down.
+//              a level of at most 2048 cells down (4096 where it can hold it, in
+//              the tolerance hierarchy).
 //  k_mg        up to 5 sweeps temporally blocked in shared memory: the
 //              coarsest level of a hierarchy without a tail, and one sweep
 //              with any alpha (the free function rbgs).

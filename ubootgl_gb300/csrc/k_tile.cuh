@@ -21,9 +21,11 @@
 // What bounds it: instruction issue and the FP32 pipe on large levels, the
 // latency of loads, six barriers and one pass through the code on small ones.
 // Against tiles in shared memory (red/black-split, 112 x 50 and 48 x 16
-// cells), ncu: level 0 of 4096x2048 52-55 us (89 with the residual, 98 with
-// the prolongation), 2048x1024 17 us (33, 38), 1024x512 8 us (18, 20), 256x128
-// 6 us.  Of the gain, bounds checks outside the blocks that need them, the
+// cells), ncu: level 0 of 4096x2048 53 us (89) with the residual, 51 (98) with
+// the prolongation, 2048x1024 17 us (33, 38), 1024x512 8 us (18, 20), 256x128
+// 7 us.  Edge cells in the registers instead of neighbours rebuilt from codes
+// and positions: 5900 -> 2260 cycles for an edge warp's six half sweeps (2000 for
+// others), 83 -> 78 us per step of 256x128.  Bounds checks outside the blocks that need them, the
 // packed magnitude check and W + E as scalar additions (no register moves)
 // are 2 us (32.4 -> 25.5 M warp instructions), f kept in shared memory for
 // the residual and one factor per cell another 2 (4096x2048 steps 660 ->
@@ -195,8 +197,9 @@ __device__ __forceinline__ void residual4(unsigned c, const float (&C)[4], const
   }
 }
 
-// One region of the level: columns from 112 * sx, rows from (NW * R - 16) * sy.  PRE: residual and restriction (a.rc); else prolongation and
-// correction (a.ec) first.  Red points are those with x + y odd; even rows
+// One region of the level: columns from 112 * sx, rows from (NW * R - 16) * sy.
+// PRE: residual and restriction (a.rc); else prolongation and correction (a.ec)
+// first.  Red points are those with x + y odd; even rows
 // hold them in the pair (1, 3).
 template <class S, class SC, bool EXT, bool PRE, int R, int NW>
 __device__ __forceinline__ void run(const MgArgsT<S, SC> &a, const int region,
