@@ -24,13 +24,13 @@
 // cells), ncu: level 0 of 4096x2048 53 us (89) with the residual, 51 (98) with
 // the prolongation, 2048x1024 17 us (33, 38), 1024x512 8 us (18, 20), 256x128
 // 7 us.  Edge cells in the registers instead of neighbours rebuilt from codes
-// and positions: 5900 -> 2260 cycles for an edge warp's six half sweeps (2000 for
-// others), 83 -> 78 us per step of 256x128.  Bounds checks outside the blocks that need them, the
-// packed magnitude check and W + E as scalar additions (no register moves)
-// are 2 us (32.4 -> 25.5 M warp instructions), f kept in shared memory for
-// the residual and one factor per cell another 2 (4096x2048 steps 660 ->
-// 647 us).  Regions of 8 rows per warp (8 warps), and of 128 x 32 cells, are
-// slower there (58-60, 65 us).
+// and positions: 5900 -> 2260 cycles for an edge warp's six half sweeps (2000
+// for others), 83 -> 78 us per step of 256x128.  Bounds checks outside the
+// blocks that need them, the packed magnitude check and W + E as scalar
+// additions (no register moves) were 2 us (32.4 -> 25.5 M warp instructions), f
+// kept in shared memory for the residual and one factor per cell another 2
+// (4096x2048 steps 660 -> 647 us).  Regions of 8 rows per warp (8 warps), and of
+// 128 x 32 cells, are slower there (58-60, 65 us).
 #pragma once
 
 namespace ubg {
