@@ -35,7 +35,9 @@ constexpr int kMaxLevels = 12;
 // rows (65x33) take one group of rows more.
 constexpr int warps_for(bool ext) { return ext ? 20 : 16; }
 constexpr int kWarps = warps_for(true);
-constexpr int kItems = 4, kMaxGroups = kItems * 32 * warps_for(false);  // groups of four cells, all levels
+// Groups of four cells of all levels that a thread loads at most, and the block.
+constexpr int kItems = 4;
+constexpr int max_groups(bool ext) { return kItems * 32 * warps_for(ext); }
 
 struct Level {
   int w, h, lsh, warps;   // lanes per row 1 << lsh; warps that hold its rows
@@ -61,7 +63,10 @@ inline int warps_of(int w, int h) {
   const int rows = 2 * (32 >> lane_shift(w));
   return (h + rows - 1) / rows;
 }
-inline bool fits(int w, int h, bool ext) { return w <= 128 && warps_of(w, h) <= warps_for(ext); }
+// Groups of four cells of a level, and its bytes: e and rhs (16 per group) and
+// codes (4), the next level's on a 16-byte boundary.
+inline size_t groups_of(int w, int h) { return (size_t)h << lane_shift(w); }
+inline size_t bytes_of(int w, int h) { return (36 * groups_of(w, h) + 15) / 16 * 16; }
 // Shared memory before the levels: arguments (indexed by level, which in the
 // parameter space would be a load from memory each time), exchanged rows of
 // the warps and of one below and one above (zeros), restriction rows, table.
@@ -435,8 +440,9 @@ __device__ __forceinline__ void run(unsigned char *smem) {
   const Args<S> &a = *reinterpret_cast<const Args<S> *>(smem + kArgs);
   // Codes of every level, the top level's right-hand side (columns past the
   // width: 0).  The levels' groups of four cells are numbered through, at
-  // most kItems per thread (128 x 32 cells, or 16 x 256, and the levels below:
-  // fewer than 2048 groups), and all their loads are in flight together.
+  // most kItems per thread (max_groups: 16 x 256 cells and the levels below are
+  // 1792 groups of the reference's hierarchy's 2048, 14 x 292 cells 2052 of the
+  // tolerance hierarchy's 2560), and all their loads are in flight together.
   const uint8_t *src[kItems];
   unsigned mask[kItems], dst[kItems], c[kItems];
   int left[kItems];

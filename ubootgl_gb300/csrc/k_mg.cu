@@ -1171,6 +1171,21 @@ void run_tail_t(MgHier &mg, int lt, const S *rhs_top, S *e_top, const float *rfa
   g_stats.launches++;
 }
 
+// Whether the one-block coarse solve holds levels lt .. last: the top level's
+// rows in the block's warps (every lower level has fewer), all levels' cells in
+// its loads and in shared memory.
+bool coarse_holds(const std::vector<MgLevel> &lv, int lt, int last, bool ext) {
+  if (lv[lt].w > 128 || coarse::warps_of(lv[lt].w, lv[lt].h) > coarse::warps_for(ext) ||
+      last - lt >= coarse::kMaxLevels)
+    return false;
+  size_t groups = 0, bytes = coarse::kLevels;
+  for (int l = lt; l <= last; l++) {
+    groups += coarse::groups_of(lv[l].w, lv[l].h);
+    bytes += coarse::bytes_of(lv[l].w, lv[l].h);
+  }
+  return groups <= (size_t)coarse::max_groups(ext) && bytes <= kCoarseSmemMax;
+}
+
 // Arguments of the coarse end of the V-cycle from level lt on (scaled: the
 // h^2-scaled form of 16-bit levels, hh = 1 and restriction weights rfac).
 template <class S>
@@ -1181,7 +1196,9 @@ coarse::Args<S> coarse_args(MgHier &mg, int lt, const S *rhs_top, S *e_top, cons
   a.nlev = nl;
   a.ext = mg.ext ? 1 : 0;
   a.ncoarse = mg.ncoarse;
-  size_t off = coarse::kLevels, groups = 0;
+  size_t off = coarse::kLevels;
+  if (!coarse_holds(mg.lv, lt, mg_coarsest(mg), mg.ext))
+    throw ArgError("coarse levels exceed one block");
   for (int t = 0; t < nl; t++) {
     MgLevel &L = mg.lv[lt + t];
     coarse::Level &C = a.L[t];
@@ -1192,17 +1209,14 @@ coarse::Args<S> coarse_args(MgHier &mg, int lt, const S *rhs_top, S *e_top, cons
     C.hh = rfac ? 1.0f : L.hh;
     C.ihsq = rfac ? 1.0f : 1.0f / L.hh / L.hh;
     C.rfac = rfac ? rfac[lt + t] : 1.0f / 16.0f;
-    const size_t n = (size_t)C.h << C.lsh;
-    groups += n;
+    const size_t n = coarse::groups_of(L.w, L.h);
     C.oe = (int)off;
     C.of = (int)(off + 16 * n);
     C.oc = (int)(off + 32 * n);
-    off = (off + 36 * n + 15) / 16 * 16;
+    off += coarse::bytes_of(L.w, L.h);
     C.code = L.code;
     C.code_pitch = L.pitch;
   }
-  if (off > kCoarseSmemMax || groups > coarse::kMaxGroups)
-    throw ArgError("coarse levels exceed one block");
   MgLevel &top = mg.lv[lt];
   a.rhs_top = rhs_top;
   a.rhs_pitch = top.pitch;
@@ -1635,8 +1649,7 @@ int choose_tail_any(const std::vector<MgLevel> &lv, int max_cells, size_t elem_b
 // a top level of at most max_cells.
 int choose_tail(const std::vector<MgLevel> &lv, int max_cells, int last, bool ext) {
   for (int lt = 1; lt <= last; lt++)
-    if (coarse::fits(lv[lt].w, lv[lt].h, ext) && last - lt < coarse::kMaxLevels &&
-        (size_t)lv[lt].w * lv[lt].h <= (size_t)max_cells)
+    if (coarse_holds(lv, lt, last, ext) && (size_t)lv[lt].w * lv[lt].h <= (size_t)max_cells)
       return lt;
   return -1;
 }
@@ -1646,8 +1659,7 @@ int choose_tail(const std::vector<MgLevel> &lv, int max_cells, int last, bool ex
 // above the tail is rounded to 16 bits in every half sweep, one in it is not.
 void set_tail(MgHier &mg, int last, int wide_cells) {
   const int any = choose_tail_any(mg.lv, wide_cells, 4, last);
-  const bool fits = any >= 1 && coarse::fits(mg.lv[any].w, mg.lv[any].h, mg.ext) &&
-                    last - any < coarse::kMaxLevels;
+  const bool fits = any >= 1 && coarse_holds(mg.lv, any, last, mg.ext);
   mg.tail_top = fits ? any : choose_tail(mg.lv, mg.tail_cells, last, mg.ext);
   mg.tail_wide = mg.tail_top < 1;
   if (mg.tail_wide) mg.tail_top = any;
