@@ -349,10 +349,12 @@ struct ubg_sim {
       fx ^= 1;
       fy ^= 1;
     }
-    launch_advect(v, fx, fy, d_sc, st, true, bc, d_umax);
+    // (the tolerance solver may throw, which leaves max|u| as it was)
+    const bool tol = opt.solver_mode == UBG_SOLVE_TOLERANCE;
+    launch_advect(v, fx, fy, d_sc, st, true, bc, tol ? nullptr : d_umax);
     fx ^= 1;
     fy ^= 1;
-    if (opt.solver_mode == UBG_SOLVE_TOLERANCE) {
+    if (tol) {
       project(nsink_cells);
       launch_vbc(v, fx, fy, bc, true, true, st, d_umax);
       return;
