@@ -272,6 +272,12 @@ int ubg_sim_device_bytes(ubg_sim *sim, size_t *bytes);
  * This compares the two bit for bit on the device for the n host values x
  * and writes the number of differences (0 expected). */
 int ubg_selftest_div(const float *x, int n, float d, unsigned *mismatches);
+/* Diagnostic: one preconditioning V-cycle of the tolerance solver, z = M r,
+ * on host arrays (flag as in ubg_create, r and z width x height, spacing h).
+ * precision: UBG_FP32, UBG_MIXED_FP16 or UBG_MIXED_BF16 coarse levels; rmax: the
+ * largest |r|, which sets the scale of 16-bit ones. */
+int ubg_selftest_vcycle(const float *flag, const float *r, int width, int height, float h,
+                        int precision, float rmax, float *z);
 
 /* ------------------------------------------------------------ step server */
 

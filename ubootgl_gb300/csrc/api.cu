@@ -2156,3 +2156,17 @@ int ubg_selftest_div(const float *x, int n, float d, unsigned *mismatches) {
     return UBG_OK;
   });
 }
+
+int ubg_selftest_vcycle(const float *flag, const float *r, int width, int height, float h,
+                        int precision, float rmax, float *z) {
+  return guarded([&] {
+    if (!flag || !r || !z || width < 8 || height < 8 || !(h > 0.0f) || !(rmax >= 0.0f))
+      throw ArgError("bad argument");
+    if (precision < UBG_FP32 || precision > UBG_MIXED_BF16) throw ArgError("unknown precision mode");
+    check_device();
+    std::vector<uint8_t> u8;
+    flag_to_u8(flag, width, height, u8, round_up(width, 32));
+    selftest_vcycle(u8.data(), r, width, height, h, precision, rmax, z);
+    return UBG_OK;
+  });
+}

@@ -2480,4 +2480,37 @@ void ext_vcycle(MgHier &mg, MgLow *lo, int prec, const unsigned *scale_bits, cud
     throw ArgError("precision");
 }
 
+void selftest_vcycle(const uint8_t *flag, const float *r, int W, int H, float h, int prec,
+                     float rmax, float *z) {
+  // freed on every path, including a failing CUDA call
+  struct Held {
+    MgHier mg;
+    MgLow lo;
+    cudaStream_t st = nullptr;
+    void *dev = nullptr;
+    ~Held() {
+      if (st) cudaStreamSynchronize(st);
+      mg_low_free(lo);
+      mg_free(mg);
+      if (dev) cudaFree(dev);
+      if (st) cudaStreamDestroy(st);
+    }
+  } a;
+  ext_hier_alloc(a.mg, W, H, h);
+  if (prec != UBG_FP32) mg_low_alloc(a.lo, a.mg, prec);
+  UBG_CUDA(cudaStreamCreateWithFlags(&a.st, cudaStreamNonBlocking));
+  const int P = a.mg.lv[0].pitch;
+  const size_t row = (size_t)W * 4, pitch = (size_t)P * 4, nflag = (size_t)P * H;
+  UBG_CUDA(cudaMalloc(&a.dev, align256(nflag) + sizeof(rmax)));
+  unsigned *bits = (unsigned *)((char *)a.dev + align256(nflag));
+  UBG_CUDA(cudaMemcpyAsync(a.dev, flag, nflag, cudaMemcpyHostToDevice, a.st));
+  UBG_CUDA(cudaMemcpyAsync(bits, &rmax, sizeof(rmax), cudaMemcpyHostToDevice, a.st));
+  ext_hier_update_fields(a.mg, (const uint8_t *)a.dev, P, a.st);
+  UBG_CUDA(cudaMemcpy2DAsync(a.mg.lv[0].rhs, pitch, r, row, row, H, cudaMemcpyHostToDevice, a.st));
+  ext_vcycle(a.mg, prec == UBG_FP32 ? nullptr : &a.lo, prec, bits, a.st);
+  UBG_CUDA(cudaMemcpy2DAsync(z, row, a.mg.lv[0].e[a.mg.cur0], pitch, row, H,
+                             cudaMemcpyDeviceToHost, a.st));
+  UBG_CUDA(cudaStreamSynchronize(a.st));
+}
+
 }  // namespace ubg

@@ -456,6 +456,10 @@ void ext_hier_alloc(MgHier &mg, int W, int H, float h0);
 // Level-0 flag from flag0 (pitch0 bytes per row), coarse flags, codes.
 void ext_hier_update_fields(MgHier &mg, const uint8_t *flag0, int pitch0, cudaStream_t st);
 void ext_vcycle(MgHier &mg, MgLow *lo, int prec, const unsigned *scale_bits, cudaStream_t st);
+// One ext_vcycle on host arrays (flag: rows of round_up(W, 32) bytes), rmax in
+// the place of max|r|.
+void selftest_vcycle(const uint8_t *flag, const float *r, int W, int H, float h, int prec,
+                     float rmax, float *z);
 
 // Device scalars of the flexible CG loop (k_krylov.cu).
 struct FcgScalars {
