@@ -62,3 +62,10 @@ def check(lib, W, H, precision, less=1.0):
 @pytest.mark.parametrize("W,H", SIZES)
 def test_bit_exact(lib, W, H, precision):
     check(lib, W, H, precision)
+
+
+@pytest.mark.parametrize("W,H,less", [(1300, 209, 17), (500, 131, 16), (257, 225, 15)])
+def test_overflow_in_the_sweeps(lib, W, H, less):
+    """A scale 2^less too large: FP16 values overflow, some within the sweeps
+    of a region that starts with finite ones; solid cells stay 0."""
+    check(lib, W, H, "fp16", 2.0 ** -less)

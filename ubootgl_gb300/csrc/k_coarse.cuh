@@ -288,7 +288,7 @@ __device__ __forceinline__ void visit(const Args<S> &a, const int t, const bool 
   }
   // sums that may not stay finite (false for infinities and NaNs too): a warp
   // alone decides for itself, several agree through shared memory
-  bool careful = __any_sync(0xffffffffu, !(sq.x + sq.y < tile::kBigSq)) != 0;
+  bool careful = __any_sync(0xffffffffu, !(sq.x + sq.y < tile::kBigSq<float>)) != 0;
   const bool multi = pl.warps > 1;
   if (multi) {
     const bool init = EXT && up;

@@ -111,9 +111,17 @@ __device__ __forceinline__ float scaled_any(float v, float s) {
   const float n = (s == kThird && fabsf(v) < __int_as_float(0x7f800000)) ? q3 : q;
   return s != 0.0f ? n : 0.0f;
 }
-// Bound of the sum of squares of what a lane holds under which six (ten)
-// half sweeps stay finite.
-constexpr float kBigSq = 0x1p+120f;
+// Bound of the sum of squares of what a lane holds, p and kWeightF f h^2, under
+// which the sweeps stay finite.  A half sweep gives at most the largest p plus
+// the largest f h^2, rounded to S: in FP32 and BF16 values below 2^60 stay below
+// 2^66 over the 32 half sweeps of the tolerance hierarchy's coarsest level; in
+// FP16 p < 2^15 and f h^2 < 2^12 stay below 57600 over a launch's six, of 65504.
+template <class S>
+constexpr bool kIsHalf = std::is_same<S, __half>::value;
+template <class S>
+constexpr float kBigSq = kIsHalf<S> ? 0x1p+30f : 0x1p+120f;
+template <class S>
+constexpr float kWeightF = kIsHalf<S> ? 8.0f : 1.0f;
 
 // Fills the table: factors by code, 32 + flag for a cell on the domain's
 // edge; then the weight sums of the prolongation and their reciprocals.
@@ -364,7 +372,7 @@ __device__ __forceinline__ void run(const MgArgsT<S, SC> &a, const int region,
       cB[KEEP ? R : 1];
   const float hh = a.hh;
   copy_wait();
-  float2 sq = make_float2(0.f, 0.f);  // sums of squares of p and f h^2
+  float2 sq = make_float2(0.f, 0.f);  // sums of squares of p and (weighted) f h^2
 #pragma unroll
   for (int r = 0; r < R; r++) {
     float *p = &pv[r].x;
@@ -396,7 +404,9 @@ __device__ __forceinline__ void run(const MgArgsT<S, SC> &a, const int region,
     B[r] = make_float2(p[1], p[3]);
     FA[r] = make_float2(F[0], F[2]);
     FB[r] = make_float2(F[1], F[3]);
-    sq = f2_fma(FB[r], FB[r], f2_fma(FA[r], FA[r], f2_fma(B[r], B[r], f2_fma(A[r], A[r], sq))));
+    const float2 ga = kIsHalf<S> ? f2_mul(FA[r], f2(kWeightF<S>)) : FA[r],
+                 gb = kIsHalf<S> ? f2_mul(FB[r], f2(kWeightF<S>)) : FB[r];
+    sq = f2_fma(gb, gb, f2_fma(ga, ga, f2_fma(B[r], B[r], f2_fma(A[r], A[r], sq))));
   }
   if (!PRE && wedge && zg) {  // edge cells: their inner neighbours' values
     auto flag = [&](unsigned c, int b, float v) { return (c >> (8 * b)) & C_CENTER ? v : 0.0f; };
@@ -430,7 +440,7 @@ __device__ __forceinline__ void run(const MgArgsT<S, SC> &a, const int region,
     slot(0, -1, 1) = slot(1, -1, 1) = slot(0, NW, 0) = slot(1, NW, 0) = res[0] =
         make_float2(0.f, 0.f);
   // false for infinities and NaNs too
-  const bool careful = __syncthreads_or(!(sq.x + sq.y < kBigSq)) != 0;
+  const bool careful = __syncthreads_or(!(sq.x + sq.y < kBigSq<S>)) != 0;
   // the block's barrier from any of the variants below
   auto sync = [] { asm volatile("bar.sync 1, %0;" ::"n"(32 * NW) : "memory"); };
 
