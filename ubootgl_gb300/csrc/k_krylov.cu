@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(BX *BY) k_fcg_fsum(const float *__restrict__ f
   float s = 0.0f;
   int ne = 0, nf = 0;
   // grid-stride over tiles of 128 x 8 cells: a few blocks per SM, so few
-  // same-address atomics in the final reduction
+  // partial sums to combine
   const int tiles_x = (W + 4 * BX - 1) / (4 * BX), ntiles = tiles_x * ((H + BY - 1) / BY);
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const int x4 = ((t % tiles_x) * BX + threadIdx.x) * 4, y = (t / tiles_x) * BY + threadIdx.y;
@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(BX *BY) k_fcg_fsum(const float *__restrict__ f
 // r = f_c + ihsq * sum_n flag_n (x_n - x) on the interior fluid cells (0
 // elsewhere), the neighbour differences in double-float; neighbours on the
 // domain edge are zero-gradient copies (difference 0).  Writes r and
-// accumulates ||r||^2 and max|r|, and with want_ff also ||f_c||^2.
+// gives ||r||^2 and max|r|, and with want_ff also ||f_c||^2.
 __global__ void __launch_bounds__(BX *BY) k_fcg_resid(const float *__restrict__ xh,
                                                       const float *__restrict__ xl,
                                                       const float *__restrict__ f,
@@ -433,7 +433,7 @@ __global__ void __launch_bounds__(BX *BY) k_fcg_dir(const float *__restrict__ z,
   const float zm = sc->zmean;
   float dq = 0.0f, dr = 0.0f;
   // grid-stride over tiles of 128 x 8 cells: a few blocks per SM, so few
-  // same-address atomics in the final reduction
+  // partial sums to combine
   const int tiles_x = (W + 4 * BX - 1) / (4 * BX), ntiles = tiles_x * ((H + BY - 1) / BY);
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const int x4 = ((t % tiles_x) * BX + threadIdx.x) * 4, y = (t / tiles_x) * BY + threadIdx.y;
@@ -823,8 +823,6 @@ int fcg_solve(FcgSolver &fs, const uint8_t *flag, const float *f, float *p, doub
   bool fresh = true, first = true;
   int it = 0, cur_d = 0;
   auto replace_residual = [&]() {
-    UBG_CUDA(cudaMemsetAsync(&fs.dev->rr, 0, sizeof(double), st));
-    UBG_CUDA(cudaMemsetAsync(&fs.dev->maxbits, 0, sizeof(unsigned), st));
     {
       ProfScope ps_(KC_KRYLOV, st);
       launch_pdl(k_fcg_resid, g_resid, blk, 0, st, fs.xh, fs.xl, f, L0.code, W, H, P, ihsq, r,
@@ -859,7 +857,7 @@ int fcg_solve(FcgSolver &fs, const uint8_t *flag, const float *f, float *p, doub
     }
     UBG_LAUNCH_CHECK();
     g_stats.launches++;
-    if (it > 0) {  // (also zeroes the accumulators of k_fcg_dir)
+    if (it > 0) {
       {
         ProfScope ps_(KC_KRYLOV, st);
         launch_pdl(k_fcg_zq, g_zq, blk, 0, st, z, fs.q, W, H, P, fs.dev, slot, fs.part);

@@ -2224,7 +2224,7 @@ void level_residual(const MgLevel &L, int cur, float *r, double *norm2, cudaStre
 //  * zero-gradient edges (corners included) on every level, so every level
 //    solves the zero-gradient system; no zero columns / rows in the
 //    prolongation;
-//  * the last level is the coarsest, with 40 sweeps.
+//  * the last level is the coarsest, with 16 sweeps.
 namespace {
 std::vector<MgLevel> ext_shapes(int W, int H, float h0) {
   std::vector<MgLevel> lv;
