@@ -326,8 +326,9 @@ __device__ __forceinline__ void st4_masked(float *row, int x, int lo, int hi, co
 // elsewhere, val the sum of the neighbours t1 .. t4 in the reference's order.
 // Faces with only open neighbours (codes k) need no selects, and the division
 // one range check for the four: the sweep is bound by issue as much as by
-// memory (405 -> 316 warp instructions per 8 faces a thread; 33 -> 28 us at
-// 4096x2048, where 151 MB at the copy rate are 22 us).
+// memory (405 -> 316 warp instructions per 8 faces a thread; two sweeps with
+// their setVBCs at 4096x2048 83.5 -> 76.8 us.  A sweep moves 151 MB, 22 us at the
+// copy rate).
 __device__ __forceinline__ void diffuse4(unsigned k, const float (&c)[4], const float (&t1)[4],
                                          const float (&t2)[4], const float (&t3)[4],
                                          const float (&t4)[4], float a, float den, float rden,
@@ -442,16 +443,22 @@ __device__ __forceinline__ void k_diffuse_body(const VelBufs &v, int srcx, int s
           [&](int a, int b, float q) { dy[(size_t)b * P + a] = q; });
   });
 }
-// A block takes one component of the velocity (blockIdx.z): 256x128 74.9 ->
-// 70.9 us per step, 4096x2048 600 -> 594, against both one after the other.
-// The members of a batch fill the chip as they are and take both (16 served
-// simulations: 9.09 against 9.16 ms).
+// On small grids a block takes one component of the velocity (blockIdx.z), which
+// fills the chip sooner: 1440x720 164 us per step against 171 with both one after
+// the other, 512x256 86.5 against 88.4.  From 3000 blocks per component on it takes
+// both, half as many blocks with twice the work each: two sweeps with their
+// setVBCs 40 us against 43 at 2900x1450 (4356 blocks), 234 against 248 at
+// 8192x4096 (1838 against 1854 per step); at 2045x1021 (2048 blocks) a step takes
+// 221 us either way.  The members of a batch fill the chip as they are and take
+// both (16 served simulations: 9.09 against 9.16 ms).
+constexpr unsigned kSplitBlocks = 3000;
 template <int EDGES>
 __global__ void __launch_bounds__(256) k_diffuse(VelBufs v, int srcx, int srcy,
                                                  const StepScalars *__restrict__ sc, int comps,
                                                  Bcs bc) {
   griddep_wait();
-  k_diffuse_body<EDGES>(v, srcx, srcy, sc, comps & (1 << blockIdx.z), bc, blockIdx.x, blockIdx.y);
+  const int c = gridDim.z == 1 ? comps : comps & (1 << blockIdx.z);
+  k_diffuse_body<EDGES>(v, srcx, srcy, sc, c, bc, blockIdx.x, blockIdx.y);
   griddep_launch();
 }
 
@@ -1250,7 +1257,9 @@ void launch_diffuse_sweep(const VelBufs &v, int srcx, int srcy, const StepScalar
                           cudaStream_t st, int edges, Bcs bc) {
   ProfScope ps_(KC_DIFFUSE, st);
   auto *k = edges == 0 ? k_diffuse<0> : (edges == 1 ? k_diffuse<1> : k_diffuse<2>);
-  launch_pdl(k, grid_vec(v.W, v.H, 2), dim3(VX, VY), 0, st, v, srcx, srcy, sc, comps, bc);
+  dim3 grid = grid_vec(v.W, v.H, 2);
+  if (grid.x * grid.y >= kSplitBlocks) grid.z = 1;
+  launch_pdl(k, grid, dim3(VX, VY), 0, st, v, srcx, srcy, sc, comps, bc);
   UBG_LAUNCH_CHECK();
   g_stats.launches++;
 }
