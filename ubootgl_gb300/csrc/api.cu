@@ -101,7 +101,7 @@ struct ubg_sim {
   MgLow lo;       // 16-bit correction hierarchy of the fixed-mode mixed solver
   FcgSolver fcg;  // tolerance-mode solver (allocated when that mode is set)
   StepScalars *d_sc = nullptr;
-  unsigned int *d_umax = nullptr;
+  unsigned int *d_umax = nullptr, *d_spare = nullptr;
   SinkCell *d_sinks = nullptr;
   // pinned host staging
   StepScalars *h_ring = nullptr;
@@ -349,9 +349,11 @@ struct ubg_sim {
       fx ^= 1;
       fy ^= 1;
     }
-    // (the tolerance solver may throw, which leaves max|u| as it was)
+    // (the tolerance solver may throw, which leaves max|u| as it was: the
+    // advection zeroes a spare word; a test for null in the kernel cost it 14
+    // instructions a warp)
     const bool tol = opt.solver_mode == UBG_SOLVE_TOLERANCE;
-    launch_advect(v, fx, fy, d_sc, st, true, bc, tol ? nullptr : d_umax);
+    launch_advect(v, fx, fy, d_sc, st, true, bc, tol ? d_spare : d_umax);
     fx ^= 1;
     fy ^= 1;
     if (tol) {
@@ -594,7 +596,7 @@ int ubg_create(const float *flag, int width, int height, float pwidth, float mu,
     s->v.cx = s->codes_x;
     s->v.cy = s->codes_y;
     s->d_sc = (StepScalars *)p; p += 256;
-    s->d_umax = (unsigned int *)p; p += 256;
+    s->d_umax = (unsigned int *)p; s->d_spare = s->d_umax + 32; p += 256;
     p += 256;
     s->d_sinks = (SinkCell *)p;
     s->v.pitch = s->P;

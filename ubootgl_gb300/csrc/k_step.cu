@@ -902,15 +902,14 @@ __device__ __forceinline__ void k_advect_body(const VelBufs &v, int srcx, int sr
   }
 }
 // umax_zero: max|u|, zeroed for the step's gradient kernel to accumulate (the
-// step's dt has been formed from it); null where the gradient kernel may not
-// follow (the tolerance solver can end in an error) and zeroes it itself.
+// step's dt has been formed from it); another word where the gradient kernel may
+// not follow (the tolerance solver can end in an error).
 template <bool BIL, bool EDGES, int TY>
 __global__ void __launch_bounds__(256, 4) k_advect(VelBufs v, int srcx, int srcy,
                                                 const StepScalars *__restrict__ sc, Bcs bc,
                                                 unsigned int *umax_zero) {
   griddep_wait();
-  if (EDGES && umax_zero && (blockIdx.x | blockIdx.y | threadIdx.x | threadIdx.y) == 0)
-    *umax_zero = 0u;
+  if (EDGES && (blockIdx.x | blockIdx.y | threadIdx.x | threadIdx.y) == 0) *umax_zero = 0u;
   k_advect_body<BIL, EDGES, TY>(v, srcx, srcy, sc, bc, blockIdx.x, blockIdx.y);
 }
 

@@ -141,7 +141,7 @@ void launch_diffuse_sweep(const VelBufs &v, int srcx, int srcy, const StepScalar
 // advected faces into buffer 1-src (faces the reference does not advect keep
 // their value).
 // edges: with the setVBCs after it, into the buffer written only; zeroes
-// *umax_zero unless that is null.
+// *umax_zero.
 void launch_advect(const VelBufs &v, int srcx, int srcy, const StepScalars *sc, cudaStream_t st,
                    bool edges = false, Bcs bc = Bcs{}, unsigned int *umax_zero = nullptr);
 // Divergence into f (simulation.cpp:166-171).
