@@ -521,6 +521,8 @@ int ubg_device_info(char *buf, size_t len) {
     UBG_CUDA(cudaGetDevice(&dev));
     cudaDeviceProp p;
     UBG_CUDA(cudaGetDeviceProperties(&p, dev));
+    // (the last key stays for callers that read it, as "cluster_top": -1 does in
+    // the autotuner's report)
     snprintf(buf, len,
              "{\"name\": \"%s\", \"sm\": \"%d.%d\", \"sms\": %d, \"mem_gb\": %.1f, "
              "\"cluster_coarse_solve\": \"%s\"}",

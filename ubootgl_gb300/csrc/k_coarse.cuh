@@ -13,10 +13,10 @@
 // inner neighbour (factor -1, as in k_tile.cuh).
 //
 // What bounds it: latency, a few hundred dependent instructions per visit.
-// 64x32 and down: 10.4 us (ncu).  It was 13.6 with the codes read level by
-// level (a memory latency each) and the tolerance hierarchy's edges behind a
-// uniform branch in every half sweep (132 against 80 cycles per half sweep of
-// one warp).  Before, with 4 columns x 2 rows per lane but always
+// 64x32 and down: 11.7 us (ncu, cold).  The codes read level by level (a memory
+// latency each) and the tolerance hierarchy's edges behind a uniform branch in
+// every half sweep (132 against 80 cycles per half sweep of one warp) were 3 us
+// more.  Before, with 4 columns x 2 rows per lane but always
 // 32 lanes per row, all 32 warps and a block barrier per half sweep, 128x64 and
 // down took 32 us: small levels waited for barriers of idle warps.  128x64 in
 // the block instead of two smoothing launches (5 us each in a step): 43

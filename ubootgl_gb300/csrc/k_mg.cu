@@ -1017,7 +1017,11 @@ void init_kernel_attributes() {
 // 64 cells, 112 x 48 stored), id 1 = 2 rows (128 x 32, 112 x 16).  The taller
 // region recomputes less; the shorter one gives a level of up to 1200 columns
 // more blocks, each with half the rows to go through per half sweep (512x256:
-// 8.5 against 10.0 us).  The autotuner tries both on every level.  A level of
+// 8.5 against 10.0 us).  The line was measured on grids wider than tall; a tall
+// grid of less width has blocks enough and takes the short region all the same
+// (V-cycle of 1024x4096 129 us against 107 with the tall one on level 0, 600x6000
+// 129 against 110; 1190x700 and 1100x1100 the same with either).  The autotuner
+// tries both on every level and finds it.  A level of
 // several members together is one launch (two, one per region, with the rule
 // above took 1442 us against 1260 for two steps of 20 members), of the shorter
 // region while it leaves SMs with fewer than two blocks (limits of 150 / 304 /

@@ -21,13 +21,13 @@
 // What bounds it: instruction issue and the FP32 pipe on large levels, the
 // latency of loads, six barriers and one pass through the code on small ones.
 // Against tiles in shared memory (red/black-split, 112 x 50 and 48 x 16
-// cells), ncu: level 0 of 4096x2048 53 us (89) with the residual, 51 (98) with
-// the prolongation, 2048x1024 17 us (33, 38), 1024x512 8 us (18, 20), 256x128
-// 7 us.  Edge cells in the registers instead of neighbours rebuilt from codes
+// cells), ncu: level 0 of 4096x2048 52.7 us (88.4) and 25.1 M warp instructions
+// with the residual, 50.8 us (96.6) and 25.3 M with the prolongation; level 1
+// (2048x1024) 18.5 us (34.3, 39.5), level 2 9 us (18.5), smaller ones 7 us.  Edge cells in the registers instead of neighbours rebuilt from codes
 // and positions: 5900 -> 2260 cycles for an edge warp's six half sweeps (2000
 // for others), 83 -> 78 us per step of 256x128.  Bounds checks outside the
 // blocks that need them, the packed magnitude check and W + E as scalar
-// additions (no register moves) were 2 us (32.4 -> 25.5 M warp instructions), f
+// additions (no register moves) were 2 us and a fifth of the instructions, f
 // kept in shared memory for the residual and one factor per cell another 2
 // (4096x2048 steps 660 -> 647 us).  Regions of 8 rows per warp (8 warps), and of
 // 128 x 32 cells, are slower there (58-60, 65 us).
@@ -624,7 +624,8 @@ __device__ __forceinline__ void run(const MgArgsT<S, SC> &a, const int region,
         const float2 va = add2(add2(make_float2(l + B[r].x, B[r].x + B[r].y), SA), NA);
         const float2 vb = add2(add2(make_float2(A[r].x + A[r].y, A[r].y + rr), SB), NB);
         const float V4[4] = {va.x, vb.x, va.y, vb.y};
-        // (-4 c is exact, so the fused form is the reference's sum)
+        // (-4 c is exact: c is a quarter of a finite sum, or not finite itself;
+        // so the fused form is the reference's sum)
 #pragma unroll
         for (int b = 0; b < 4; b++)
           q[b] = rnd<S>(F4[b] + __fmaf_rn(-4.0f, C4[b], V4[b]) * a.ihsq);
